@@ -12,6 +12,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <cmath>
+
 #include <string>
 #include <vector>
 
@@ -115,6 +117,37 @@ struct StencilView {
         return d[0][id];
     }
 };
+
+// ---- division by a constant -----------------------------------------------
+// x / d for a divisor known in advance, correctly rounded, in three FP64
+// operations (a division costs about nine on GB300's slow FP64 pipe):
+// q = RN(x y) with y = RN(1/d), the exact remainder x - q d by a fused
+// multiply-add, and one correction (Brisebarre, Muller and Raina,
+// "Accelerating correctly rounded floating-point division when the divisor is
+// known in advance", IEEE Trans. Computers 53(8), 2004, theorem 3).  The
+// theorem wants no under- or overflow: operands outside a wide exponent range
+// (zeros among them) take the division.
+struct DivBy {
+    double d, y;
+    int ok;   // the divisor lies in the range
+};
+
+inline DivBy div_by_const(double d)
+{
+    int e = 0;
+    std::frexp(d, &e);
+    return DivBy{d, 1.0 / d, std::isfinite(d) && d != 0.0 && e > -200 && e < 200};
+}
+
+__device__ __forceinline__ double div_by(double x, const DivBy& c)
+{
+    const int e = (__double2hiint(x) >> 20) & 0x7ff;
+    if (c.ok && e > 1023 - 700 && e < 1023 + 700) {
+        const double q = x * c.y;
+        return fma(fma(-q, c.d, x), c.y, q);
+    }
+    return x / c.d;
+}
 
 // ---- deterministic block reductions -----------------------------------------
 template <int NV>

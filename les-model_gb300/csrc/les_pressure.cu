@@ -37,19 +37,108 @@ __device__ __forceinline__ bool cell_coords(const Geo& g, int& i, int& j, int& k
 }
 
 // fast_apply_laplacian body, src/pressure.cpp:721-744 (bounds tests kept so
-// that the summation matches term for term).
+// that the summation matches term for term).  POW2: every off-diagonal
+// coefficient is a power of two (or its double, or zero), so its product is
+// exact and one fused multiply-add rounds as the multiply and the add do.
+template <bool POW2>
 __device__ __forceinline__ double apply_row(const StencilView& A, const double* __restrict__ p,
-                                            const Geo& g, int i, int j, int k, int id)
+                                            const Geo& g, int i, int j, int k, int id, double pc)
 {
     Coef7 a = A.at(id);
-    double val = a.c * p[id];
-    if (i > 0) val += a.w * p[id - g.si];
-    if (i < g.nx - 1) val += a.e * p[id + g.si];
-    if (j > 0) val += a.s * p[id - g.sj];
-    if (j < g.ny - 1) val += a.n * p[id + g.sj];
-    if (k > 0) val += a.b * p[id - 1];
-    if (k < g.nz - 1) val += a.t * p[id + 1];
+    double val = a.c * pc;
+    auto add = [&](double m, double x) { val = POW2 ? fma(m, x, val) : val + m * x; };
+    if (i > 0) add(a.w, p[id - g.si]);
+    if (i < g.nx - 1) add(a.e, p[id + g.si]);
+    if (j > 0) add(a.s, p[id - g.sj]);
+    if (j < g.ny - 1) add(a.n, p[id + g.sj]);
+    if (k > 0) add(a.b, p[id - 1]);
+    if (k < g.nz - 1) add(a.t, p[id + 1]);
     return val;
+}
+
+// How the rows of A are formed.  GB300 runs about two FP64 operations per SM
+// and clock, so the FP64 kernels are bound by the number of operations of a
+// row; each form gives the reference's roundings.
+//   GENERAL  seven products and six sums (13), a matrix of the caller
+//   POW2     one product and six fused multiply-adds (7), a device-built
+//            matrix whose 1/h^2 are powers of two
+//   SHARED   a device-built matrix of any spacing (8 to 10): the product
+//            x1 * p of a cell is the same number for its two i-neighbours
+//            (doubled exactly at a mirror, src/pressure.cpp:663-696), so it
+//            is formed once per cell and handed on -- along i in registers as
+//            the block marches, along j and k in shared memory; one product
+//            serves all axes whose spacings are equal
+// An FP64 Chebyshev(4)-PCG step of 256x128x128 (POW2, with step 0 and r.z in
+// the kernels next to them): 586 -> 415 ms.
+enum RowForm { ROW_GENERAL = 0, ROW_POW2 = 1, ROW_SHARED = 2 };
+
+struct RowTile {
+    double v[2][2][TBJ + 2][TBK + 2];   // [plane parity][y, z products]
+};
+
+// multiplier 0, 1 or 2 of a base coefficient
+__device__ __forceinline__ double mult(unsigned pack, unsigned state)
+{
+    const unsigned m = (pack >> (2 * state)) & 3u;
+    return m == 0u ? 0.0 : (m == 1u ? 1.0 : 2.0);
+}
+
+// Calls f(i, id, x_c, (A x)_c) for the cells of this thread's column on the
+// planes [blockIdx.z * ci, + ci).  Every thread of the block must call it.
+template <int FORM, class F>
+__device__ __forceinline__ void march_rows(const StencilView& A, const double* __restrict__ x, const Geo& g, int ci,
+                                           F f)
+{
+    const int k = blockIdx.x * TBK + threadIdx.x, j = blockIdx.y * TBJ + threadIdx.y;
+    const int i0 = blockIdx.z * ci, i1 = min(g.nx, i0 + ci);
+    const bool in = k < g.nz && j < g.ny;
+    if (FORM != ROW_SHARED) {
+        if (in)
+            for (int i = i0; i < i1; ++i) {
+                const int id = i * g.si + j * g.sj + k;
+                const double xc = x[id];
+                f(i, id, xc, apply_row<FORM == ROW_POW2>(A, x, g, i, j, k, id, xc));
+            }
+        return;
+    }
+    __shared__ RowTile tile;
+    const StencilCoef& c = A.k;
+    const bool same_y = c.y1 == c.x1, same_z = c.z1 == c.y1;
+    const int tj = threadIdx.y + 1, tk = threadIdx.x + 1;
+    const bool lo_j = in && threadIdx.y == 0 && j > 0, hi_j = in && threadIdx.y == TBJ - 1 && j < g.ny - 1;
+    const bool lo_k = in && threadIdx.x == 0 && k > 0, hi_k = in && threadIdx.x == TBK - 1 && k < g.nz - 1;
+    int id = i0 * g.si + j * g.sj + k;
+    double xc = in ? x[id] : 0.0;
+    double pw = in && i0 > 0 ? c.x1 * x[id - g.si] : 0.0, pc = c.x1 * xc;
+    for (int i = i0; i < i1; ++i, id += g.si) {
+        auto& ty = tile.v[i & 1][0];
+        auto& tz = tile.v[i & 1][same_z ? 0 : 1];
+        const double py = same_y ? pc : c.y1 * xc;
+        ty[tj][tk] = py;
+        if (!same_z) tz[tj][tk] = c.z1 * xc;
+        if (lo_j) ty[0][tk] = c.y1 * x[id - g.sj];
+        if (hi_j) ty[TBJ + 1][tk] = c.y1 * x[id + g.sj];
+        if (lo_k) tz[tj][0] = c.z1 * x[id - 1];
+        if (hi_k) tz[tj][TBK + 1] = c.z1 * x[id + 1];
+        const double xe = in && i < g.nx - 1 ? x[id + g.si] : 0.0;
+        const double pe = c.x1 * xe;
+        __syncthreads();   // one barrier per plane: the planes alternate between two tiles
+        if (in) {
+            const unsigned code = A.code[id];
+            const unsigned cd = code ? code - 1u : 0u, xs = cd % 5u, r = cd / 5u, ys = r & 3u, zs = r >> 2;
+            double val = c.c0 * xc;
+            if (i > 0) val = fma(mult(XW_PACK, xs), pw, val);
+            if (i < g.nx - 1) val = fma(mult(XE_PACK, xs), pe, val);
+            if (j > 0) val = fma(mult(YL_PACK, ys), ty[tj - 1][tk], val);
+            if (j < g.ny - 1) val = fma(mult(YH_PACK, ys), ty[tj + 1][tk], val);
+            if (k > 0) val = fma(mult(YL_PACK, zs), tz[tj][tk - 1], val);
+            if (k < g.nz - 1) val = fma(mult(YH_PACK, zs), tz[tj][tk + 1], val);
+            f(i, id, xc, code ? val : xc);   // code 0: identity row
+        }
+        xc = xe;
+        pw = pc;
+        pc = pe;
+    }
 }
 
 // calculate_divergence (src/pressure.cpp:256-329) + build_b_vector
@@ -144,20 +233,17 @@ __global__ void k_expand_stencil(Geo g, StencilView A, double* c, double* n, dou
 // out = A in (+ optional dot in.out reduced into the state).
 enum { DOT_NONE = 0, DOT_ALPHA = 1, DOT_SCAL0 = 2 };
 
-__global__ void k_spmv(Geo g, StencilView A, const double* __restrict__ p, double* __restrict__ q,
+template <int FORM>
+__global__ void k_spmv(Geo g, StencilView A, int ci, const double* __restrict__ p, double* __restrict__ q,
                        double* partials, unsigned* counter, SolverState* st, int dot_mode)
 {
     __shared__ double sm[32];
     if (dot_mode == DOT_ALPHA && st->done) return;
-    int i, j, k;
     double pq[1] = {0.0};
-    if (cell_coords(g, i, j, k))
-        for (; i < g.nx; i += gridDim.z) {   // planes blockIdx.z, + gridDim.z, ...
-            const int id = i * g.si + j * g.sj + k;
-            double val = apply_row(A, p, g, i, j, k, id);
-            q[id] = val;
-            pq[0] += p[id] * val;
-        }
+    march_rows<FORM>(A, p, g, ci, [&](int, int id, double pc, double val) {
+        q[id] = val;
+        pq[0] = fma(pc, val, pq[0]);
+    });
     if (dot_mode == DOT_NONE) return;
     if (last_block_sum<1>(pq, partials, counter, sm)) {
         if (threadIdx.x == 0 && threadIdx.y == 0) {
@@ -199,10 +285,11 @@ __global__ void k_resid(Geo g, const double* __restrict__ b, const double* __res
 // x += alpha p; r -= alpha q; ||r||; convergence test; k += 1
 // (src/pressure.cpp:381-392).  With the Jacobi preconditioner fused
 // (z = r / A_c, :420-428) it also forms r.z and the next beta.
+// z0 != nullptr: also the Chebyshev preconditioner's step 0, z0 = alpha0 r.
 __global__ void k_update(Geo g, StencilView A, double* __restrict__ x, double* __restrict__ r,
                          const double* __restrict__ p, const double* __restrict__ q,
                          double* __restrict__ z, double* partials, unsigned* counter,
-                         SolverState* st, int jacobi)
+                         SolverState* st, int jacobi, DivBy by_c0, double alpha0, double* __restrict__ z0)
 {
     __shared__ double sm[64];
     if (st->done) return;
@@ -215,12 +302,13 @@ __global__ void k_update(Geo g, StencilView A, double* __restrict__ x, double* _
             x[id] += alpha * p[id];
             double rv = r[id] + (-alpha) * q[id];
             r[id] = rv;
-            acc[0] += rv * rv;
+            acc[0] = fma(rv, rv, acc[0]);
             if (jacobi) {
-                double zv = rv / A.diag(id);
+                const double zv = A.code ? (A.code[id] ? div_by(rv, by_c0) : rv) : rv / A.d[0][id];
                 z[id] = zv;
-                acc[1] += rv * zv;
+                acc[1] = fma(rv, zv, acc[1]);
             }
+            if (z0) z0[id] = fma(alpha0, rv, 0.0);
         }
     if (last_block_sum<2>(acc, partials, counter, sm)) {
         if (threadIdx.x == 0 && threadIdx.y == 0) {
@@ -241,10 +329,18 @@ __global__ void k_update(Geo g, StencilView A, double* __restrict__ x, double* _
     }
 }
 
-enum { RD_RHO = 0, RD_BETA = 1, RD_SCAL0 = 2 };
+enum { RD_RHO = 0, RD_BETA = 1, RD_SCAL0 = 2, RD_NONE = 3 };
 
-// dot(a, b) reduced into the state: RD_RHO sets rho (:369); RD_BETA forms
-// beta = rz/rho and rho = rz (:399-408); RD_SCAL0 stores into scal[0].
+// What a kernel that ends with r.z does with the sum: RD_RHO sets rho (:369),
+// RD_BETA forms beta = rz/rho and rho = rz (:399-408), RD_SCAL0 stores it.
+__device__ __forceinline__ void dot_done(SolverState* st, int mode, double s)
+{
+    if (mode == RD_RHO) st->rho = s;
+    else if (mode == RD_BETA) { st->rz = s; st->beta = s / st->rho; st->rho = s; }
+    else st->scal[0] = s;
+}
+
+// dot(a, b) reduced into the state.
 __global__ void k_dot(Geo g, const double* __restrict__ a, const double* __restrict__ b,
                       double* partials, unsigned* counter, SolverState* st, int mode, int skip_done)
 {
@@ -255,14 +351,10 @@ __global__ void k_dot(Geo g, const double* __restrict__ a, const double* __restr
     if (cell_coords(g, i, j, k))
         for (; i < g.nx; i += gridDim.z) {   // planes blockIdx.z, + gridDim.z, ...
             const int id = i * g.si + j * g.sj + k;
-            s[0] += a[id] * b[id];
+            s[0] = fma(a[id], b[id], s[0]);
         }
     if (last_block_sum<1>(s, partials, counter, sm)) {
-        if (threadIdx.x == 0 && threadIdx.y == 0) {
-            if (mode == RD_RHO) st->rho = s[0];
-            else if (mode == RD_BETA) { st->rz = s[0]; st->beta = s[0] / st->rho; st->rho = s[0]; }
-            else st->scal[0] = s[0];
-        }
+        if (threadIdx.x == 0 && threadIdx.y == 0) dot_done(st, mode, s[0]);
     }
 }
 
@@ -288,13 +380,13 @@ __global__ void k_pupdate(Geo g, const double* __restrict__ z, double* __restric
 }
 
 __global__ void k_jacobi_pc(Geo g, StencilView A, const double* __restrict__ r, double* __restrict__ z,
-                            SolverState* st, int skip_done)
+                            SolverState* st, int skip_done, DivBy by_c0)
 {
     if (skip_done && st->done) return;
     int i, j, k;
     if (!cell_coords(g, i, j, k)) return;
     const int id = i * g.si + j * g.sj + k;
-    z[id] = r[id] / A.diag(id);
+    z[id] = A.code ? (A.code[id] ? div_by(r[id], by_c0) : r[id]) : r[id] / A.d[0][id];
 }
 
 // Chebyshev preconditioner, src/pressure.cpp:851-906.  Step 0:
@@ -306,26 +398,36 @@ __global__ void k_cheb0(Geo g, double alpha0, const double* __restrict__ r, doub
     int i, j, k;
     if (!cell_coords(g, i, j, k)) return;
     const int id = i * g.si + j * g.sj + k;
-    z[id] = 0.0 + alpha0 * r[id];
+    z[id] = fma(alpha0, r[id], 0.0);
 }
 
 // One inner step: res = r - A z; p = res + beta p; z' = z + alpha p.
-// pin == nullptr means p_{k-1} = r (first step).
-__global__ void k_cheb_step(Geo g, StencilView A, double alpha, double beta,
+// pin == nullptr means p_{k-1} = r (first step).  dot_mode != RD_NONE: also
+// r.z' (the last step).
+//
+// Bound by the FP64 pipe: 7 to 8 operations for the row and 5 for the
+// recurrence per cell (18 with every product rounded by itself).
+template <int FORM>
+__global__ void k_cheb_step(Geo g, StencilView A, int ci, double alpha, double beta,
                             const double* __restrict__ r, const double* __restrict__ zin,
                             const double* pin, double* pout, double* __restrict__ zout,
-                            SolverState* st, int skip_done)
+                            SolverState* st, int skip_done, double* partials, unsigned* counter, int dot_mode)
 {
+    __shared__ double sm[32];
     if (skip_done && st->done) return;
-    int i, j, k;
-    if (!cell_coords(g, i, j, k)) return;
-    const int id = i * g.si + j * g.sj + k;
-    double az = apply_row(A, zin, g, i, j, k, id);
-    double rv = r[id];
-    double res = rv - az;
-    double pv = res + beta * (pin ? pin[id] : rv);
-    pout[id] = pv;
-    zout[id] = zin[id] + alpha * pv;
+    double rz[1] = {0.0};
+    march_rows<FORM>(A, zin, g, ci, [&](int, int id, double zc, double az) {
+        const double rv = r[id];
+        const double res = rv - az;
+        const double pv = res + beta * (pin ? pin[id] : rv);
+        if (pout) pout[id] = pv;
+        const double zv = zc + alpha * pv;
+        zout[id] = zv;
+        rz[0] = fma(rv, zv, rz[0]);
+    });
+    if (dot_mode == RD_NONE) return;
+    if (last_block_sum<1>(rz, partials, counter, sm))
+        if (threadIdx.x == 0 && threadIdx.y == 0) dot_done(st, dot_mode, rz[0]);
 }
 
 // apply_pressure_BCs, src/pressure.cpp:14-93, face part.  The ordered face
@@ -497,11 +599,57 @@ __global__ void k_init_state(SolverState* st, double tol, int max_iter, int keep
 
 namespace les {
 
+// Grid of the FP64 solver's reductions in its iterations: every (k, j) tile
+// once and the i-planes shared out so that about eight blocks per SM run,
+// each summing its planes before the grid sum -- one partial, fence and
+// atomic per block instead of one per block and plane (16384 at
+// 256x128x128).  The kernels loop over planes i = blockIdx.z + t gridDim.z,
+// the row marches over chunks of consecutive planes.
+static dim3 reduce_grid(const les_ctx* c)
+{
+    dim3 gr = cell_grid(c->g);
+    const long long tiles = (long long)gr.x * gr.y;
+    const long long z = (8LL * c->sms + tiles - 1) / tiles;
+    gr.z = (unsigned)(z < 1 ? 1 : (z > c->g.nx ? c->g.nx : z));
+    return gr;
+}
+
+// A row march's chunks: the reductions' split
+struct MarchGrid {
+    dim3 grid;
+    int ci;
+};
+
+static MarchGrid march_grid(const les_ctx* c)
+{
+    MarchGrid m{reduce_grid(c), 0};
+    m.ci = (c->g.nx + (int)m.grid.z - 1) / (int)m.grid.z;
+    m.grid.z = (unsigned)((c->g.nx + m.ci - 1) / m.ci);
+    return m;
+}
+
+static int row_form(const les_ctx* c)
+{
+    if (c->stencil_mode != 1) return ROW_GENERAL;
+    auto pow2 = [](double v) { int e; return std::fabs(std::frexp(v, &e)) == 0.5; };
+    return pow2(c->coef.x1) && pow2(c->coef.y1) && pow2(c->coef.z1) ? ROW_POW2 : ROW_SHARED;
+}
+
+static void launch_spmv(les_ctx* c, int pid, const double* in, double* out, int dot_mode)
+{
+    const MarchGrid m = march_grid(c);
+    const int f = row_form(c);
+    auto k = f == ROW_POW2 ? k_spmv<ROW_POW2> : (f == ROW_SHARED ? k_spmv<ROW_SHARED> : k_spmv<ROW_GENERAL>);
+    if (pid >= 0) launch_p(c, pid, k, m.grid, cell_block(), c->g, stencil_view(c), m.ci, in, out, c->partials,
+                           c->counters + 1, c->state, dot_mode);
+    else launch(c, k, m.grid, cell_block(), c->g, stencil_view(c), m.ci, in, out, c->partials, c->counters + 1,
+                c->state, dot_mode);
+}
+
 les_status spmv_dev(les_ctx* c, const double* in, double* out)
 {
     if (!c->stencil_mode) return fail(c, LES_BAD_ARG, "no matrix: call les_build_stencil or les_set_stencil");
-    launch(c, k_spmv, cell_grid(c->g), cell_block(), c->g, stencil_view(c), in, out, c->partials,
-                                                             c->counters + 1, c->state, DOT_NONE);
+    launch_spmv(c, -1, in, out, DOT_NONE);
     return check_launch(c, "spmv");
 }
 
@@ -536,51 +684,80 @@ les_status pressure_bcs_dev(les_ctx* c, double* p)
     return check_launch(c, "pressure bcs");
 }
 
+// the two buffers of a Chebyshev apply: step 0 lands so that the last step
+// writes `z`
+static double* cheb_z0(les_ctx* c, const les_pcg_opts* o, double* z) { return (o->degree - 1) % 2 == 0 ? z : c->w[6]; }
+
+static double cheb_alpha0(const les_pcg_opts* o) { return 2.0 / ((o->lambda_max + o->lambda_min) / 2.0); }
+
 // Preconditioner application r -> z for PCG; kernels are skipped once the
-// state says done (skip_done).
-les_status precond_dev(les_ctx* c, const les_pcg_opts* o, const double* r, double* z, int skip_done)
+// state says done (skip_done).  dot_mode != RD_NONE: r.z too.  z0_done: the
+// update kernel has written Chebyshev's step 0.
+static les_status precond_dot(les_ctx* c, const les_pcg_opts* o, const double* r, double* z, int skip_done,
+                              int dot_mode, bool z0_done)
 {
     const Geo& g = c->g;
     StencilView A = stencil_view(c);
+    les_status st = LES_OK;
     switch (o->precond) {
     case LES_PC_JACOBI:
-        launch(c, k_jacobi_pc, cell_grid(g), cell_block(), g, A, r, z, c->state, skip_done);
-        return check_launch(c, "jacobi pc");
+        launch(c, k_jacobi_pc, cell_grid(g), cell_block(), g, A, r, z, c->state, skip_done, div_by_const(c->coef.c0));
+        st = check_launch(c, "jacobi pc");
+        break;
     case LES_PC_CHEBYSHEV: {
         if (o->degree < 1) return fail(c, LES_BAD_ARG, "Chebyshev degree must be >= 1");
-        les_status st = ensure_work(c);
-        if (st) return st;
+        if ((st = ensure_work(c))) return st;
         const double d = (o->lambda_max + o->lambda_min) / 2.0;
         const double cc = (o->lambda_max - o->lambda_min) / 2.0;
-        double alpha = 2.0 / d;
+        double alpha = cheb_alpha0(o);
         const int steps = o->degree - 1;
-        // ping-pong z so that the last write lands in `z`
         double* zb[2] = {z, c->w[6]};
         int cur = (steps % 2 == 0) ? 0 : 1;
-        launch(c, k_cheb0, cell_grid(g), cell_block(), g, alpha, r, zb[cur], c->state, skip_done);
+        if (!z0_done)
+            launch(c, k_cheb0, cell_grid(g), cell_block(), g, alpha, r, zb[cur], c->state, skip_done);
         double* pbuf = c->w[7];
+        const MarchGrid m = march_grid(c);
+        const int f = row_form(c);
+        auto kc = f == ROW_POW2 ? k_cheb_step<ROW_POW2>
+                                : (f == ROW_SHARED ? k_cheb_step<ROW_SHARED> : k_cheb_step<ROW_GENERAL>);
         for (int kq = 1; kq <= steps; ++kq) {
             double beta = (cc * alpha / 2.0) * (cc * alpha / 2.0);
             alpha = 1.0 / (d - beta);
-            launch_p(c, PROF_CHEB64, k_cheb_step, cell_grid(g), cell_block(), 
-                g, A, alpha, beta, r, zb[cur], kq == 1 ? nullptr : pbuf, pbuf, zb[cur ^ 1], c->state,
-                skip_done);
+            const bool last = kq == steps;
+            launch_p(c, PROF_CHEB64, kc, m.grid, cell_block(), g, A, m.ci, alpha, beta, r, (const double*)zb[cur],
+                     (const double*)(kq == 1 ? nullptr : pbuf), last ? nullptr : pbuf, zb[cur ^ 1], c->state,
+                     skip_done, c->partials, c->counters + 2, last ? dot_mode : (int)RD_NONE);
             cur ^= 1;
         }
-        return check_launch(c, "chebyshev pc");
+        if (steps > 0) return check_launch(c, "chebyshev pc");   // the last step formed r.z
+        st = check_launch(c, "chebyshev pc");
+        break;
     }
     case LES_PC_IC:
         if (!c->have_L) return fail(c, LES_BAD_ARG, "IC preconditioner needs les_build_ic or les_set_ic_factor");
-        return ic_apply_dev(c, r, z, nullptr, skip_done);
+        st = ic_apply_dev(c, r, z, nullptr, skip_done);
+        break;
     case LES_PC_IC_A: {
         // the factor arrays are A itself (src/pressure.cpp:363, :396)
         if (!c->A_valid) return fail(c, LES_BAD_ARG, "internal: IC-with-A needs A as arrays");
         const double* Ad[7] = {c->A[0], c->A[1], c->A[2], c->A[3], c->A[4], c->A[5], c->A[6]};
-        return ic_apply_dev(c, r, z, Ad, skip_done);
+        st = ic_apply_dev(c, r, z, Ad, skip_done);
+        break;
     }
     default:
         return fail(c, LES_BAD_ARG, "unknown preconditioner");
     }
+    if (!st && dot_mode != RD_NONE) {
+        launch(c, k_dot, reduce_grid(c), cell_block(), g, r, (const double*)z, c->partials, c->counters + 2, c->state,
+               dot_mode, skip_done);
+        st = check_launch(c, "r.z");
+    }
+    return st;
+}
+
+les_status precond_dev(les_ctx* c, const les_pcg_opts* o, const double* r, double* z, int skip_done)
+{
+    return precond_dot(c, o, r, z, skip_done, RD_NONE, false);
 }
 
 // The IC-with-A mode needs A as arrays; expand the coded matrix on demand.
@@ -601,20 +778,6 @@ les_status ensure_stored_A(les_ctx* c)
     return check_launch(c, "expand stencil");
 }
 
-// Grid of the FP64 solver's reductions in its iterations: every (k, j) tile
-// once and the i-planes shared out so that about eight blocks per SM run,
-// each summing its planes before the grid sum -- one partial, fence and
-// atomic per block instead of one per block and plane (16384 at
-// 256x128x128).  The kernels loop over planes i = blockIdx.z + t gridDim.z.
-static dim3 reduce_grid(const les_ctx* c)
-{
-    dim3 gr = cell_grid(c->g);
-    const long long tiles = (long long)gr.x * gr.y;
-    const long long z = (8LL * c->sms + tiles - 1) / tiles;
-    gr.z = (unsigned)(z < 1 ? 1 : (z > c->g.nx ? c->g.nx : z));
-    return gr;
-}
-
 // PCG of src/pressure.cpp:342-414 in FP64 with the solution in P and the
 // right-hand side in B.  The loop runs on the device; the host only polls
 // the state between batches of iterations (kernels after convergence exit
@@ -633,11 +796,10 @@ les_status pcg_fp64(les_ctx* c, const les_pcg_opts* o, les_pcg_result* res, int 
     double *r = c->w[0], *z = c->w[1], *p = c->w[2], *q = c->w[3];
     const dim3 gr = cell_grid(g), bl = cell_block();
     launch(c, k_init_state, 1, 1, c->state, o->tol, o->max_iter, keep_tol);
-    launch(c, k_spmv, gr, bl, g, A, x, q, c->partials, c->counters + 1, c->state, DOT_NONE);
+    launch_spmv(c, -1, x, q, DOT_NONE);
     launch(c, k_resid, gr, bl, g, b, q, r, c->partials, c->counters + 4, c->state);
-    st = precond_dev(c, o, r, p, 1);
+    st = precond_dot(c, o, r, p, 1, RD_RHO, false);
     if (st) return st;
-    launch(c, k_dot, gr, bl, g, r, p, c->partials, c->counters + 2, c->state, RD_RHO, 1);
     st = check_launch(c, "pcg init");
     if (st) return st;
     if (o->max_iter == 0) {
@@ -649,17 +811,17 @@ les_status pcg_fp64(les_ctx* c, const les_pcg_opts* o, les_pcg_result* res, int 
     }
     const bool jac = o->precond == LES_PC_JACOBI;
     const dim3 grr = reduce_grid(c);
+    const bool cheb = o->precond == LES_PC_CHEBYSHEV;
+    const double alpha0 = cheb ? cheb_alpha0(o) : 0.0;
+    double* z0 = cheb ? cheb_z0(c, o, z) : nullptr;
+    const DivBy by_c0 = div_by_const(c->coef.c0);
     int launched = 0, batch = 4;
     for (;;) {
         for (int it = 0; it < batch; ++it) {
-            launch_p(c, PROF_SPMV64, k_spmv, grr, bl, g, A, p, q, c->partials, c->counters + 1, c->state, DOT_ALPHA);
-            launch_p(c, PROF_UPDATE64, k_update, grr, bl, g, A, x, r, p, q, z, c->partials, c->counters + 5, c->state,
-                                                jac ? 1 : 0);
-            if (!jac) {
-                st = precond_dev(c, o, r, z, 1);
-                if (st) return st;
-                launch(c, k_dot, grr, bl, g, r, z, c->partials, c->counters + 2, c->state, RD_BETA, 1);
-            }
+            launch_spmv(c, PROF_SPMV64, p, q, DOT_ALPHA);
+            launch_p(c, PROF_UPDATE64, k_update, grr, bl, g, A, x, r, (const double*)p, (const double*)q, z, c->partials,
+                     c->counters + 5, c->state, jac ? 1 : 0, by_c0, alpha0, z0);
+            if (!jac && (st = precond_dot(c, o, r, z, 1, RD_BETA, cheb))) return st;
             launch(c, k_pupdate, gr, bl, g, z, p, c->state);
         }
         launched += batch;
@@ -890,10 +1052,9 @@ les_status les_lambda_max(les_ctx* c, int n_iter, const double* v0, double* lamb
     st = check_cuda(c, cudaMemcpyAsync(v, v0, sizeof(double) * g.n, cudaMemcpyHostToDevice, c->stream), "upload v0");
     if (st) return st;
     const dim3 gr = cell_grid(g), bl = cell_block();
-    StencilView A = stencil_view(c);
     double lam = 0.0;
     for (int it = 0; it < n_iter; ++it) {
-        launch(c, k_spmv, gr, bl, g, A, v, w, c->partials, c->counters + 1, c->state, DOT_SCAL0);
+        launch_spmv(c, -1, v, w, DOT_SCAL0);
         // lambda = v.w (spmv's fused dot is p.q = v.w)
         st = read_state(c);
         if (st) return st;
