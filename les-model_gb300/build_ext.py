@@ -33,6 +33,9 @@ UNITS = {
     "les_col_sj64.cu": [],
     "les_col_sj128.cu": [],
     "les_col_sj256.cu": [],
+    "les_plane.cu": [],
+    "les_plane_lo.cu": [],
+    "les_plane_hi.cu": [],
     "les_ensemble.cu": [],
     "les_tune.cu": [],
     "les_adjoint.cu": ["-fmad=false"],

@@ -49,14 +49,22 @@
 namespace {
 
 // x += e + alpha p_last (FP64 solution, FP32 correction)
-__global__ void k_x_update(Geo g, double* __restrict__ x, const float* __restrict__ e, const float* __restrict__ p0,
-                           const float* __restrict__ p1, const SolverState* in)
+// (pitch: row length of e and p)
+__device__ __forceinline__ void x_update(const Geo& g, int pitch, int t, double* __restrict__ x,
+                                         const float* __restrict__ e, const float* __restrict__ p0,
+                                         const float* __restrict__ p1, const SolverState* in)
 {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= g.n) return;
+    const int f = pitch == g.nz ? t : t + (t / g.nz) * (pitch - g.nz);
     const float a = (float)in->alpha;
     const float* p = in->buf ? p1 : p0;
-    x[t] = __dadd_rn(x[t], (double)fmaf(a, p[t], e[t]));
+    x[t] = __dadd_rn(x[t], (double)fmaf(a, p[f], e[f]));
+}
+
+__global__ void k_x_update(Geo g, int pitch, double* __restrict__ x, const float* __restrict__ e,
+                           const float* __restrict__ p0, const float* __restrict__ p1, const SolverState* in)
+{
+    x_update(g, pitch, blockIdx.x * blockDim.x + threadIdx.x, x, e, p0, p1, in);
 }
 
 // ---- batched over the cases of an ensemble ------------------------------------
@@ -95,11 +103,7 @@ __global__ void k_x_update_batch(const BatchCase* __restrict__ cs, const int* __
     const int c = batch_case(pre, n, blockIdx.x);
     const BatchCase& C = cs[c];
     if (!C.act) return;
-    const int t = (blockIdx.x - __ldg(pre + c)) * blockDim.x + threadIdx.x;
-    if (t >= C.g.n) return;
-    const float a = (float)C.in->alpha;
-    const float* p = C.in->buf ? C.p1 : C.p0;
-    C.x[t] = __dadd_rn(C.x[t], (double)fmaf(a, p[t], C.e[t]));
+    x_update(C.g, C.g.nz, (blockIdx.x - __ldg(pre + c)) * blockDim.x + threadIdx.x, C.x, C.e, C.p0, C.p1, C.in);
 }
 
 // ---- launch plumbing ----------------------------------------------------------
@@ -222,6 +226,14 @@ les_status col_plan(les_ctx* c, const les_pcg_opts* o, ViewF A, SolverState* in,
     P.in = in;
     P.out = out;
     P.cap = o->max_iter;
+    P.plane = plane_used(c, o);
+    if (P.plane) {
+        les_status st = plane_maps(c, o, P);
+        if (st) return st;
+        if ((size_t)2 * P.blocks_b + (size_t)P.blocks_a > c->partials_len)
+            return fail(c, LES_BAD_ARG, "plane march grid exceeds the reduction scratch");
+        return LES_OK;
+    }
     const int tja = (c->tune_tja == 8 || c->tune_tja == 16) ? c->tune_tja : 8;
     const int tjb = valid_tj_b(P.S, c->tune_tjb) ? c->tune_tjb : default_tj_b(P.S);
     const int wa = threads_a(tja) / 32, wb = threads_b(P.S, tjb) / 32;
@@ -240,21 +252,23 @@ static Coef coef_of(const ColPlan& P) { return Coef{P.A.k.c0, P.A.k.x1, P.A.k.y1
 
 les_status col_pass_a(les_ctx* c, const ColPlan& P, bool first, int pc)
 {
+    if (P.plane) return plane_pass_a(c, P, first, pc);
     float *z = c->f[1], *pb[2] = {c->f[2], c->f[3]}, *q = c->f[4], *e = c->f[5];
     float2* const part = reinterpret_cast<float2*>(c->partials);   // pass B's pairs, then pass A's
     const Defer df{part, P.blocks_b, part + 2 * (size_t)P.blocks_b};
-    launch_pdl(c, PROF_IN_SPMV, pick_a(stride_of(c), P.ma.tj, first), P.blocks_a, threads_a(P.ma.tj), c->g, P.ma, coef_of(P), (const float*)z,
+    launch_pdl(c, PROF_IN_SPMV, 0, pick_a(stride_of(c), P.ma.tj, first), P.blocks_a, threads_a(P.ma.tj), c->g, P.ma, coef_of(P), (const float*)z,
              (const float*)pb[pc], pb[pc ^ 1], q, e, c->partials, c->counters + 15, P.in, pc ^ 1, df, P.out, P.cap);
     return check_launch(c, "column pass A");
 }
 
 les_status col_pass_b(les_ctx* c, const ColPlan& P, bool first, int rin)
 {
+    if (P.plane) return plane_pass_b(c, P, first, rin);
     float* r[2] = {c->f[0], c->f[6]};
     float *z = c->f[1], *q = c->f[4];
     float2* const part = reinterpret_cast<float2*>(c->partials);
     const Defer df{part + 2 * (size_t)P.blocks_b, P.blocks_a, part};
-    launch_pdl(c, PROF_IN_CHEB, pick_b(stride_of(c), P.S, P.mb.tj, first), P.blocks_b, threads_b(P.S, P.mb.tj), c->g, P.mb, P.c3, P.inv_c0,
+    launch_pdl(c, PROF_IN_CHEB, 0, pick_b(stride_of(c), P.S, P.mb.tj, first), P.blocks_b, threads_b(P.S, P.mb.tj), c->g, P.mb, P.c3, P.inv_c0,
              (const float*)r[rin], r[rin ^ 1], (const float*)q, z, c->partials, c->counters + 14, P.in, P.out, P.cap,
              df);
     return check_launch(c, "column pass B");
@@ -320,10 +334,10 @@ les_status col_batch_x_update(cudaStream_t s, const BatchCase* cs, const int* pr
     return cudaPeekAtLastError() == cudaSuccess ? LES_OK : LES_CUDA_ERROR;
 }
 
-les_status col_x_update(les_ctx* c)
+les_status col_x_update(les_ctx* c, int pitch)
 {
     const Geo& g = c->g;
-    launch(c, k_x_update, (g.n + 255) / 256, 256, g, c->slot[LES_P], (const float*)c->f[5], (const float*)c->f[2],
+    launch(c, k_x_update, (g.n + 255) / 256, 256, g, pitch, c->slot[LES_P], (const float*)c->f[5], (const float*)c->f[2],
            (const float*)c->f[3], (const SolverState*)(c->state + 1));
     return check_launch(c, "solution update");
 }

@@ -8,6 +8,7 @@
 #include <vector>
 
 #include "les_internal.cuh"
+#include "les_mixed.cuh"
 
 using namespace les;
 
@@ -61,9 +62,10 @@ les_status ensure_work32(les_ctx* c)
 {
     if (c->f[0]) return LES_OK;
     for (int q = 0; q < 8; ++q) {
-        cudaError_t e = cudaMalloc(&c->f[q], sizeof(float) * (size_t)c->g.n);
+        const size_t bytes = sizeof(float) * (size_t)c->g.nx * c->g.ny * plane_pitch(c->g.nz);   // rows may be padded
+        cudaError_t e = cudaMalloc(&c->f[q], bytes);
         if (e != cudaSuccess) return check_cuda(c, e, "cudaMalloc(work32)");
-        cudaMemsetAsync(c->f[q], 0, sizeof(float) * (size_t)c->g.n, c->stream);
+        cudaMemsetAsync(c->f[q], 0, bytes, c->stream);
     }
     return LES_OK;
 }
@@ -421,10 +423,10 @@ les_status les_set_option(les_ctx* c, int option, int value)
     case LES_OPT_COL_STRIDE: c->col_stride = value ? 1 : 0; return LES_OK;
     case LES_OPT_FUSED: c->fused = value == 2 ? 2 : (value ? 1 : 0); return LES_OK;
     case LES_OPT_TMA: c->opt_tma = value ? 1 : 0; return LES_OK;
-    case LES_OPT_ROWS_A: c->tune_tja = value; return LES_OK;
-    case LES_OPT_ROWS_B: c->tune_tjb = value; return LES_OK;
-    case LES_OPT_CHUNK_A: c->tune_cia = value < 0 ? 0 : value; return LES_OK;
-    case LES_OPT_CHUNK_B: c->tune_cib = value < 0 ? 0 : value; return LES_OK;
+    case LES_OPT_ROWS_A: c->tune_tja = value; c->tune_plane = 0; return LES_OK;
+    case LES_OPT_ROWS_B: c->tune_tjb = value; c->tune_plane = 0; return LES_OK;
+    case LES_OPT_CHUNK_A: c->tune_cia = value < 0 ? 0 : value; c->tune_plane = 0; return LES_OK;
+    case LES_OPT_CHUNK_B: c->tune_cib = value < 0 ? 0 : value; c->tune_plane = 0; return LES_OK;
     default: return fail(c, LES_BAD_ARG, "unknown option");
     }
 }

@@ -970,7 +970,7 @@ les_status capture_mixed_fused(les_ctx* c, const les_pcg_opts* o, ViewF A, int k
     FusedPlan P;
     les_status st = fused_plan(c, o, A, in, out, P);
     if (st) return st;
-    if ((st = emit_outer_start(c, o, keep_tol))) return st;   // tol, r = b - A x, ||r||
+    if ((st = emit_outer_start(c, o, keep_tol, inner_pitch(c, o)))) return st;   // tol, r = b - A x, ||r||
     auto set_outer = [&](cudaGraphConditionalHandle h) -> les_status {
         launch(c, k_cond_outer, 1, 1, (const SolverState*)out, h, max_outer, o->max_iter);
         return check_launch(c, "outer condition");
@@ -996,7 +996,7 @@ les_status capture_mixed_fused(les_ctx* c, const les_pcg_opts* o, ViewF A, int k
             return set_inner(hi);
         });
         if (s2) return s2;
-        if ((s2 = emit_outer_update(c, P.col))) return s2;                   // x += e, r = b - A x, ||r||
+        if ((s2 = emit_outer_update(c, o, P.col))) return s2;                   // x += e, r = b - A x, ||r||
         return set_outer(ho);
     });
 }

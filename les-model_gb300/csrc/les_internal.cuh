@@ -320,6 +320,7 @@ struct les_ctx {
     int opt_tma = 0;              // LES_OPT_TMA: TMA-staged fused passes where the grid allows
     int tune_cia = 0, tune_cib = 0, tune_s = -1;   // autotuned march chunk lengths (0: occupancy rule)
     int tune_tja = 0, tune_tjb = 0;                // autotuned strip rows of the column passes (0: default)
+    int tune_plane = 0;           // the autotuner found the plane marches faster than any strips
     double share = 1.0;           // fraction of the GPU's resident warps the column passes size
                                   // their chunks for (1/k when k cases run together)
     struct les::TmaCache* tma = nullptr;
@@ -417,15 +418,17 @@ inline void launch_p(les_ctx* c, int pid, void (*k)(KArgs...), dim3 grid, dim3 b
 
 // Same, as a programmatic dependent launch when c->pdl is set: the kernel may
 // start while the kernel before it in the stream drains, so it must execute
-// dep_wait() before its first access to device memory.
+// dep_wait() before its first access to device memory.  smem: dynamic shared
+// memory.
 template <typename... KArgs, typename... Args>
-inline void launch_pdl(les_ctx* c, int pid, void (*k)(KArgs...), dim3 grid, dim3 block, Args... args)
+inline void launch_pdl(les_ctx* c, int pid, size_t smem, void (*k)(KArgs...), dim3 grid, dim3 block, Args... args)
 {
     cudaEvent_t e1 = nullptr;
     if (c->prof_on) prof_begin(c, pid, &e1);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
     cfg.stream = c->stream;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;

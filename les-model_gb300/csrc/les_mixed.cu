@@ -70,13 +70,13 @@ inline dim3 resid_grid(const Geo& g)
 }
 
 // Outer residual: r = b - A x in FP64, its FP32 copy for the inner solve, and
-// ||r||^2 in FP64.  Sets the outer state done once ||r|| < tol.
+// ||r||^2 in FP64 (pitch: row length of r32).  Sets the outer state done once ||r|| < tol.
 // (bx, by, bz): block coordinates in the grid of resid_grid(g); (lb, nb):
 // this block among the blocks of the reduction
 __device__ __forceinline__ void outer_resid(const Geo& g, const StencilView& A, const double* __restrict__ x,
-                                            const double* __restrict__ b, float* __restrict__ r32, double* partials,
-                                            unsigned* counter, SolverState* st, int outer, int bx, int by, int bz,
-                                            int lb, int nb)
+                                            const double* __restrict__ b, float* __restrict__ r32, int pitch,
+                                            double* partials, unsigned* counter, SolverState* st, int outer, int bx,
+                                            int by, int bz, int lb, int nb)
 {
     __shared__ double sm[32];
     const int k = bx * TBK + threadIdx.x, j = by * TBJ + threadIdx.y;
@@ -86,7 +86,10 @@ __device__ __forceinline__ void outer_resid(const Geo& g, const StencilView& A, 
         for (int i = i0; i < i1; ++i) {
             const int id = i * g.si + j * g.sj + k;
             const double r = b[id] - row64(A, x, g, i, j, k, id);
-            r32[id] = d2f_bits(r);
+            float* const row = r32 + (size_t)(i * g.ny + j) * pitch;
+            row[k] = d2f_bits(r);
+            if (k == g.nz - 1)
+                for (int q = g.nz; q < pitch; ++q) row[q] = 0.f;   // the pads stay zero
             rr[0] = fma(r, r, rr[0]);
         }
     }
@@ -103,10 +106,10 @@ __device__ __forceinline__ void outer_resid(const Geo& g, const StencilView& A, 
 }
 
 __global__ void k_outer_resid(Geo g, StencilView A, const double* __restrict__ x, const double* __restrict__ b,
-                              float* __restrict__ r32, double* partials, unsigned* counter, SolverState* st,
-                              int outer)
+                              float* __restrict__ r32, int pitch, double* partials, unsigned* counter,
+                              SolverState* st, int outer)
 {
-    outer_resid(g, A, x, b, r32, partials, counter, st, outer, blockIdx.x, blockIdx.y, blockIdx.z, block_linear_id(),
+    outer_resid(g, A, x, b, r32, pitch, partials, counter, st, outer, blockIdx.x, blockIdx.y, blockIdx.z, block_linear_id(),
                 block_count());
 }
 
@@ -119,7 +122,7 @@ __global__ void k_outer_resid_batch(const BatchCase* __restrict__ cs, const int*
     if (!C.act) return;
     const int b0 = __ldg(pre + c), nb = __ldg(pre + c + 1) - b0, lb = blockIdx.x - b0;
     const int gx = (C.g.nz + TBK - 1) / TBK, gy = (C.g.ny + TBJ - 1) / TBJ;
-    outer_resid(C.g, C.A, C.x, C.b, C.r0, C.partials, C.counters + 8, C.out, -1, lb % gx, (lb / gx) % gy,
+    outer_resid(C.g, C.A, C.x, C.b, C.r0, C.g.nz, C.partials, C.counters + 8, C.out, -1, lb % gx, (lb / gx) % gy,
                 lb / (gx * gy), lb, nb);
 }
 
@@ -436,7 +439,8 @@ les_status pcg_mixed_impl(les_ctx* c, const les_pcg_opts* o, les_pcg_result* res
     const int max_outer = o->max_outer > 0 ? o->max_outer : 50;
 
     launch(c, k_set_outer, 1, 1, out, o->tol, keep_tol);
-    launch_p(c, PROF_OUTER, k_outer_resid, resid_grid(g), bl, g, A, x, b, r, c->partials, c->counters + 8, out, 0);
+    const int pitch = inner_pitch(c, o);
+    launch_p(c, PROF_OUTER, k_outer_resid, resid_grid(g), bl, g, A, x, b, r, pitch, c->partials, c->counters + 8, out, 0);
     st = check_launch(c, "outer residual");
     if (st) return st;
     st = read_state(c);
@@ -489,13 +493,13 @@ les_status pcg_mixed_impl(les_ctx* c, const les_pcg_opts* o, les_pcg_result* res
         }
         // ---- correction and the new FP64 residual
         if (c->fused && col_supported(c, o)) {
-            st = col_x_update(c);   // x += e + alpha p: the column passes defer the last update of e
+            st = col_x_update(c, pitch);   // x += e + alpha p: the column passes defer the last update of e
             if (st) return st;
         } else {
             launch(c, k_x_add, gr, bl, g, x, e);
         }
         ++outer;
-        launch_p(c, PROF_OUTER, k_outer_resid, resid_grid(g), bl, g, A, x, b, r, c->partials, c->counters + 8, out, outer);
+        launch_p(c, PROF_OUTER, k_outer_resid, resid_grid(g), bl, g, A, x, b, r, pitch, c->partials, c->counters + 8, out, outer);
         st = check_launch(c, "outer correction");
         if (st) return st;
         st = read_state(c);
@@ -533,12 +537,12 @@ les_status batch_outer_resid(cudaStream_t s, const BatchCase* cs, const int* pre
 
 // Launch helpers for the graph-captured mixed solve (les_fused.cu): the same
 // kernels as pcg_mixed_impl, with the outer count kept on the device.
-les_status emit_outer_start(les_ctx* c, const les_pcg_opts* o, int keep_tol)
+les_status emit_outer_start(les_ctx* c, const les_pcg_opts* o, int keep_tol, int pitch)
 {
     const Geo& g = c->g;
     launch(c, k_set_outer, 1, 1, c->state, o->tol, keep_tol);
     launch_p(c, PROF_OUTER, k_outer_resid, resid_grid(g), cell_block(), g, stencil_view(c), (const double*)c->slot[LES_P],
-             (const double*)c->slot[LES_B], c->f[0], c->partials, c->counters + 8, c->state, 0);
+             (const double*)c->slot[LES_B], c->f[0], pitch, c->partials, c->counters + 8, c->state, 0);
     return check_launch(c, "outer start");
 }
 
@@ -548,17 +552,17 @@ les_status emit_inner_start(les_ctx* c, const les_pcg_opts* o, int inner_cap)
     return check_launch(c, "inner start");
 }
 
-les_status emit_outer_update(les_ctx* c, bool deferred)
+les_status emit_outer_update(les_ctx* c, const les_pcg_opts* o, bool deferred)
 {
     const Geo& g = c->g;
     if (deferred) {
-        les_status st = col_x_update(c);
+        les_status st = col_x_update(c, inner_pitch(c, o));
         if (st) return st;
     } else {
         launch(c, k_x_add, cell_grid(g), cell_block(), g, c->slot[LES_P], (const float*)c->f[5]);
     }
     launch_p(c, PROF_OUTER, k_outer_resid, resid_grid(g), cell_block(), g, stencil_view(c), (const double*)c->slot[LES_P],
-             (const double*)c->slot[LES_B], c->f[0], c->partials, c->counters + 8, c->state, -1);
+             (const double*)c->slot[LES_B], c->f[0], inner_pitch(c, o), c->partials, c->counters + 8, c->state, -1);
     return check_launch(c, "outer update");
 }
 

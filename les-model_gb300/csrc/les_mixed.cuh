@@ -135,7 +135,20 @@ struct ColMap {
     int items;     // strips x chunks = warps with work
 };
 
+// Work split of one plane-march pass (les_plane.cuh): block b owns the k tile
+// b % nk, the row tile (b / nk) % nj and the plane chunk b / (nk * nj).
+struct PlaneMap {
+    int kw, nk;       // owned cells of a tile along k (a multiple of four), tiles
+    int tj, nj;       // owned rows of a tile, tiles
+    int ci;           // planes per chunk
+    int lk, groups;   // four-cell vectors of a tile row (halo included), row pairs
+    int items;        // blocks
+    int threads;      // lk * groups in whole warps
+};
+
 struct ColPlan {
+    bool plane = false;    // the plane marches (pa, pb) instead of the strips (ma, mb)
+    PlaneMap pa{}, pb{};
     int S = 0;             // Chebyshev levels (degree - 1); 0 = Jacobi
     ColCheb c3{};
     float inv_c0 = 1.f;
@@ -147,6 +160,15 @@ struct ColPlan {
     int cap = 0;
 };
 
+// rows of the plane marches' vectors, padded to whole 16-byte vectors
+constexpr int plane_pitch(int nz) { return (nz + 3) / 4 * 4; }
+bool plane_used(const les_ctx* c, const les_pcg_opts* o);   // the plane marches serve this solve
+les_status plane_maps(les_ctx* c, const les_pcg_opts* o, ColPlan& P);
+les_status plane_pass_a(les_ctx* c, const ColPlan& P, bool first, int pc);
+les_status plane_pass_b(les_ctx* c, const ColPlan& P, bool first, int rin);
+// row length of the inner vectors of this solve
+inline int inner_pitch(const les_ctx* c, const les_pcg_opts* o) { return plane_used(c, o) ? plane_pitch(c->g.nz) : c->g.nz; }
+
 // the column passes serve this solve (device-built matrix, Jacobi or
 // Chebyshev degree 2..7, option LES_OPT_FUSED = 1 without TMA)
 bool col_supported(const les_ctx* c, const les_pcg_opts* o);
@@ -155,7 +177,7 @@ les_status col_plan(les_ctx* c, const les_pcg_opts* o, ViewF A, SolverState* in,
 les_status col_pass_a(les_ctx* c, const ColPlan& P, bool first, int pc);
 les_status col_pass_b(les_ctx* c, const ColPlan& P, bool first, int rin);
 // x += e + alpha p_last: the update the column passes defer to the end of the solve
-les_status col_x_update(les_ctx* c);
+les_status col_x_update(les_ctx* c, int pitch);
 les_status inner_solve_fused(les_ctx* c, const les_pcg_opts* o, ViewF A, SolverState* in, SolverState* out,
                              int inner_cap);
 // ---- batched ensemble solve (les_ensemble.cu) ------------------------------
@@ -274,9 +296,10 @@ les_status capture_while_on(cudaStream_t* stream, Check check, Entry entry, Body
 }
 
 // graph capture of the whole mixed solve (fused inner iteration)
-les_status emit_outer_start(les_ctx* c, const les_pcg_opts* o, int keep_tol);
+// pitch: row length of the inner vectors of the passes that follow
+les_status emit_outer_start(les_ctx* c, const les_pcg_opts* o, int keep_tol, int pitch);
 les_status emit_inner_start(les_ctx* c, const les_pcg_opts* o, int inner_cap);
-les_status emit_outer_update(les_ctx* c, bool deferred);
+les_status emit_outer_update(les_ctx* c, const les_pcg_opts* o, bool deferred);
 les_status capture_mixed_fused(les_ctx* c, const les_pcg_opts* o, ViewF A, int keep_tol);
 ViewF view32_of(les_ctx* c);
 

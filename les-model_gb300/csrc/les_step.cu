@@ -133,7 +133,8 @@ les_status les::emit_step_pre(les_ctx* c, const les_step_params* prm, bool outer
     if ((st = physics_dev(c, prm, dt, dtp))) return st;
     if ((st = velocity_bcs_dev(c))) return st;
     if ((st = div_b_dev(c, dt, prm->rho, prm->rel_tol, dtp))) return st;
-    return outer_start ? emit_outer_start(c, &prm->pcg, prm->rel_tol > 0 ? 1 : 0) : LES_OK;
+    // (outer_start: the batched passes of an ensemble follow, on unpadded rows)
+    return outer_start ? emit_outer_start(c, &prm->pcg, prm->rel_tol > 0 ? 1 : 0, c->g.nz) : LES_OK;
 }
 
 les_status les::emit_step_post(les_ctx* c, const les_step_params* prm)

@@ -73,7 +73,7 @@ les_status prep(les_ctx* c)
     les_status st = ensure_work(c);
     if (!st) st = ensure_work32(c);
     if (st) return st;
-    const int n = c->g.n;
+    const int n = c->g.nx * c->g.ny * plane_pitch(c->g.nz);
     launch(c, k_tune_prep, (n + 255) / 256, 256, n, c->f[0], c->f[1], c->f[2], c->f[3], c->f[4], c->f[5], c->f[6]);
     launch(c, k_tune_partials, (unsigned)((c->partials_len + 255) / 256), 256, c->partials, c->partials_len);
     launch(c, k_tune_state, 1, 1, c->state + 1, c->state);
@@ -201,8 +201,27 @@ les_status tune_pass(std::vector<Case>& cs, cudaStream_t main, bool pass_b, doub
 les_status tune(std::vector<Case>& cs, cudaStream_t main, double base, double* best_us)
 {
     double ua = 0, ub = 0;
+    for (auto& q : cs) {
+        q.c->tune_plane = 0;
+        ++q.c->version;
+    }
     les_status st = tune_pass(cs, main, false, base, &ua);
     if (!st) st = tune_pass(cs, main, true, base, &ub);
+    // the plane marches, which choose their own tiles, against the best strips
+    bool plane = true;
+    for (auto& q : cs) {
+        q.c->tune_plane = 1;
+        q.c->share = base;
+        if (!plane_used(q.c, &q.o)) plane = false;
+    }
+    double up = 0;
+    if (!st && plane) st = time_round(cs, main, &up);
+    plane = plane && !st && up < ub;
+    for (auto& q : cs) {
+        q.c->tune_plane = plane;
+        ++q.c->version;
+    }
+    if (plane) ub = up;
     if (!st && best_us) *best_us = ub;   // an iteration with both chosen shapes
     // the next solve's own initialisation clears the frozen state
     for (auto& q : cs) q.c->share = base;
