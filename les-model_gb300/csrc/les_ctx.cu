@@ -221,6 +221,7 @@ void les_destroy(les_ctx* c)
     cudaFree(c->state);
     cudaFree(c->gsync);
     cudaFree(c->wave_prog);
+    cudaFree(c->gs_buf);
     if (c->h_state) cudaFreeHost(c->h_state);
     for (auto& e : c->prof_ev) cudaEventDestroy(e);
     for (auto& e : c->marks) cudaEventDestroy(e);

@@ -139,6 +139,9 @@ inline DivBy div_by_const(double d)
     return DivBy{d, 1.0 / d, std::isfinite(d) && d != 0.0 && e > -200 && e < 200};
 }
 
+// out of line: rare, and large where it is inlined
+__device__ __noinline__ static double div_slow(double x, double d) { return x / d; }
+
 __device__ __forceinline__ double div_by(double x, const DivBy& c)
 {
     const int e = (__double2hiint(x) >> 20) & 0x7ff;
@@ -146,7 +149,7 @@ __device__ __forceinline__ double div_by(double x, const DivBy& c)
         const double q = x * c.y;
         return fma(fma(-q, c.d, x), c.y, q);
     }
-    return x / c.d;
+    return div_slow(x, c.d);
 }
 
 // ---- deterministic block reductions -----------------------------------------
@@ -351,6 +354,8 @@ struct les_ctx {
     int* wave_prog = nullptr;
     int wave_prog_len = 0;
     int wave_epoch = 0;
+    double* gs_buf = nullptr;     // GS-SOR's skewed arrays
+    size_t gs_len = 0;
     std::string err;
     // accounting: kernel launches issued by this context, and optional CUDA
     // event timing of the solver's hot kernels (les_profile)

@@ -37,6 +37,10 @@
 
 using namespace les;
 
+namespace les {
+les_status pressure_bcs_dev(les_ctx* c, double* p);
+}
+
 namespace {
 
 struct Plane {
@@ -117,15 +121,15 @@ __device__ __forceinline__ void st_release(int* p, int v)
     asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
 
-// One thread: waits until *p has reached target (wrap-safe); false once the
-// wait gave up (~2 s) or another block raised the error flag.
-__device__ bool wait_progress(const int* p, int target, int* err)
+// Waits until *p has reached target (wrap-safe); false once the wait gave up
+// (~2 s) or another block raised the error flag.  seen: the last value read.
+__device__ bool wait_progress(const int* p, int target, int* err, int& seen)
 {
-    if (ld_acquire(p) - target >= 0) return true;
+    if ((seen = ld_acquire(p)) - target >= 0) return true;
     const unsigned long long t0 = globaltimer_ns();
     unsigned spins = 0;
     for (;;) {
-        if (ld_acquire(p) - target >= 0) return true;
+        if ((seen = ld_acquire(p)) - target >= 0) return true;
         if (*(volatile int*)err) return false;
         if ((++spins & 63u) == 0u && globaltimer_ns() - t0 > 2000000000ull) {
             atomicExch(err, 1);
@@ -135,19 +139,35 @@ __device__ bool wait_progress(const int* p, int target, int* err)
     }
 }
 
-// Max over the warp, the same value in every lane.
-__device__ __forceinline__ double warp_max_all(double v)
+// One counter that a lane of warp 0 watches for its block: before the steps
+// up to tend, *p must have reached base + min(tend + ahead, steps).  A value
+// seen earlier that already covers the target saves the read.
+struct Watch {
+    const int* p;   // nullptr: nothing to wait for
+    int base, ahead, seen;
+};
+
+// Waits for every lane's counter (all lanes at once: a read costs an L2 round
+// trip); false in every thread when a wait gave up.
+__device__ __forceinline__ bool wait_steps(const Wave& W, Watch& w, int tend, int* flag)
 {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
+    if (threadIdx.x < 32) {
+        bool ok = true;
+        if (w.p && tend + w.ahead > 0) {
+            const int target = w.base + min(tend + w.ahead, W.steps);
+            if (w.seen - target < 0) ok = wait_progress(w.p, target, W.err, w.seen);
+        }
+        ok = __all_sync(0xffffffffu, ok);
+        if (threadIdx.x == 0) *flag = ok;
+    }
+    __syncthreads();
+    return *flag != 0;
 }
 
-// Publishes `value` as the tile's progress after every thread's stores.
+// Publishes `value` as the tile's progress; after a block barrier that follows
+// every thread's stores (the release covers what the barrier ordered).
 __device__ __forceinline__ void publish(int* p, int value)
 {
-    __threadfence();
-    __syncthreads();
     if (threadIdx.x == 0) st_release(p, value);
 }
 
@@ -171,21 +191,16 @@ __device__ __forceinline__ TileDeps tile_deps(const Wave& W, int J, int K, int t
     return d;
 }
 
-// Waits for the progress a batch of steps [tau0, tend) needs.  A tile's row
-// next to this one is its row TJ-1 (skewed TJ-1 steps behind its row 0), so
-// the j-producer must be TJ-1 steps ahead; the k-producer's far lane reaches
-// a plane 31 steps after its near lane.  Returns false in every thread when a
-// wait gave up.
-__device__ __forceinline__ bool wait_batch(const Wave& W, const TileDeps& d, int base, int tend, int* flag)
+// The producers' counters, lanes 0 and 1.  A tile's row next to this one is its
+// row TJ-1 (skewed TJ-1 steps behind its row 0), so the j-producer must be
+// TJ-1 steps ahead; the k-producer's far lane reaches a plane 31 steps after
+// its near lane.
+__device__ __forceinline__ Watch watch_producers(const int* prog, const TileDeps& d, int base)
 {
-    if (threadIdx.x == 0) {
-        int ok = 1;
-        if (d.dj >= 0 && !wait_progress(W.prog + d.dj, base + min(tend + WAVE_TJ - 1, W.steps), W.err)) ok = 0;
-        if (ok && d.dk >= 0 && !wait_progress(W.prog + d.dk, base + min(tend + 31, W.steps), W.err)) ok = 0;
-        *flag = ok;
-    }
-    __syncthreads();
-    return *flag != 0;
+    Watch w{nullptr, base, 0, base - (1 << 20)};
+    if (threadIdx.x == 0 && d.dj >= 0) { w.p = prog + d.dj; w.ahead = WAVE_TJ - 1; }
+    if (threadIdx.x == 1 && d.dk >= 0) { w.p = prog + d.dk; w.ahead = 31; }
+    return w;
 }
 
 // ---- operand staging: every step's read-only (or not yet written) operands
@@ -265,13 +280,14 @@ __device__ bool ic_tile(const Wave& W, int t, int base, const T* __restrict__ Lc
         cp_async<sizeof(T)>(&sg.v[sl][4][w][lane], Lc + id);
         cp_commit();
     };
+    Watch watch = watch_producers(W.prog, d, base);
     T prev = T(0), outp = T(0);
     sg.xs[0][w][lane] = sg.xs[1][w][lane] = T(0);
 #pragma unroll
     for (int q = 0; q < WD - 1; ++q) stage(q);
     for (int tau0 = 0; tau0 < W.steps; tau0 += WB) {
         const int tend = min(tau0 + WB, W.steps);
-        if (!wait_batch(W, d, base, tend, &sg.flag)) {
+        if (!wait_steps(W, watch, tend, &sg.flag)) {
             cp_wait<0>();
             return false;
         }
@@ -343,207 +359,456 @@ __global__ void __launch_bounds__(WT) k_ic_wave(Wave W, int base, const T* __res
         ok = ic_tile<T, -1>(W, W.ntiles - 1 - t, base + W.steps + 1, Lc, Lw, Ls, Lb, r, z, sg);
 }
 
-// One lexicographic SOR sweep of one tile over the interior, :216-234:
+// ---- GS-SOR, src/pressure.cpp:212-246 -------------------------------------------
 // p = (1-omega) p + omega coef ((p_e + p_w)/dx2 + (p_n + p_s)/dy2 + (p_t + p_b)/dz2 - rhs)
 // with the west, south and bottom neighbours already updated in this sweep
-// and the east, north and top ones not yet.  POW2: dx2, dy2, dz2 are powers
-// of two, so x / d2 is exactly x * (1 / d2) and the divisions become
-// multiplications (same results bit for bit).  Accumulates the thread's max
-// |dp| into maxr.  Staged WD steps ahead: the old values a step reads -- the
-// cell, its east, north and top neighbours -- and rhs.  Those cells are
-// written only at later steps: the cell by this thread at its step, the east
-// one a step later, the north one by the next warp a step later (or by the
-// tile above, which waits for this tile's progress, published only after the
-// copies that read it completed), the top one by the next lane a step later.
-struct GsStage {
-    double v[WD][5][WAVE_TJ][32];   // p, p_east, p_north, p_top, rhs
-    double xs[2][WAVE_TJ][32];      // each row's result of the last two steps
-    int flag;
+// and the east, north and top ones not yet; after each sweep
+// apply_pressure_BCs and the test max|dp| < tol.
+//
+// Sweeps in flight.  A cell of sweep s needs, besides the new values of its
+// west, south and bottom neighbours, only values of sweep s-1 one hyperplane
+// ahead, so sweep s can follow sweep s-1 through the grid.  A block runs every
+// Q-th sweep of its tile and Q blocks share a tile, each waiting for the
+// progress of the one before on its own tile and on the tiles above, after
+// and diagonal to it (watch_old), in addition to the producers of its own
+// sweep.  One sweep at a time spends 700 of its 1000 steps filling and
+// draining the wavefront with one warp per SM sub-partition (256x128x128: 1.18
+// ms per sweep, FP64 pipe idle); in flight the sweeps keep several blocks on
+// every SM busy.  256x128x128: 1180 -> 195 us per sweep (the FP64 pipe alone
+// needs about 95); h = 1/161, 191x161x115: 2070 -> 370 us; 67x46x53: 570 -> 80.
+//
+// Boundary conditions inside a run of sweeps.  Faces: the value that
+// apply_pressure_BCs leaves on the face next to an interior cell is that
+// cell's own new value (0 at the outlet), so the cell's thread stores it.
+// Obstacle: a solid cell with a fluid neighbour takes that neighbour's value
+// after the sweep.  p keeps what the sweep computed (the sweep's own later
+// cells read that), and the value the next sweep must see as the cell's old
+// one goes to rep[sweep & 1], stored by the thread that computes the source
+// cell; two buffers, because a source west, south or below of its cell is
+// computed before the cell's old value is read.  A source's next-but-one value
+// cannot overtake a reader: source and cell are neighbours, so the source's
+// sweep s+2 waits for the cell's sweep s+1.  Which cells read rep (bit `planes`
+// words `rd`) or store to it (`wr`, with directions in `fl`) is found once per
+// solve (k_gs_flags).
+//
+// The test.  Sweeps run in batches of 1, 2, 4, ... 32; a batch records every
+// sweep's max|dp|.  If one before the batch's last was below tol, the field is
+// restored to the batch's start and exactly that many sweeps are run: the
+// result is that of testing after every sweep.
+//
+// Layout.  The lanes of a warp work on 32 different planes at a time, so in the
+// field's own layout every lane's 8 bytes lie in another sector (424 us per
+// sweep at 256x128x128, bound by those accesses).  The solve therefore runs on
+// skewed copies of p's interior and of the right-hand side: element (tile,
+// step, warp, lane) holds the cell that this thread works on at that step.
+// Every access of a step is then contiguous, and the old values of the east,
+// north and top neighbours are the next step's own elements of the same
+// thread, the next warp and the next lane: a step copies one new value per
+// cell instead of four.  Faces stay in p.
+struct Skew {
+    int wj, steps;
+    __device__ __forceinline__ size_t at(int i, int j, int k) const   // interior coordinates
+    {
+        const int l = k & 31, w = j % WAVE_TJ, t = (k >> 5) * wj + j / WAVE_TJ;
+        return ((size_t)t * steps + (i + l + w)) * WT + w * 32 + l;
+    }
 };
 
-template <bool POW2>
-__device__ bool gs_tile(const Wave& W, int t, int base, double d2x, double d2y, double d2z, double one_m_omega,
-                        double omega_coef, const double* __restrict__ rhs, double* p, double& maxr, GsStage& sg)
+struct GsArgs {
+    Wave W;
+    int Q, nb;                  // sweeps in flight, blocks per sweep
+    DivBy dx, dy, dz;           // dx2, dy2, dz2
+    double omega, coef, tol;
+    int max_iter;
+    double* p;                  // the field: its faces during the sweeps
+    const double* rhs;          // skewed, like the next ones
+    double* ps;                 // p's interior
+    double* rep[2];
+    size_t len;                 // elements of a skewed array
+    double *ps_back, *face_back, *rep_back;
+    const unsigned *rd, *wr;    // per column (j, k) of the grid and 32 planes: cells that read / store rep
+    const uint8_t* fl;          // per cell: bits 0..5 directions to store to, bit 7 the cell's own old value is 0
+    const int* solid_list;
+    int n_solid;
+    unsigned long long* gmax;   // max|dp| of each sweep of a batch (bit pattern)
+    SolverState* st;
+    GridSync gs;
+    int nx, ny, nz;
+};
+constexpr int GS_BATCH = 32;    // most sweeps in a batch
+constexpr int GS_MAX_FLIGHT = 8;
+// FP64 operations of a cell: divisions by any d (19), products by powers of
+// two joined to the sums (11), equal powers of two applied once (10) -- the
+// same roundings.
+enum GsForm { GS_DIV = 0, GS_POW2 = 1, GS_EQUAL = 2 };
+
+// Copied WD steps ahead: the cells' old values and rhs, the row above the
+// tile's last row and the column after its last lane.
+struct GsStage {
+    double own[WD][WAVE_TJ][32], rhs[WD][WAVE_TJ][32];
+    double north[WD][32], top[WD][WAVE_TJ];
+    double inlet[WAVE_TJ][32];      // the inlet face next to each column's first cell
+    double xs[2][WAVE_TJ][32];      // each row's result of the last two steps
+    int flag, flag0;
+};
+
+// The counters of sweep s-1, lanes 2 to 5: on this tile and the ones above,
+// after and diagonal to it.  The copies of a step read old values of its own
+// hyperplane and the next one, and the sources of solid cells there one more,
+// so this tile's sweep s-1 must be two steps past the last copied one; the
+// tile above reaches the same hyperplane TJ-1 of its own steps earlier (its
+// first row), the tile after 31 (its first lane).
+__device__ __forceinline__ void watch_old(Watch& w, const Wave& W, const int* prog, int J, int K, int t, int base)
+{
+    const bool n = J < W.wj - 1, top = K < W.wk - 1;
+    const int q = threadIdx.x;
+    if (q < 2 || q > 5) return;
+    if ((q == 3 && !n) || (q == 4 && !top) || (q == 5 && !(n && top))) return;
+    w.p = prog + t + (q == 3 || q == 5 ? 1 : 0) + (q == 4 || q == 5 ? W.wj : 0);
+    w.base = base;
+    w.ahead = WD - 1 + 3 - (q == 3 || q == 5 ? WAVE_TJ - 1 : 0) - (q == 4 || q == 5 ? 31 : 0);
+    w.seen = base - (1 << 20);
+}
+
+// Sweep `s` of a batch over tile t, the solve's sweep number `num`.  base:
+// progress value of this sweep's start (the one before: base - steps - 1).
+template <int FORM>
+__device__ bool gs_tile(const GsArgs& A, int t, int s, int num, int base, double one_m_omega, double omega_coef,
+                        unsigned long long& maxr, GsStage& sg)
 {
     constexpr unsigned FULL = 0xffffffffu;
+    const Wave& W = A.W;
+    int* const prog = W.prog + (s % A.Q) * W.ntiles;
+    const int* const prog_old = W.prog + ((s + A.Q - 1) % A.Q) * W.ntiles;
+    double* const p = A.p;
+    const Skew sk{W.wj, W.steps};
+    double* const rep_new = A.rep[num & 1];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int J = t % W.wj, K = t / W.wj;
-    const int jb = J * WAVE_TJ, rows = min(WAVE_TJ, W.ny - jb);
-    const int k = K * 32 + lane;   // interior coordinates: grid cell (i+1, j+1, k+1)
-    const bool kin = k < W.nz;
-    const int kc = min(k, W.nz - 1);
+    const int jb = J * WAVE_TJ, rows = min(WAVE_TJ, W.ny - jb), kb = K * 32, cols = min(32, W.nz - kb);
     const TileDeps d = tile_deps<1>(W, J, K, t);
-    const bool wact = w < rows;
+    const bool cell = w < rows && lane < cols;    // this thread has a column
+    const int jr = jb + min(w, rows - 1), k = kb + min(lane, cols - 1);
     const int ssi = W.si, ssj = W.sj;
-    const int rb = W.off + (jb + min(w, rows - 1)) * ssj + kc;   // (i = 0, this warp's row)
-    const int rs = W.off + (jb - 1) * ssj + kc;                  // the row below the tile (the wall before the first)
-    auto div2 = [&](double x, double dd) { return POW2 ? x * dd : x / dd; };
-    auto clampi = [&](int i) { return min(max(i, 0), W.nx - 1); };
+    const int rb = W.off + jr * ssj + k;          // (i = 0) in the field
+    const bool last_row = w == rows - 1, last_col = lane == cols - 1;
+    const bool wall_n = jr == W.ny - 1, wall_t = k == W.nz - 1;
+    const size_t tile = (size_t)W.steps * WT;     // elements of a tile
+    const size_t tb = t * tile + threadIdx.x;
+    const size_t nb = (t + 1) * tile + lane, ob = (t + W.wj) * tile + w * 32;   // the tiles above and after
+    // which old values lie in rep: bits of 32 planes of this column, the one
+    // above and the one after
+    const bool use_rep = num > 0 && A.n_solid > 0;
+    const int col = (jr + 1) * A.nz + k + 1, ncol = A.ny * A.nz;
+    const double* const rep_old = A.rep[(num & 1) ^ 1];
+    unsigned ro = 0, rn = 0, rt = 0, wo = 0;
+    int word = -1, wword = -1;
     auto stage = [&](int tau) {
-        const int id = rb + clampi(tau - lane - w) * ssi;
-        const int sl = tau & (WD - 1);
-        cp_async<8>(&sg.v[sl][0][w][lane], p + id);
-        cp_async<8>(&sg.v[sl][1][w][lane], p + id + ssi);
-        cp_async<8>(&sg.v[sl][2][w][lane], p + id + ssj);   // the row above (the wall past the last row)
-        cp_async<8>(&sg.v[sl][3][w][lane], p + id + 1);
-        cp_async<8>(&sg.v[sl][4][w][lane], rhs + id);
+        const int i = tau - lane - w, sl = tau & (WD - 1);
+        if (i >= 0 && i < W.nx && cell) {
+            const double *po = A.ps, *pn = A.ps, *pt = A.ps;
+            if (use_rep) {
+                const int gi = i + 1;   // grid plane
+                if ((gi >> 5) != word) {
+                    word = gi >> 5;
+                    const unsigned* const c = A.rd + (size_t)word * ncol + col;
+                    ro = __ldg(c);
+                    rn = __ldg(c + A.nz);
+                    rt = __ldg(c + 1);
+                }
+                if ((ro >> (gi & 31)) & 1u) po = rep_old;
+                if ((rn >> (gi & 31)) & 1u) pn = rep_old;
+                if ((rt >> (gi & 31)) & 1u) pt = rep_old;
+            }
+            const size_t at = tb + (size_t)tau * WT;
+            cp_async<8>(&sg.own[sl][w][lane], po + at);
+            cp_async<8>(&sg.rhs[sl][w][lane], A.rhs + at);
+            if (last_row) cp_async<8>(&sg.north[sl][lane], wall_n ? p + rb + i * ssi + ssj : pn + nb + (size_t)(tau - w) * WT);
+            if (last_col) cp_async<8>(&sg.top[sl][w], wall_t ? p + rb + i * ssi + 1 : pt + ob + (size_t)(tau - lane) * WT);
+            if (i == 0) cp_async<8>(&sg.inlet[w][lane], p + rb - ssi);
+        }
         cp_commit();
     };
+    // the outlet face is 0 after every sweep
+    const double outlet = num == 0 ? __ldcg(p + rb + W.nx * ssi) : 0.0;
     double prev = 0.0, outp = 0.0;
     sg.xs[0][w][lane] = sg.xs[1][w][lane] = 0.0;
+    Watch watch = watch_producers(prog, d, base);
+    if (s > 0) {
+        watch_old(watch, W, prog_old, J, K, t, base - W.steps - 1);
+        if (!wait_steps(W, watch, 0, &sg.flag0)) return false;
+    }
 #pragma unroll
     for (int q = 0; q < WD - 1; ++q) stage(q);
+    cp_wait<WD - 3>();   // steps 0 and 1; the barrier of the first wait makes them visible
     for (int tau0 = 0; tau0 < W.steps; tau0 += WB) {
         const int tend = min(tau0 + WB, W.steps);
-        if (!wait_batch(W, d, base, tend, &sg.flag)) {
+        if (!wait_steps(W, watch, tend, &sg.flag)) {
             cp_wait<0>();
             return false;
         }
-        // the row below the tile (updated by the tile below, or the wall row
-        // j = 0) for every step of warp 0, and the column before the near
-        // lane's (the tile before in k, or the wall column k = 0): clamped loads
-        double ps0[WB];
+        // new values of other tiles, through L2: the last row of the tile below
+        // (or the wall's face) for every step of warp 0, and the last lane of
+        // the tile before (lane q holds step tau0 + q's)
+        double ps0[WB], pb0 = 0.0;
 #pragma unroll
-        for (int q = 0; q < WB; ++q) ps0[q] = __ldcg(p + rs + clampi(tau0 + q - lane) * ssi);
-        const double pb0 = __ldcg(p + rb - kc + K * 32 - 1 + clampi(tau0 + (lane & (WB - 1)) - w) * ssi);
+        for (int q = 0; q < WB; ++q) {
+            const int i = tau0 + q - lane;
+            ps0[q] = 0.0;
+            if (w == 0 && cell && i >= 0 && i < W.nx)
+                ps0[q] = __ldcg(d.dj >= 0 ? A.ps + (t - 1) * tile + (size_t)(tau0 + q + WAVE_TJ - 1) * WT + 32 * (WAVE_TJ - 1) + lane
+                                          : p + rb + i * ssi - ssj);
+        }
+        {
+            const int q = lane & (WB - 1), i = tau0 + q - w;
+            if (w < rows && i >= 0 && i < W.nx)
+                pb0 = __ldcg(d.dk >= 0 ? A.ps + (t - W.wj) * tile + (size_t)(tau0 + q + 31) * WT + w * 32 + 31
+                                       : p + W.off + jr * ssj + i * ssi - 1);
+        }
 #pragma unroll
         for (int q = 0; q < WB; ++q) {
             const int tau = tau0 + q;
             if (tau >= tend) break;   // block-uniform
             stage(tau + WD - 1);
-            cp_wait<WD - 1>();        // step tau's old values are in
             const int i = tau - lane - w;
-            const bool act = wact && kin && i >= 0 && i < W.nx;
-            const int sl = tau & (WD - 1);
-            // plane i = 0: the west neighbour is the inlet face
-            const double pw = i == 0 ? __ldcg(p + rb - ssi) : prev;
+            const bool act = cell && i >= 0 && i < W.nx;
+            const int sl = tau & (WD - 1), sn = (tau + 1) & (WD - 1);
+            const double po = sg.own[sl][w][lane], rh = sg.rhs[sl][w][lane];
+            const double pe = i == W.nx - 1 ? outlet : sg.own[sn][w][lane];
+            const double pn = last_row ? sg.north[sl][lane] : sg.own[sn][min(w + 1, WAVE_TJ - 1)][lane];
+            const double pt = last_col ? sg.top[sl][w] : sg.own[sn][w][min(lane + 1, 31)];
+            const double pw = i == 0 ? sg.inlet[w][lane] : prev;
             double pb = __shfl_up_sync(FULL, outp, 1);
             const double v0 = __shfl_sync(FULL, pb0, q);
             pb = lane == 0 ? v0 : pb;
             const double ps = w == 0 ? ps0[q] : sg.xs[(tau - 1) & 1][w - 1][lane];
-            const double po = sg.v[sl][0][w][lane];
-            const double v = one_m_omega * po +
-                             omega_coef * ((div2(sg.v[sl][1][w][lane] + pw, d2x) + div2(sg.v[sl][2][w][lane] + ps, d2y)) +
-                                           div2(sg.v[sl][3][w][lane] + pb, d2z) - sg.v[sl][4][w][lane]);
-            if (act) p[rb + i * ssi] = v;
-            const double res = fabs(v - po);
-            maxr = (act && res > maxr) ? res : maxr;
+            const double ew = pe + pw, ns = pn + ps, tb2 = pt + pb;
+            double x;
+            if (FORM == GS_EQUAL) x = fma((ew + ns) + tb2, A.dx.y, -rh);
+            else if (FORM == GS_POW2) x = fma(tb2, A.dz.y, fma(ns, A.dy.y, ew * A.dx.y)) - rh;
+            else x = ((div_by(ew, A.dx) + div_by(ns, A.dy)) + div_by(tb2, A.dz)) - rh;
+            const double v = one_m_omega * po + omega_coef * x;
+            if (act) {
+                A.ps[tb + (size_t)tau * WT] = v;
+                // the faces next to this cell, src/pressure.cpp:14-72
+                const int id = rb + i * ssi;
+                if (i == 0) p[id - ssi] = v;
+                if (i == W.nx - 1) p[id + ssi] = 0.0;
+                if (jr == 0) p[id - ssj] = v;
+                if (wall_n) p[id + ssj] = v;
+                if (k == 0) p[id - 1] = v;
+                if (wall_t) p[id + 1] = v;
+                if (A.n_solid > 0) {
+                    const int gi = i + 1;
+                    if ((gi >> 5) != wword) {
+                        wword = gi >> 5;
+                        wo = __ldg(A.wr + (size_t)wword * ncol + col);
+                    }
+                    if ((wo >> (gi & 31)) & 1u) {   // the source of solid cells, or solid next to the outlet
+                        const unsigned f = A.fl[id];
+                        if (f & 1u) rep_new[sk.at(i + 1, jr, k)] = v;
+                        if (f & 2u) rep_new[sk.at(i - 1, jr, k)] = v;
+                        if (f & 4u) rep_new[sk.at(i, jr + 1, k)] = v;
+                        if (f & 8u) rep_new[sk.at(i, jr - 1, k)] = v;
+                        if (f & 16u) rep_new[sk.at(i, jr, k + 1)] = v;
+                        if (f & 32u) rep_new[sk.at(i, jr, k - 1)] = v;
+                        if (f & 128u) rep_new[sk.at(i, jr, k)] = 0.0;
+                    }
+                }
+                // max over non-negative doubles by their bit patterns; NaN is not selected
+                const unsigned long long r = (unsigned long long)__double_as_longlong(fabs(v - po));
+                if (r > maxr && r <= 0x7ff0000000000000ull) maxr = r;
+            }
             prev = outp = v;
             sg.xs[tau & 1][w][lane] = v;
-            __syncthreads();          // the next step reads this step's rows
+            cp_wait<WD - 3>();        // steps tau + 1 and tau + 2 of this thread are in
+            __syncthreads();          // the next step reads this step's rows and others' copies
         }
-        if (t != W.stall) publish(W.prog + t, base + tend);   // block-uniform
+        if (t != W.stall) publish(prog + t, base + tend);   // block-uniform
     }
     cp_wait<0>();
     return true;
 }
 
-// solve_pressure_GS, src/pressure.cpp:212-246: up to max_iter SOR sweeps over
-// the interior, each a pipelined wavefront followed by apply_pressure_BCs
-// (face closed form, then the obstacle copy) and the max|dp| < tol test.
-template <bool POW2>
-__global__ void __launch_bounds__(WT) k_gs_wave(Wave W, int base, double d2x, double d2y, double d2z, double omega,
-                                                double coef, double tol, int max_iter,
-                                                const double* __restrict__ rhs, double* p,
-                                                const uint8_t* __restrict__ solid, const int* __restrict__ solid_list,
-                                                int n_solid, double* block_max, SolverState* st, GridSync gs,
-                                                int nx, int ny, int nz)
+// Flags of the obstacle copy, src/pressure.cpp:73-92: a solid interior cell
+// takes its first fluid neighbour's value, in the order +i, -i, +j, -j, +k, -k.
+// If that neighbour is a face, the face next to the cell holds the cell's own
+// value (nothing to do) or, at the outlet, 0.
+__device__ __forceinline__ int first_fluid(const uint8_t* solid, int id, int si, int sj)
 {
-    __shared__ GsStage sg;
-    __shared__ double wmax[WAVE_TJ];
-    const int b = blockIdx.x, nb = gridDim.x;   // one tile per block at a time
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int gt = b * WT + threadIdx.x, gn = nb * WT;
-    const double one_m_omega = 1 - omega;
-    const double omega_coef = omega * coef;
+    if (!solid[id + si]) return 0;
+    if (!solid[id - si]) return 1;
+    if (!solid[id + sj]) return 2;
+    if (!solid[id - sj]) return 3;
+    if (!solid[id + 1]) return 4;
+    if (!solid[id - 1]) return 5;
+    return 6;
+}
+
+// One thread per column and word of 32 planes.
+__global__ void k_gs_flags(int nx, int ny, int nz, const uint8_t* __restrict__ solid, unsigned* __restrict__ rd,
+                           unsigned* __restrict__ wr, uint8_t* __restrict__ fl)
+{
     const int si = ny * nz, sj = nz;
-    const int nfaces_i = ny * nz;
-    int sweeps = 0;
-    bool converged = false;
-    for (int iter = 0; iter < max_iter; ++iter) {
-        double maxr = 0.0;
-        bool ok = true;
-        const int bs = base + iter * (W.steps + 1);
-        for (int t = b; t < W.ntiles && ok; t += nb)
-            ok = gs_tile<POW2>(W, t, bs, d2x, d2y, d2z, one_m_omega, omega_coef, rhs, p, maxr, sg);
-        if (!grid_barrier(gs) || !ok) return;
-        // apply_pressure_BCs faces: every face cell from interior values
-        {
-            const int nface = 2 * nfaces_i + 2 * (nx - 2) * nz + 2 * (nx - 2) * (ny - 2);
-            for (int q = gt; q < nface; q += gn) {
-                int i, j, k;
-                if (q < 2 * nfaces_i) {
-                    const int e = q % nfaces_i;
-                    i = (q < nfaces_i) ? 0 : nx - 1;
-                    j = e / nz; k = e - j * nz;
-                } else if (q < 2 * nfaces_i + 2 * (nx - 2) * nz) {
-                    int e = q - 2 * nfaces_i;
-                    const int half = (nx - 2) * nz;
-                    j = (e < half) ? 0 : ny - 1;
-                    e = e % half;
-                    i = 1 + e / nz; k = e % nz;
-                } else {
-                    int e = q - 2 * nfaces_i - 2 * (nx - 2) * nz;
-                    const int half = (nx - 2) * (ny - 2);
-                    k = (e < half) ? 0 : nz - 1;
-                    e = e % half;
-                    i = 1 + e / (ny - 2); j = 1 + e % (ny - 2);
+    const int col = blockIdx.x * blockDim.x + threadIdx.x, wi = blockIdx.y;
+    if (col >= si) return;
+    const int j = col / nz, k = col - j * nz;
+    unsigned r = 0u, w = 0u;
+    auto interior = [&](int i, int jj, int kk) {
+        return i >= 1 && i <= nx - 2 && jj >= 1 && jj <= ny - 2 && kk >= 1 && kk <= nz - 2;
+    };
+    for (int b = 0; b < 32; ++b) {
+        const int i = wi * 32 + b;
+        if (i >= nx) break;
+        const int id = i * si + col;
+        unsigned f = 0u;
+        if (interior(i, j, k)) {
+            if (solid[id]) {
+                const int q = first_fluid(solid, id, si, sj);
+                const int di[7] = {1, -1, 0, 0, 0, 0, 0}, dj[7] = {0, 0, 1, -1, 0, 0, 0}, dk[7] = {0, 0, 0, 0, 1, -1, 0};
+                if (q < 6) {
+                    if (interior(i + di[q], j + dj[q], k + dk[q])) r |= 1u << b;
+                    else if (q == 0) { r |= 1u << b; f = 128u; }   // the outlet face
                 }
-                const int id = i * si + j * sj + k;
-                if (i == nx - 1) { p[id] = 0.0; continue; }
-                const int jc = j < 1 ? 1 : (j > ny - 2 ? ny - 2 : j);
-                const int kc = k < 1 ? 1 : (k > nz - 2 ? nz - 2 : k);
-                const int ic = i == 0 ? 1 : i;
-                p[id] = __ldcg(p + ic * si + jc * sj + kc);
+            } else {   // the solid neighbours this cell is the first fluid neighbour of
+                if (interior(i + 1, j, k) && solid[id + si] && first_fluid(solid, id + si, si, sj) == 1) f |= 1u;
+                if (interior(i - 1, j, k) && solid[id - si] && first_fluid(solid, id - si, si, sj) == 0) f |= 2u;
+                if (interior(i, j + 1, k) && solid[id + sj] && first_fluid(solid, id + sj, si, sj) == 3) f |= 4u;
+                if (interior(i, j - 1, k) && solid[id - sj] && first_fluid(solid, id - sj, si, sj) == 2) f |= 8u;
+                if (interior(i, j, k + 1) && solid[id + 1] && first_fluid(solid, id + 1, si, sj) == 5) f |= 16u;
+                if (interior(i, j, k - 1) && solid[id - 1] && first_fluid(solid, id - 1, si, sj) == 4) f |= 32u;
             }
         }
-        if (!grid_barrier(gs)) return;
-        for (int q = gt; q < n_solid; q += gn) {
-            const int id = solid_list[q];
-            if (!solid[id + si]) p[id] = __ldcg(p + id + si);
-            else if (!solid[id - si]) p[id] = __ldcg(p + id - si);
-            else if (!solid[id + sj]) p[id] = __ldcg(p + id + sj);
-            else if (!solid[id - sj]) p[id] = __ldcg(p + id - sj);
-            else if (!solid[id + 1]) p[id] = __ldcg(p + id + 1);
-            else if (!solid[id - 1]) p[id] = __ldcg(p + id - 1);
-        }
-        // block max -> global max (exact), the same value in every thread (so
-        // that the break below is uniform)
-        maxr = warp_max_all(maxr);
-        if (lane == 0) wmax[w] = maxr;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double m = 0.0;
-            for (int q = 0; q < WAVE_TJ; ++q) m = fmax(m, wmax[q]);
-            block_max[b] = m;
-        }
-        if (!grid_barrier(gs)) return;
-        double gmax = 0.0;
-        for (int q = lane; q < nb; q += 32) gmax = fmax(gmax, __ldcg(block_max + q));
-        gmax = warp_max_all(gmax);
-        sweeps = iter + 1;
-        if (gmax < tol) { converged = true; break; }
-        // block_max is rewritten next sweep only after the sweep's barrier
+        if (f) w |= 1u << b;
+        fl[id] = (uint8_t)f;
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        st->iters = sweeps;
-        st->k = sweeps;
-        st->done = 1;
-        st->status = converged ? LES_OK : LES_NOT_CONVERGED;
+    rd[(size_t)wi * si + col] = r;
+    wr[(size_t)wi * si + col] = w;
+}
+
+// Skewed copies: p's interior and the right-hand side, src/pressure.cpp:197-210.
+__global__ void k_gs_skew(Geo g, Skew sk, double coef, DivBy two_dx, DivBy two_dy, DivBy two_dz,
+                          const double* __restrict__ u, const double* __restrict__ v, const double* __restrict__ w,
+                          const double* __restrict__ p, double* __restrict__ ps, double* __restrict__ rhs)
+{
+    const int k = blockIdx.x * TBK + threadIdx.x, j = blockIdx.y * TBJ + threadIdx.y, i = blockIdx.z;
+    if (i < 1 || i > g.nx - 2 || j < 1 || j > g.ny - 2 || k < 1 || k > g.nz - 2) return;
+    const int id = i * g.si + j * g.sj + k;
+    const size_t at = sk.at(i - 1, j - 1, k - 1);
+    const double div = div_by(u[id + g.si] - u[id - g.si], two_dx) + div_by(v[id + g.sj] - v[id - g.sj], two_dy) +
+                       div_by(w[id + 1] - w[id - 1], two_dz);
+    ps[at] = p[id];
+    rhs[at] = coef * div;
+}
+
+__global__ void k_gs_unskew(Geo g, Skew sk, const double* __restrict__ ps, double* __restrict__ p)
+{
+    const int k = blockIdx.x * TBK + threadIdx.x, j = blockIdx.y * TBJ + threadIdx.y, i = blockIdx.z;
+    if (i < 1 || i > g.nx - 2 || j < 1 || j > g.ny - 2 || k < 1 || k > g.nz - 2) return;
+    p[i * g.si + j * g.sj + k] = ps[sk.at(i - 1, j - 1, k - 1)];
+}
+
+// What a batch may have to go back to: p's interior and faces, and the old
+// values of solid cells (rep of the sweep before the batch); to: into the
+// backup, else from it.
+__device__ void gs_backup(const GsArgs& A, int num, bool to, int gt, int gn)
+{
+    auto move = [&](double* x, double* b) {
+        if (to) *b = __ldcg(x);
+        else *x = *b;
+    };
+    for (size_t c = gt; c < A.len; c += gn) move(A.ps + c, A.ps_back + c);
+    // the faces that sweeps read: next to the interior
+    const int mi = A.nx - 2, mj = A.ny - 2, mk = A.nz - 2, si = A.ny * A.nz, sj = A.nz;
+    const int fi = mj * mk, fj = mi * mk, fk = mi * mj;
+    for (int q = gt; q < 2 * (fi + fj + fk); q += gn) {
+        int e = q, id;
+        if (e < 2 * fi) {
+            const int h = e >= fi;
+            e -= h * fi;
+            id = (h ? A.nx - 1 : 0) * si + (1 + e / mk) * sj + 1 + e % mk;
+        } else if ((e -= 2 * fi) < 2 * fj) {
+            const int h = e >= fj;
+            e -= h * fj;
+            id = (1 + e / mk) * si + (h ? A.ny - 1 : 0) * sj + 1 + e % mk;
+        } else {
+            e -= 2 * fj;
+            const int h = e >= fk;
+            e -= h * fk;
+            id = (1 + e / mj) * si + (1 + e % mj) * sj + (h ? A.nz - 1 : 0);
+        }
+        move(A.p + id, A.face_back + q);
+    }
+    if (num > 0) {
+        const Skew sk{A.W.wj, A.W.steps};
+        for (int q = gt; q < A.n_solid; q += gn) {
+            const int id = A.solid_list[q], i = id / si, r = id - i * si, j = r / sj, k = r - j * sj;
+            move(A.rep[(num & 1) ^ 1] + sk.at(i - 1, j - 1, k - 1), A.rep_back + q);
+        }
     }
 }
 
-__global__ void k_stat_rhs_gs(Plane P, double coef, double two_dx, double two_dy, double two_dz,
-                              const double* __restrict__ u, const double* __restrict__ v,
-                              const double* __restrict__ w, double* __restrict__ rhs, int n)
+template <int FORM>
+__global__ void __launch_bounds__(WT, FORM == GS_DIV ? 5 : 6) k_gs_wave(const __grid_constant__ GsArgs A, int base)
 {
-    int id = blockIdx.x * blockDim.x + threadIdx.x;
-    if (id >= n) return;
-    int i = id / P.si, rem = id - i * P.si, j = rem / P.sj, k = rem - j * P.sj;
-    if (i < 1 || i > P.nx - 2 || j < 1 || j > P.ny - 2 || k < 1 || k > P.nz - 2) { rhs[id] = 0.0; return; }
-    double div = (u[id + P.si] - u[id - P.si]) / two_dx + (v[id + P.sj] - v[id - P.sj]) / two_dy +
-                 (w[id + 1] - w[id - 1]) / two_dz;
-    rhs[id] = coef * div;
+    __shared__ GsStage sg;
+    __shared__ unsigned long long wmax[WAVE_TJ];
+    const Wave& W = A.W;
+    const int blk = blockIdx.x % A.nb, q0 = blockIdx.x / A.nb;   // this block's tiles and sweeps
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int gt = blockIdx.x * WT + threadIdx.x, gn = gridDim.x * WT;
+    const double one_m_omega = 1 - A.omega, omega_coef = A.omega * A.coef;
+    int done = 0, run = 1, epoch = base;   // sweeps finished, sweeps of this batch, its first progress value
+    bool converged = false, redo = false;
+    while (done < A.max_iter && !converged) {
+        if (!redo) {
+            run = min(run, A.max_iter - done);
+            if (run > 1) gs_backup(A, done, true, gt, gn);
+        }
+        if (gt < GS_BATCH) A.gmax[gt] = 0ull;
+        if (!grid_barrier(A.gs)) return;
+        bool ok = true;
+        for (int s = q0; s < run && ok; s += A.Q) {
+            unsigned long long maxr = 0ull;
+            for (int t = blk; t < W.ntiles && ok; t += A.nb)
+                ok = gs_tile<FORM>(A, t, s, done + s, epoch + s * (W.steps + 1), one_m_omega, omega_coef, maxr, sg);
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                const unsigned long long x = __shfl_xor_sync(0xffffffffu, maxr, o);
+                maxr = x > maxr ? x : maxr;
+            }
+            if (lane == 0) wmax[w] = maxr;
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                for (int q = 1; q < WAVE_TJ; ++q) maxr = wmax[q] > maxr ? wmax[q] : maxr;
+                atomicMax(A.gmax + s, maxr);
+            }
+            __syncthreads();
+        }
+        if (!grid_barrier(A.gs) || !ok) return;
+        epoch += GS_BATCH * (W.steps + 1);
+        // the first sweep whose max|dp| is below tol (the same in every thread)
+        int hit = run;
+        for (int s = 0; s < run && hit == run; ++s)
+            if (__longlong_as_double((long long)__ldcg(A.gmax + s)) < A.tol) hit = s;
+        if (hit < run - 1) {   // before the batch's last: run that many again from its start
+            run = hit + 1;
+            redo = true;
+            gs_backup(A, done, false, gt, gn);
+        } else {
+            done += run;
+            converged = hit < run;
+            redo = false;
+            run = min(2 * run, GS_BATCH);
+        }
+        if (!grid_barrier(A.gs)) return;   // every thread has read gmax; restored values are in place
+    }
+    if (gt == 0) {
+        A.st->iters = done;
+        A.st->k = done;
+        A.st->done = 1;
+        A.st->status = converged ? LES_OK : LES_NOT_CONVERGED;
+    }
 }
 
 Plane plane_of(const Geo& g) { return Plane{g.nx, g.ny, g.nz, g.si, g.sj}; }
@@ -598,7 +863,8 @@ les_status check_barrier(les_ctx* c)
 // starting at grid cell `off`, and the progress base of this launch: the
 // launch uses progress values in (base, base + span]; the counters are only
 // compared against later bases, so they need no reset between launches.
-les_status wave_setup(les_ctx* c, int nx, int ny, int nz, int off, int span, Wave& W, int& base)
+// sets: progress counters per tile (GS-SOR: one set per sweep in flight).
+les_status wave_setup(les_ctx* c, int nx, int ny, int nz, int off, long long span, int sets, Wave& W, int& base)
 {
     W.nx = nx;
     W.ny = ny;
@@ -610,26 +876,27 @@ les_status wave_setup(les_ctx* c, int nx, int ny, int nz, int off, int span, Wav
     W.wk = (nz + 31) / 32;
     W.ntiles = W.wj * W.wk;
     W.steps = nx + 31 + WAVE_TJ - 1;
-    if (c->wave_prog_len < W.ntiles) {
+    const int len = W.ntiles * sets;
+    if (c->wave_prog_len < len) {
         cudaFree(c->wave_prog);
         c->wave_prog = nullptr;
         c->wave_prog_len = 0;
-        les_status st = check_cuda(c, cudaMalloc(&c->wave_prog, sizeof(int) * (size_t)W.ntiles), "cudaMalloc(wave)");
+        les_status st = check_cuda(c, cudaMalloc(&c->wave_prog, sizeof(int) * (size_t)len), "cudaMalloc(wave)");
         if (st) return st;
-        c->wave_prog_len = W.ntiles;
+        c->wave_prog_len = len;
         c->wave_epoch = 0;
-        st = check_cuda(c, cudaMemsetAsync(c->wave_prog, 0, sizeof(int) * (size_t)W.ntiles, c->stream), "memset");
+        st = check_cuda(c, cudaMemsetAsync(c->wave_prog, 0, sizeof(int) * (size_t)len, c->stream), "memset");
         if (st) return st;
     }
     if (span < 0 || span > (1 << 29)) return fail(c, LES_BAD_ARG, "wavefront: too many sweeps in one launch");
-    if (c->wave_epoch > (1 << 30) - span) {   // restart the counters well before the int range ends
+    if (c->wave_epoch > (1 << 30) - (int)span) {   // restart the counters well before the int range ends
         les_status st = check_cuda(c, cudaMemsetAsync(c->wave_prog, 0, sizeof(int) * (size_t)c->wave_prog_len,
                                                       c->stream), "memset");
         if (st) return st;
         c->wave_epoch = 0;
     }
     base = c->wave_epoch;
-    c->wave_epoch += span + 1;
+    c->wave_epoch += (int)span + 1;
     W.prog = c->wave_prog;
     W.err = (int*)(c->gsync + 2);
     W.stall = c->test_stall ? 0 : -1;
@@ -639,17 +906,21 @@ les_status wave_setup(les_ctx* c, int nx, int ny, int nz, int off, int span, Wav
 // Cooperative launch of a pipelined sweep: one tile per block at a time, as many blocks
 // as tiles but no more than can be resident at once (the tiles are handed out
 // in producer-first order, so any resident count finishes).
-les_status wave_launch(les_ctx* c, const void* fn, void** args, const Wave& W, GridSync* gs, int pid)
+// grid: blocks, no more than wave_resident.
+les_status wave_resident(les_ctx* c, const void* fn, int* blocks)
 {
     int per_sm = 0;
     les_status st = check_cuda(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, WT, 0), "occupancy");
     if (st) return st;
     if (per_sm < 1) return fail(c, LES_CUDA_ERROR, "wavefront kernel cannot be resident");
-    const long long cap = (long long)per_sm * c->sms;
-    const int grid = (int)(W.ntiles < cap ? W.ntiles : cap);
-    gs->nblocks = (unsigned)grid;
+    *blocks = per_sm * c->sms;
+    return LES_OK;
+}
+
+les_status wave_launch(les_ctx* c, const void* fn, void** args, int grid, int pid)
+{
     // count and generation only: the error word stays set until the host reads it
-    st = check_cuda(c, cudaMemsetAsync(c->gsync, 0, sizeof(unsigned) * 2, c->stream), "reset barrier");
+    les_status st = check_cuda(c, cudaMemsetAsync(c->gsync, 0, sizeof(unsigned) * 2, c->stream), "reset barrier");
     if (st) return st;
     cudaEvent_t e1 = nullptr;
     if (pid >= 0 && c->prof_on) prof_begin(c, pid, &e1);
@@ -672,30 +943,40 @@ les_status ic_apply_dev(les_ctx* c, const double* r, double* z, const double* co
     const double* const* L = Lsrc ? Lsrc : (const double* const*)c->L;
     Wave W;
     int base = 0;
-    les_status st = wave_setup(c, c->g.nx, c->g.ny, c->g.nz, 0, 2 * (c->g.nx + 32 + WAVE_TJ), W, base);
+    les_status st = wave_setup(c, c->g.nx, c->g.ny, c->g.nz, 0, 2 * (c->g.nx + 32 + WAVE_TJ), 1, W, base);
     if (st) return st;
     const double *Lc = L[0], *Lw = L[4], *Ls = L[2], *Lb = L[6];
-    GridSync gs = grid_sync(c, 0);
+    const void* fn = (const void*)k_ic_wave<double>;
+    int resident = 0;
+    st = wave_resident(c, fn, &resident);
+    if (st) return st;
+    const int grid = W.ntiles < resident ? W.ntiles : resident;
+    GridSync gs = grid_sync(c, grid);
     const SolverState* stp = c->state;
     int skip = skip_done;
     void* args[] = {&W, &base, (void*)&Lc, (void*)&Lw, (void*)&Ls, (void*)&Lb, (void*)&r, (void*)&z, &gs,
                     (void*)&stp, &skip};
-    return wave_launch(c, (const void*)k_ic_wave<double>, args, W, &gs, PROF_IC);
+    return wave_launch(c, fn, args, grid, PROF_IC);
 }
 
 les_status ic_apply_dev32(les_ctx* c, const float* r, float* z, const float* const* L, SolverState* st)
 {
     Wave W;
     int base = 0;
-    les_status s2 = wave_setup(c, c->g.nx, c->g.ny, c->g.nz, 0, 2 * (c->g.nx + 32 + WAVE_TJ), W, base);
+    les_status s2 = wave_setup(c, c->g.nx, c->g.ny, c->g.nz, 0, 2 * (c->g.nx + 32 + WAVE_TJ), 1, W, base);
     if (s2) return s2;
     const float *Lc = L[0], *Lw = L[4], *Ls = L[2], *Lb = L[6];
-    GridSync gs = grid_sync(c, 0);
+    const void* fn = (const void*)k_ic_wave<float>;
+    int resident = 0;
+    s2 = wave_resident(c, fn, &resident);
+    if (s2) return s2;
+    const int grid = W.ntiles < resident ? W.ntiles : resident;
+    GridSync gs = grid_sync(c, grid);
     const SolverState* stp = st;
     int skip = st ? 1 : 0;
     void* args[] = {&W, &base, (void*)&Lc, (void*)&Lw, (void*)&Ls, (void*)&Lb, (void*)&r, (void*)&z, &gs,
                     (void*)&stp, &skip};
-    return wave_launch(c, (const void*)k_ic_wave<float>, args, W, &gs, PROF_IC);
+    return wave_launch(c, fn, args, grid, PROF_IC);
 }
 
 les_status build_ic_dev(les_ctx* c)
@@ -726,39 +1007,92 @@ les_status solve_gs_dev(les_ctx* c, double dt, double rho, int max_iter, double 
     les_status st = ensure_work(c);
     if (st) return st;
     const les_mesh& m = c->mesh;
-    Plane P = plane_of(c->g);
-    double* rhs = c->w[0];
-    // one slot per warp of the cooperative grid
-    double* block_max = c->partials;
-    launch(c, k_stat_rhs_gs, (c->g.n + 255) / 256, 256, P, rho / dt, 2 * m.dx, 2 * m.dy, 2 * m.dz,
-                                                               c->slot[LES_U], c->slot[LES_V], c->slot[LES_W],
-                                                               rhs, c->g.n);
-    st = check_launch(c, "gs rhs");
-    if (st) return st;
     const double dx2 = m.dx * m.dx, dy2 = m.dy * m.dy, dz2 = m.dz * m.dz;
     const double coef = 1.0 / (2.0 * (1.0 / dx2 + 1.0 / dy2 + 1.0 / dz2));
     const Geo& g = c->g;
     if (g.nx < 3 || g.ny < 3 || g.nz < 3) return fail(c, LES_BAD_ARG, "GS-SOR needs an interior");
-    Wave W;
-    int base = 0;
-    st = wave_setup(c, g.nx - 2, g.ny - 2, g.nz - 2, g.si + g.sj + 1, max_iter * (g.nx - 2 + 32 + WAVE_TJ), W, base);
-    if (st) return st;
     // x / d2 for a power of two d2 is exactly x * (1 / d2)
     auto pow2 = [](double v) { int e; return std::frexp(v, &e) == 0.5; };
     const bool p2 = pow2(dx2) && pow2(dy2) && pow2(dz2);
-    double d2x = p2 ? 1.0 / dx2 : dx2, d2y = p2 ? 1.0 / dy2 : dy2, d2z = p2 ? 1.0 / dz2 : dz2;
-    double* p = c->slot[LES_P];
-    const uint8_t* solid = c->mask;
-    const int* list = c->solid_list;
-    int ns = c->n_solid;
-    SolverState* stp = c->state;
-    GridSync gs = grid_sync(c, 0);
-    int nx = g.nx, ny = g.ny, nz = g.nz;
-    void* args[] = {&W, &base, &d2x, &d2y, &d2z, &omega, (void*)&coef, &tol, &max_iter, (void*)&rhs, &p,
-                    (void*)&solid, (void*)&list, &ns, &block_max, &stp, &gs, &nx, &ny, &nz};
-    if ((size_t)W.ntiles > c->partials_len) return fail(c, LES_BAD_ARG, "internal: partials too small");
-    st = wave_launch(c, p2 ? (const void*)k_gs_wave<true> : (const void*)k_gs_wave<false>, args, W, &gs, -1);
+    const void* fn = !p2 ? (const void*)k_gs_wave<GS_DIV>
+                         : (dx2 == dy2 && dy2 == dz2 ? (const void*)k_gs_wave<GS_EQUAL> : (const void*)k_gs_wave<GS_POW2>);
+    int resident = 0;
+    st = wave_resident(c, fn, &resident);
     if (st) return st;
+    // Sweeps in flight: as many as there are resident blocks for, up to what a
+    // sweep's length has room for (a sweep starts about 20 steps behind the
+    // one before: the staging depth, the waits' granularity).
+    const int ntiles = ((g.ny - 2 + WAVE_TJ - 1) / WAVE_TJ) * ((g.nz - 2 + 31) / 32);
+    const int room = (g.nx - 2 + 31 + WAVE_TJ - 1) / 20 + 1;
+    int Q = resident / ntiles;
+    Q = Q < 1 ? 1 : (Q > room ? room : Q);
+    if (Q > GS_MAX_FLIGHT) Q = GS_MAX_FLIGHT;
+    if (Q > max_iter && max_iter > 0) Q = max_iter;
+    GsArgs a{};
+    int base = 0;
+    // progress values: every batch (about max_iter / GS_BATCH and the doubling
+    // ones before, one run again) takes GS_BATCH sweeps' worth
+    const long long batches = max_iter / GS_BATCH + 8;
+    st = wave_setup(c, g.nx - 2, g.ny - 2, g.nz - 2, g.si + g.sj + 1,
+                    batches * GS_BATCH * (long long)(g.nx - 2 + 32 + WAVE_TJ), Q, a.W, base);
+    if (st) return st;
+    a.len = (size_t)a.W.ntiles * a.W.steps * WT;
+    if (c->gs_len < 5 * a.len) {   // the skewed arrays, kept for the next solve
+        cudaFree(c->gs_buf);
+        c->gs_buf = nullptr;
+        c->gs_len = 0;
+        st = check_cuda(c, cudaMalloc(&c->gs_buf, sizeof(double) * 5 * a.len), "cudaMalloc(skewed sweeps)");
+        if (st) return st;
+        c->gs_len = 5 * a.len;
+    }
+    const int words = (g.nx + 31) / 32;
+    a.Q = Q;
+    a.nb = ntiles < resident ? ntiles : resident;
+    a.dx = div_by_const(dx2);
+    a.dy = div_by_const(dy2);
+    a.dz = div_by_const(dz2);
+    a.omega = omega;
+    a.coef = coef;
+    a.tol = tol;
+    a.max_iter = max_iter;
+    a.p = c->slot[LES_P];
+    a.ps = c->gs_buf;
+    double* const rhs = c->gs_buf + a.len;
+    a.rhs = rhs;
+    a.ps_back = c->gs_buf + 2 * a.len;
+    a.rep[0] = c->gs_buf + 3 * a.len;
+    a.rep[1] = c->gs_buf + 4 * a.len;
+    a.face_back = c->w[0];
+    a.rep_back = c->w[1];
+    unsigned* const rd = reinterpret_cast<unsigned*>(c->w[2]);   // two words per column and 32 planes: n doubles hold them
+    uint8_t* const fl = reinterpret_cast<uint8_t*>(c->w[3]);
+    a.rd = rd;
+    a.wr = rd + (size_t)words * g.si;
+    a.fl = fl;
+    a.solid_list = c->solid_list;
+    a.n_solid = c->n_solid;
+    a.gmax = reinterpret_cast<unsigned long long*>(c->partials);
+    a.st = c->state;
+    a.nx = g.nx;
+    a.ny = g.ny;
+    a.nz = g.nz;
+    const int grid = a.nb * Q;
+    a.gs = grid_sync(c, grid);
+    const Skew sk{a.W.wj, a.W.steps};
+    launch(c, k_gs_skew, cell_grid(g), cell_block(), g, sk, rho / dt, div_by_const(2 * m.dx), div_by_const(2 * m.dy),
+           div_by_const(2 * m.dz), (const double*)c->slot[LES_U], (const double*)c->slot[LES_V],
+           (const double*)c->slot[LES_W], (const double*)a.p, a.ps, rhs);
+    if (c->n_solid)
+        launch(c, k_gs_flags, dim3((g.si + 255) / 256, words), 256, g.nx, g.ny, g.nz, (const uint8_t*)c->mask, rd,
+               rd + (size_t)words * g.si, fl);
+    if ((st = check_launch(c, "gs set-up"))) return st;
+    void* args[] = {&a, &base};
+    if (max_iter > 0) {
+        st = wave_launch(c, fn, args, grid, -1);
+        if (st) return st;
+        launch(c, k_gs_unskew, cell_grid(g), cell_block(), g, sk, (const double*)a.ps, a.p);
+        if ((st = pressure_bcs_dev(c, a.p))) return st;   // of the last sweep
+    }
     st = check_barrier(c);
     if (st) return st;
     st = read_state(c);
