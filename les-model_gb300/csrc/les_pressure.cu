@@ -465,7 +465,7 @@ __global__ void k_pbc_obstacle(Geo g, const int* __restrict__ list, int n, const
 }
 
 // Interior RHS of the stationary solvers, src/pressure.cpp:119-132 / :197-210.
-__global__ void k_stat_rhs(Geo g, double coef, double two_dx, double two_dy, double two_dz,
+__global__ void k_stat_rhs(Geo g, double coef, DivBy two_dx, DivBy two_dy, DivBy two_dz,
                            const double* __restrict__ u, const double* __restrict__ v,
                            const double* __restrict__ w, double* __restrict__ rhs)
 {
@@ -473,85 +473,106 @@ __global__ void k_stat_rhs(Geo g, double coef, double two_dx, double two_dy, dou
     if (!cell_coords(g, i, j, k)) return;
     const int id = i * g.si + j * g.sj + k;
     if (i < 1 || i > g.nx - 2 || j < 1 || j > g.ny - 2 || k < 1 || k > g.nz - 2) { rhs[id] = 0.0; return; }
-    double div = (u[id + g.si] - u[id - g.si]) / two_dx + (v[id + g.sj] - v[id - g.sj]) / two_dy +
-                 (w[id + 1] - w[id - 1]) / two_dz;
+    double div = div_by(u[id + g.si] - u[id - g.si], two_dx) + div_by(v[id + g.sj] - v[id - g.sj], two_dy) +
+                 div_by(w[id + 1] - w[id - 1], two_dz);
     rhs[id] = coef * div;
 }
 
-// One Jacobi sweep, src/pressure.cpp:139-157, plus max|dp| reduced into the
-// state (max is order-independent, so this is exact).
-__global__ void k_jacobi_sweep(Geo g, double dx2, double dy2, double dz2, double denom,
-                               const double* __restrict__ cur, double* __restrict__ nxt,
-                               const double* __restrict__ rhs, double* partials, unsigned* counter,
-                               SolverState* st)
+// One Jacobi sweep, src/pressure.cpp:139-157, the faces of apply_pressure_BCs
+// (:14-72: every face cell takes the new value of the interior cell it clamps
+// to, the outlet 0, so that cell's thread stores it) and max|dp| (its bit
+// pattern: the order of non-negative doubles is that of their patterns, and
+// NaN is not selected).  The test of the sweep before, max|dp| < tol
+// (:164-170), is made by every block here: three slots of maxdp rotate, one
+// read, one formed, one cleared for the next sweep.
+//
+// Bound by the FP64 pipe: 10 operations per cell when the three 1/h^2 are the
+// same power of two, 11 for three powers of two, 19 with divisions by a
+// constant (45 with divisions as such).  Per sweep, 256x128x128: 550 -> 100 us
+// (78 at the FP64 rate); 200x100x100, h = 1/100: 268 -> 116 us (75).
+constexpr int JAC_PLANES = 4;   // planes per thread: one maximum for the block's four tiles
+enum JacForm { JAC_DIV = 0, JAC_POW2 = 1, JAC_EQUAL = 2 };
+
+template <int FORM>
+__global__ void k_jacobi_sweep(Geo g, DivBy dx2, DivBy dy2, DivBy dz2, DivBy denom, const double* __restrict__ cur,
+                               double* __restrict__ nxt, const double* __restrict__ rhs, unsigned long long* maxdp,
+                               SolverState* st, int sweep, int cur_buf)
 {
-    __shared__ double sm[32];
-    __shared__ int am_last;
+    __shared__ unsigned long long sm[TBJ];
+    const bool first = blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && threadIdx.x == 0 && threadIdx.y == 0;
     if (st->done) return;
-    int i, j, k;
-    double m = 0.0;
-    if (cell_coords(g, i, j, k) && i >= 1 && i <= g.nx - 2 && j >= 1 && j <= g.ny - 2 && k >= 1 &&
-        k <= g.nz - 2) {
-        const int id = i * g.si + j * g.sj + k;
-        double p_old = cur[id];
-        double v = ((cur[id + g.si] + cur[id - g.si]) / dx2 + (cur[id + g.sj] + cur[id - g.sj]) / dy2 +
-                    (cur[id + 1] + cur[id - 1]) / dz2 - rhs[id]) /
-                   denom;
-        nxt[id] = v;
-        m = fabs(v - p_old);
+    if (sweep > 0 && __longlong_as_double((long long)maxdp[(sweep + 2) % 3]) < st->tol) {
+        if (first) {   // the sweep before met the tolerance
+            st->iters = st->k = sweep;
+            st->buf = cur_buf;
+            st->status = LES_OK;
+            st->done = 1;
+        }
+        return;
     }
-    const int tid = threadIdx.x + blockDim.x * threadIdx.y, lane = tid & 31, warp = tid >> 5;
-    m = warp_max(m);
-    if (lane == 0) sm[warp] = m;
-    __syncthreads();
-    const int nw = (blockDim.x * blockDim.y) >> 5, nb = block_count(), bid = block_linear_id();
-    if (tid == 0) {
-        double a = 0.0;
-        for (int q = 0; q < nw; ++q) a = fmax(a, sm[q]);
-        partials[bid] = a;
-        __threadfence();
-        am_last = atomicAdd(counter, 1u) == (unsigned)nb - 1u;
+    if (first) maxdp[(sweep + 1) % 3] = 0ull;
+    const int k = blockIdx.x * TBK + threadIdx.x, j = blockIdx.y * TBJ + threadIdx.y;
+    unsigned long long m = 0ull;
+    if (j >= 1 && j <= g.ny - 2 && k >= 1 && k <= g.nz - 2) {
+        const int i0 = max(1, (int)blockIdx.z * JAC_PLANES), i1 = min(g.nx - 1, ((int)blockIdx.z + 1) * JAC_PLANES);
+        const bool edge = j == 1 || j == g.ny - 2 || k == 1 || k == g.nz - 2;
+        int id = i0 * g.si + j * g.sj + k;
+        double pw = i0 < i1 ? cur[id - g.si] : 0.0, pc = i0 < i1 ? cur[id] : 0.0;
+        for (int i = i0; i < i1; ++i, id += g.si) {
+            const double pe = cur[id + g.si];
+            const double ew = pe + pw, ns = cur[id + g.sj] + cur[id - g.sj], tb = cur[id + 1] + cur[id - 1];
+            double x;
+            if (FORM == JAC_EQUAL) x = fma((ew + ns) + tb, dx2.y, -rhs[id]);
+            else if (FORM == JAC_POW2) x = fma(tb, dz2.y, fma(ns, dy2.y, ew * dx2.y)) - rhs[id];
+            else x = ((div_by(ew, dx2) + div_by(ns, dy2)) + div_by(tb, dz2)) - rhs[id];
+            const double v = div_by(x, denom);
+            nxt[id] = v;
+            if (edge || i == 1 || i == g.nx - 2) {
+                const int js[3] = {j, j == 1 ? 0 : -1, j == g.ny - 2 ? g.ny - 1 : -1};
+                const int ks[3] = {k, k == 1 ? 0 : -1, k == g.nz - 2 ? g.nz - 1 : -1};
+                for (int a = 0; a < 3; ++a)
+                    for (int b = 0; b < 3; ++b) {
+                        if (js[a] < 0 || ks[b] < 0) continue;
+                        const int c = js[a] * g.sj + ks[b];
+                        if (a || b) nxt[i * g.si + c] = v;
+                        if (i == 1) nxt[c] = v;
+                        if (i == g.nx - 2) nxt[(g.nx - 1) * g.si + c] = 0.0;
+                    }
+            }
+            const unsigned long long r = (unsigned long long)__double_as_longlong(fabs(v - pc));
+            if (r > m && r <= 0x7ff0000000000000ull) m = r;
+            pw = pc;
+            pc = pe;
+        }
     }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const unsigned long long t = __shfl_xor_sync(0xffffffffu, m, o);
+        m = t > m ? t : m;
+    }
+    if (threadIdx.x == 0) sm[threadIdx.y] = m;
     __syncthreads();
-    if (!am_last) return;
-    __threadfence();
-    double a = 0.0;
-    for (int q = tid; q < nb; q += blockDim.x * blockDim.y) a = fmax(a, __ldcg(partials + q));
-    a = warp_max(a);
-    __syncthreads();
-    if (lane == 0) sm[warp] = a;
-    __syncthreads();
-    if (tid == 0) {
-        double r = 0.0;
-        for (int q = 0; q < nw; ++q) r = fmax(r, sm[q]);
-        st->maxdp = r;
-        *counter = 0u;
+    if (threadIdx.x == 0 && threadIdx.y == 0) {
+        for (int q = 1; q < TBJ; ++q) m = sm[q] > m ? sm[q] : m;
+        if (m) atomicMax(maxdp + sweep % 3, m);
     }
 }
 
-// After the BCs of a sweep: count it and test max|dp| < tol (:164-170).
-__global__ void k_stat_check(SolverState* st, int sweep_buf)
+// The test of the last sweep launched so far.
+__global__ void k_jacobi_test(SolverState* st, const unsigned long long* maxdp, int sweeps, int buf)
 {
     if (st->done) return;
-    st->k += 1;
-    st->buf = sweep_buf;
-    if (st->maxdp < st->tol) { st->done = 1; st->iters = st->k; st->status = LES_OK; }
-    else if (st->k >= st->max_iter) { st->done = 1; st->iters = st->k; st->status = LES_NOT_CONVERGED; }
-}
-
-__global__ void k_pbc_faces_guarded(Geo g, const double* in, double* out, SolverState* st)
-{
-    if (st->done) return;
-    int i, j, k;
-    if (!cell_coords(g, i, j, k)) return;
-    bool jk_in = j >= 1 && j <= g.ny - 2 && k >= 1 && k <= g.nz - 2;
-    if (jk_in && i > 0 && i < g.nx - 1) return;
-    const int id = i * g.si + j * g.sj + k;
-    if (i == g.nx - 1) { out[id] = 0.0; return; }
-    int jj = j < 1 ? 1 : (j > g.ny - 2 ? g.ny - 2 : j);
-    int kk = k < 1 ? 1 : (k > g.nz - 2 ? g.nz - 2 : k);
-    int ii = i == 0 ? 1 : i;
-    out[id] = in[ii * g.si + jj * g.sj + kk];
+    st->k = sweeps;
+    st->buf = buf;
+    if (__longlong_as_double((long long)maxdp[(sweeps + 2) % 3]) < st->tol) {
+        st->iters = sweeps;
+        st->status = LES_OK;
+        st->done = 1;
+    } else if (sweeps >= st->max_iter) {
+        st->iters = sweeps;
+        st->status = LES_NOT_CONVERGED;
+        st->done = 1;
+    }
 }
 
 __global__ void k_pbc_obstacle_guarded(Geo g, const int* __restrict__ list, int n,
@@ -859,28 +880,36 @@ les_status solve_jacobi_dev(les_ctx* c, double dt, double rho, int max_iter, dou
     double* bufs[2] = {c->slot[LES_P], c->w[1]};
     const double dx2 = m.dx * m.dx, dy2 = m.dy * m.dy, dz2 = m.dz * m.dz;
     const double denom = 2 * (1.0 / dx2 + 1.0 / dy2 + 1.0 / dz2);
-    launch(c, k_stat_rhs, gr, bl, g, rho / dt, 2 * m.dx, 2 * m.dy, 2 * m.dz, c->slot[LES_U],
-                                         c->slot[LES_V], c->slot[LES_W], rhs);
+    launch(c, k_stat_rhs, gr, bl, g, rho / dt, div_by_const(2 * m.dx), div_by_const(2 * m.dy), div_by_const(2 * m.dz),
+           (const double*)c->slot[LES_U], (const double*)c->slot[LES_V], (const double*)c->slot[LES_W], rhs);
     launch(c, k_init_state, 1, 1, c->state, tol, max_iter, 0);
-    int launched = 0, batch = 8;
+    unsigned long long* const maxdp = reinterpret_cast<unsigned long long*>(c->partials);
+    st = check_cuda(c, cudaMemsetAsync(maxdp, 0, 3 * sizeof *maxdp, c->stream), "memset");
+    if (st) return st;
+    // x / d for a power of two d is exactly x * (1 / d)
+    auto pow2 = [](double v) { int e; return std::frexp(v, &e) == 0.5; };
+    const bool p2 = pow2(dx2) && pow2(dy2) && pow2(dz2);
+    auto sweep = !p2 ? k_jacobi_sweep<JAC_DIV>
+                     : (dx2 == dy2 && dy2 == dz2 ? k_jacobi_sweep<JAC_EQUAL> : k_jacobi_sweep<JAC_POW2>);
+    const dim3 gs(gr.x, gr.y, (g.nx + JAC_PLANES - 1) / JAC_PLANES);
+    int launched = 0, batch = 16;
     int cur = 0;
-    for (;;) {
+    while (launched < max_iter) {
         for (int it = 0; it < batch && launched < max_iter; ++it, ++launched) {
-            launch(c, k_jacobi_sweep, gr, bl, g, dx2, dy2, dz2, denom, bufs[cur], bufs[cur ^ 1], rhs,
-                                                     c->partials, c->counters + 6, c->state);
+            launch(c, sweep, gs, bl, g, div_by_const(dx2), div_by_const(dy2), div_by_const(dz2), div_by_const(denom),
+                   (const double*)bufs[cur], bufs[cur ^ 1], (const double*)rhs, maxdp, c->state, launched, cur);
             cur ^= 1;
-            launch(c, k_pbc_faces_guarded, gr, bl, g, bufs[cur], bufs[cur], c->state);
             if (c->n_solid)
-                launch(c, k_pbc_obstacle_guarded, (c->n_solid + 255) / 256, 256, 
-                    g, c->solid_list, c->n_solid, c->mask, bufs[cur], c->state);
-            launch(c, k_stat_check, 1, 1, c->state, cur);
+                launch(c, k_pbc_obstacle_guarded, (c->n_solid + 255) / 256, 256, g, (const int*)c->solid_list,
+                       c->n_solid, (const uint8_t*)c->mask, bufs[cur], c->state);
         }
+        launch(c, k_jacobi_test, 1, 1, c->state, (const unsigned long long*)maxdp, launched, cur);
         st = check_launch(c, "jacobi sweeps");
         if (st) return st;
         st = read_state(c);
         if (st) return st;
-        if (c->h_state->done || launched >= max_iter) break;
-        batch = 16;
+        if (c->h_state->done) break;
+        batch = 32;
     }
     if (max_iter <= 0) {
         if (sweeps) *sweeps = 0;
