@@ -25,6 +25,7 @@ UNITS = {
     "les_physics.cu": ["-fmad=false"],
     "les_physics32.cu": [],
     "les_pressure.cu": ["-fmad=false"],
+    "les_coop64.cu": ["-fmad=false"],
     "les_wavefront.cu": ["-fmad=false"],
     "les_mixed.cu": [],
     "les_fused.cu": [],

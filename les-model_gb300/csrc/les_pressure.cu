@@ -24,6 +24,8 @@ les_status ic_apply_dev(les_ctx* c, const double* r, double* z, const double* co
 les_status wave_check(les_ctx* c);
 les_status build_ic_dev(les_ctx* c);
 les_status pcg_mixed(les_ctx* c, const les_pcg_opts* o, les_pcg_result* res);
+bool pcg64_coop_used(const les_ctx* c, const les_pcg_opts* o);   // les_coop64.cu
+les_status pcg64_coop(les_ctx* c, const les_pcg_opts* o, bool pow2, int keep_tol);
 }
 
 namespace {
@@ -811,6 +813,18 @@ les_status pcg_fp64(les_ctx* c, const les_pcg_opts* o, les_pcg_result* res, int 
     if (o->precond == LES_PC_IC_A) {
         st = ensure_stored_A(c);
         if (st) return st;
+    }
+    if (pcg64_coop_used(c, o)) {
+        if ((st = pcg64_coop(c, o, row_form(c) == ROW_POW2, keep_tol))) return st;
+        if ((st = wave_check(c))) return st;   // the exchanges' bounded waits
+        if ((st = read_state(c))) return st;
+        const SolverState& h = *c->h_state;
+        if (res) {
+            res->iters = h.iters;
+            res->outer = 0;
+            res->residual = h.err;
+        }
+        return (les_status)h.status;
     }
     StencilView A = stencil_view(c);
     double *x = c->slot[LES_P], *b = c->slot[LES_B];
