@@ -241,6 +241,157 @@ __device__ __forceinline__ void zero_pads(Vec& v, const TilePos& t)
     }
 }
 
+// ---- the heads -------------------------------------------------------------------
+// The deferred sums and decisions of head_a / head_b (les_col_march.cuh) for a
+// few hundred partials at most, with nothing on the FP64 pipe where a
+// dependent operation takes 64 cycles and more: the sums stay (hi, lo) pairs,
+// quotients are formed from pairs on the FP32 pipe, and the root of ||r||^2 is
+// taken once, at the end of a solve.  The partials and the state are read
+// together.  64x32x32: 12.6 -> 11.5 us per iteration, 128x64x64:
+// 16.4 -> 15.0, 256x128x128: 40.1 -> 38.7.
+
+// num / den to FP32 precision from pairs
+__device__ __forceinline__ float df_quotient(const Acc& n, const Acc& d)
+{
+    const float q = __fdiv_rn(n.hi, d.hi);
+    const float r = __fadd_rn(fmaf(-q, d.hi, n.hi), fmaf(-q, d.lo, n.lo));
+    return fmaf(r, __frcp_rn(d.hi), q);
+}
+
+// Sums NV vectors of nb partials, the totals in thread 0.
+template <int NV>
+__device__ __forceinline__ void head_sum(const float2* __restrict__ part, int nb, Acc (&v)[NV], float2* sm)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int nw = min((int)blockDim.x, (nb + 31) & ~31) >> 5;   // warps that hold partials
+    if (warp < nw) {
+        for (int b = threadIdx.x; b < nb; b += blockDim.x)
+#pragma unroll
+            for (int q = 0; q < NV; ++q) {
+                const float2 t = __ldcg(part + q * nb + b);
+                Acc x;
+                x.hi = t.x;
+                x.lo = t.y;
+                v[q] = df_add(v[q], x);
+            }
+#pragma unroll
+        for (int q = 0; q < NV; ++q)
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                Acc t;
+                t.hi = __shfl_down_sync(FULL, v[q].hi, o);
+                t.lo = __shfl_down_sync(FULL, v[q].lo, o);
+                v[q] = df_add(v[q], t);
+            }
+        if (lane == 0)
+#pragma unroll
+            for (int q = 0; q < NV; ++q) sm[q * 16 + warp] = make_float2(v[q].hi, v[q].lo);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0)
+        for (int w = 1; w < nw; ++w)
+#pragma unroll
+            for (int q = 0; q < NV; ++q) {
+                Acc x;
+                x.hi = sm[q * 16 + w].x;
+                x.lo = sm[q * 16 + w].y;
+                v[q] = df_add(v[q], x);
+            }
+}
+
+// The inner state's fields that the plane passes hand to each other in pairs
+// lie in the double fields: rho, rho_next (bit patterns of float2).
+__device__ __forceinline__ Acc get_pair(const double* f)
+{
+    const float2 t = __ldcg(reinterpret_cast<const float2*>(f));
+    Acc a;
+    a.hi = t.x;
+    a.lo = t.y;
+    return a;
+}
+__device__ __forceinline__ void put_pair(double* f, const Acc& a) { *reinterpret_cast<float2*>(f) = make_float2(a.hi, a.lo); }
+
+// Pass A: pass B's sums ||r'||^2 and r'.z, the convergence test, beta.
+template <bool FIRST>
+__device__ __noinline__ HeadOut plane_head_a(const float2* __restrict__ pin, int nb_in, SolverState* st,
+                                             SolverState* outer, int total_cap, int pslot, int blk)
+{
+    __shared__ float2 sm[32];
+    __shared__ HeadOut so;
+    Acc v[2], rho_old;
+    double tol = 0.0;
+    int done = 0, kk = 0, total = 0, max_iter = 0, frozen = 0;
+    if (threadIdx.x == 0) {
+        done = __ldcg(&st->done);
+        if (!FIRST) {
+            rho_old = get_pair(&st->rho);
+            tol = __ldcg(&st->tol);
+            kk = __ldcg(&st->k);   // committed by pass B
+            total = __ldcg(&outer->iters);
+            max_iter = __ldcg(&st->max_iter);
+            frozen = __ldcg(&st->frozen);
+        }
+    }
+    head_sum<2>(pin, nb_in, v, sm);
+    if (threadIdx.x == 0) {
+        const bool w0 = blk == 0;
+        so.end = 1;
+        if (!done) {
+            int status = -1;
+            so.coef = 0.f;
+            if (!FIRST) {
+                const double rr = (double)v[0].hi + (double)v[0].lo;
+                if (rr < tol * tol) status = tol > 0.0 ? LES_OK : -1;
+                else if (!(rr < 1.7976931348623157e308)) status = LES_NONFINITE;
+                if (status < 0 && (kk >= max_iter || total >= total_cap)) status = LES_NOT_CONVERGED;
+                if (frozen) status = -1;
+                so.coef = frozen ? 0.f : df_quotient(v[1], rho_old);
+            }
+            if (w0) {
+                if (status >= 0) {   // the solve ends at iteration kk: the final state
+                    st->err = sqrt((double)v[0].hi + (double)v[0].lo);
+                    st->status = status;
+                    st->done = 1;
+                } else {
+                    put_pair(&st->rho_next, v[1]);
+                    st->buf = pslot;   // buffer holding this iteration's p
+                }
+            }
+            so.end = status >= 0;   // no work after the last iteration
+        }
+    }
+    __syncthreads();
+    return so;
+}
+
+// Pass B: pass A's sum p.q, alpha and the commit of the iteration.
+__device__ __noinline__ HeadOut plane_head_b(const float2* __restrict__ pin, int nb_in, SolverState* st,
+                                             SolverState* outer, int blk)
+{
+    __shared__ float2 sm[16];
+    __shared__ HeadOut so;
+    Acc v[1], rho;
+    int done = 0, frozen = 0;
+    if (threadIdx.x == 0) {
+        done = __ldcg(&st->done);
+        rho = get_pair(&st->rho_next);
+        frozen = __ldcg(&st->frozen);
+    }
+    head_sum<1>(pin, nb_in, v, sm);
+    if (threadIdx.x == 0) {
+        so.end = done;
+        so.coef = frozen ? 0.f : df_quotient(rho, v[0]);
+        if (blk == 0 && !done) {
+            st->alpha = (double)so.coef;
+            put_pair(&st->rho, rho);
+            st->k = st->k + 1;
+            outer->iters = outer->iters + 1;
+        }
+    }
+    __syncthreads();
+    return so;
+}
+
 // ---- pass A -----------------------------------------------------------------
 // p = z + beta p_old, e += alpha_prev p_old, q = A p, p.q (les_col.cu).
 template <int TMAX, int FORM, bool FIRST>
@@ -268,7 +419,7 @@ __device__ __forceinline__ void plane_a(const PlaneArgsA& a, int blk, int nblk)
     };
     dep_wait();
     fetch(is);   // on its way while the head sums
-    const HeadOut h = head_a<FIRST>(a.df.pin, a.df.nb_in, a.st, a.outer, a.total_cap, a.pslot, blk);
+    const HeadOut h = plane_head_a<FIRST>(a.df.pin, a.df.nb_in, a.st, a.outer, a.total_cap, a.pslot, blk);
     if (h.end) return;
     const float beta = h.coef, aprev = FIRST ? 0.f : (float)a.st->alpha;
     Acc acc;
@@ -492,7 +643,7 @@ __device__ __forceinline__ void plane_b(const PlaneArgsB& a, int blk, int nblk)
     fetch(is);   // on its way while the head sums
     float alpha = 0.f;
     if (!FIRST) {   // pass A's sum, alpha and the commit of the iteration
-        const HeadOut h = head_b<true>(a.df.pin, a.df.nb_in, a.st, a.outer, blk);
+        const HeadOut h = plane_head_b(a.df.pin, a.df.nb_in, a.st, a.outer, blk);
         if (h.end) return;
         alpha = h.coef;
     } else if (a.st->done) {
@@ -524,7 +675,7 @@ __device__ __forceinline__ void plane_b0(const PlaneArgsB& a, int blk, int nblk)
     dep_wait();
     float alpha = 0.f;
     if (!FIRST) {
-        const HeadOut h = head_b<true>(a.df.pin, a.df.nb_in, a.st, a.outer, blk);
+        const HeadOut h = plane_head_b(a.df.pin, a.df.nb_in, a.st, a.outer, blk);
         if (h.end) return;
         alpha = h.coef;
     } else if (a.st->done) {
