@@ -211,7 +211,6 @@ void les_destroy(les_ctx* c)
     for (auto& p : c->w) cudaFree(p);
     for (auto& p : c->f) cudaFree(p);
     for (auto& p : c->A32) cudaFree(p);
-    for (auto& p : c->L32) cudaFree(p);
     cudaFree(c->mask);
     cudaFree(c->solid_list);
     cudaFree(c->code);
@@ -221,7 +220,7 @@ void les_destroy(les_ctx* c)
     cudaFree(c->state);
     cudaFree(c->gsync);
     cudaFree(c->wave_prog);
-    cudaFree(c->gs_buf);
+    cudaFree(c->skew_buf);
     if (c->h_state) cudaFreeHost(c->h_state);
     for (auto& e : c->prof_ev) cudaEventDestroy(e);
     for (auto& e : c->marks) cudaEventDestroy(e);

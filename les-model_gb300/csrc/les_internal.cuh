@@ -337,10 +337,9 @@ struct les_ctx {
     // work vectors (FP64)
     double* w[8] = {};
     // FP32 work vectors for the mixed-precision inner solve, and FP32 copies
-    // of a stored A / of the IC factor for it
+    // of a stored A for it
     float* f[8] = {};
     float* A32[7] = {};
-    float* L32[7] = {};
     // reductions / state
     double* partials = nullptr;
     size_t partials_len = 0;
@@ -354,8 +353,8 @@ struct les_ctx {
     int* wave_prog = nullptr;
     int wave_prog_len = 0;
     int wave_epoch = 0;
-    double* gs_buf = nullptr;     // GS-SOR's skewed arrays
-    size_t gs_len = 0;
+    double* skew_buf = nullptr;   // skewed arrays (les_wavefront.cu): GS-SOR's vectors, the IC records
+    size_t skew_len = 0;
     std::string err;
     // accounting: kernel launches issued by this context, and optional CUDA
     // event timing of the solver's hot kernels (les_profile)

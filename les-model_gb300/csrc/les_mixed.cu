@@ -30,7 +30,8 @@ using namespace les;
 
 namespace les {
 les_status ensure_stored_A(les_ctx* c);
-les_status ic_apply_dev32(les_ctx* c, const float* r, float* z, const float* const* L32, SolverState* st);
+les_status ic_records32(les_ctx* c, const double* const* L);
+les_status ic_apply_dev32(les_ctx* c, const float* r, float* z, SolverState* st);
 les_status wave_check(les_ctx* c);
 }
 
@@ -366,7 +367,7 @@ namespace les {
 // Preconditioner in FP32 inside the inner loop: r -> z.  mode 0 Jacobi (fused
 // in k_in_update), 1 Chebyshev, 2 IC (L or A).
 static les_status inner_precond(les_ctx* c, const les_pcg_opts* o, ViewF A, float* r, float* z, SolverState* in,
-                                const float* const* L32, int skip_done, int init)
+                                int skip_done, int init)
 {
     const Geo& g = c->g;
     const dim3 gr = cell_grid(g), bl = cell_block();
@@ -392,7 +393,7 @@ static les_status inner_precond(les_ctx* c, const les_pcg_opts* o, ViewF A, floa
         return check_launch(c, "inner chebyshev");
     }
     // IC: wavefront solve in FP32, then r.z
-    les_status st = ic_apply_dev32(c, r, z, L32, skip_done ? in : nullptr);
+    les_status st = ic_apply_dev32(c, r, z, skip_done ? in : nullptr);
     if (st) return st;
     launch(c, k_in_dot_beta, gr, bl, g, r, z, c->partials, c->counters + 13, in, init);
     return check_launch(c, "inner ic");
@@ -410,19 +411,11 @@ les_status pcg_mixed_impl(les_ctx* c, const les_pcg_opts* o, les_pcg_result* res
         st = ensure_f32_copy(c, c->A32, c->A);
         if (st) return st;
     }
-    const float* L32[7] = {};
-    if (o->precond == LES_PC_IC || o->precond == LES_PC_IC_A) {
+    if (o->precond == LES_PC_IC || o->precond == LES_PC_IC_A) {   // the factor, laid out for the FP32 applies
         if (o->precond == LES_PC_IC && !c->have_L) return fail(c, LES_BAD_ARG, "IC preconditioner needs a factor");
-        if (o->precond == LES_PC_IC_A) {
-            st = ensure_stored_A(c);
-            if (st) return st;
-        }
-        double* src[7] = {};
-        double* const* from = (o->precond == LES_PC_IC) ? c->L : c->A;
-        src[0] = from[0]; src[2] = from[2]; src[4] = from[4]; src[6] = from[6];
-        st = ensure_f32_copy(c, c->L32, src);
+        if (o->precond == LES_PC_IC_A && (st = ensure_stored_A(c))) return st;
+        st = ic_records32(c, (const double* const*)(o->precond == LES_PC_IC ? c->L : c->A));
         if (st) return st;
-        for (int q = 0; q < 7; ++q) L32[q] = c->L32[q];
     }
     const int mode = o->precond == LES_PC_JACOBI ? 0 : (o->precond == LES_PC_CHEBYSHEV ? 1 : 2);
     ViewF A32 = view32(c);
@@ -454,13 +447,13 @@ les_status pcg_mixed_impl(les_ctx* c, const les_pcg_opts* o, les_pcg_result* res
             if (st) return st;
         } else if (mode == 2) {
             launch(c, k_zero_f, gr, bl, g, e);
-            st = inner_precond(c, o, A32, r, z, in, L32, 0, 1);
+            st = inner_precond(c, o, A32, r, z, in, 0, 1);
         } else {
             // Chebyshev: the first z must land where the recurrence expects it
             int steps = o->degree - 1;
             float* z0 = (mode == 1 && steps % 2 == 1) ? c->f[6] : z;
             launch(c, k_in_pc0, gr, bl, g, A32, mode, alpha0, r, z0, e, c->partials, c->counters + 9, in);
-            if (mode == 1 && steps > 0) st = inner_precond(c, o, A32, r, z, in, L32, 0, 1);
+            if (mode == 1 && steps > 0) st = inner_precond(c, o, A32, r, z, in, 0, 1);
         }
         if (st) return st;
         int cur = 0, launched = 0, batch = 4;
@@ -474,12 +467,12 @@ les_status pcg_mixed_impl(les_ctx* c, const les_pcg_opts* o, les_pcg_result* res
                     float* z0 = (steps % 2 == 1) ? c->f[6] : z;
                     launch_p(c, PROF_IN_UPDATE, k_in_update, gr, bl, g, A32, mode, alpha0, e, r, pb[cur], q, z0, c->partials,
                                                           c->counters + 11, in, out, o->max_iter);
-                    if (steps > 0) st = inner_precond(c, o, A32, r, z, in, L32, 1, 0);
+                    if (steps > 0) st = inner_precond(c, o, A32, r, z, in, 1, 0);
                     else launch(c, k_in_dot_beta, gr, bl, g, r, z, c->partials, c->counters + 13, in, 0);
                 } else {
                     launch_p(c, PROF_IN_UPDATE, k_in_update, gr, bl, g, A32, mode, alpha0, e, r, pb[cur], q, z, c->partials,
                                                           c->counters + 11, in, out, o->max_iter);
-                    if (mode == 2) st = inner_precond(c, o, A32, r, z, in, L32, 1, 0);
+                    if (mode == 2) st = inner_precond(c, o, A32, r, z, in, 1, 0);
                 }
                 if (st) return st;
             }

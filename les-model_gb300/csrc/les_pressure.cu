@@ -20,7 +20,8 @@
 using namespace les;
 
 namespace les {
-les_status ic_apply_dev(les_ctx* c, const double* r, double* z, const double* const* Lsrc, int skip_done);
+les_status ic_records64(les_ctx* c, const double* const* L);
+les_status ic_apply_dev(les_ctx* c, const double* r, double* z, int skip_done);
 les_status wave_check(les_ctx* c);
 les_status build_ic_dev(les_ctx* c);
 les_status pcg_mixed(les_ctx* c, const les_pcg_opts* o, les_pcg_result* res);
@@ -757,16 +758,9 @@ static les_status precond_dot(les_ctx* c, const les_pcg_opts* o, const double* r
         break;
     }
     case LES_PC_IC:
-        if (!c->have_L) return fail(c, LES_BAD_ARG, "IC preconditioner needs les_build_ic or les_set_ic_factor");
-        st = ic_apply_dev(c, r, z, nullptr, skip_done);
+    case LES_PC_IC_A:
+        st = ic_apply_dev(c, r, z, skip_done);   // with the records of ic_ready
         break;
-    case LES_PC_IC_A: {
-        // the factor arrays are A itself (src/pressure.cpp:363, :396)
-        if (!c->A_valid) return fail(c, LES_BAD_ARG, "internal: IC-with-A needs A as arrays");
-        const double* Ad[7] = {c->A[0], c->A[1], c->A[2], c->A[3], c->A[4], c->A[5], c->A[6]};
-        st = ic_apply_dev(c, r, z, Ad, skip_done);
-        break;
-    }
     default:
         return fail(c, LES_BAD_ARG, "unknown preconditioner");
     }
@@ -776,11 +770,6 @@ static les_status precond_dot(les_ctx* c, const les_pcg_opts* o, const double* r
         st = check_launch(c, "r.z");
     }
     return st;
-}
-
-les_status precond_dev(les_ctx* c, const les_pcg_opts* o, const double* r, double* z, int skip_done)
-{
-    return precond_dot(c, o, r, z, skip_done, RD_NONE, false);
 }
 
 // The IC-with-A mode needs A as arrays; expand the coded matrix on demand.
@@ -801,6 +790,25 @@ les_status ensure_stored_A(les_ctx* c)
     return check_launch(c, "expand stencil");
 }
 
+// Lays out the factor of an IC preconditioner for the applies that follow.
+static les_status ic_ready(les_ctx* c, const les_pcg_opts* o)
+{
+    if (o->precond == LES_PC_IC) {
+        if (!c->have_L) return fail(c, LES_BAD_ARG, "IC preconditioner needs les_build_ic or les_set_ic_factor");
+        return ic_records64(c, (const double* const*)c->L);
+    }
+    if (o->precond == LES_PC_IC_A) {   // the factor arrays are A itself (src/pressure.cpp:363, :396)
+        les_status st = ensure_stored_A(c);
+        return st ? st : ic_records64(c, (const double* const*)c->A);
+    }
+    return LES_OK;
+}
+
+les_status precond_dev(les_ctx* c, const les_pcg_opts* o, const double* r, double* z, int skip_done)
+{
+    return precond_dot(c, o, r, z, skip_done, RD_NONE, false);
+}
+
 // PCG of src/pressure.cpp:342-414 in FP64 with the solution in P and the
 // right-hand side in B.  The loop runs on the device; the host only polls
 // the state between batches of iterations (kernels after convergence exit
@@ -810,10 +818,7 @@ les_status pcg_fp64(les_ctx* c, const les_pcg_opts* o, les_pcg_result* res, int 
     const Geo& g = c->g;
     les_status st = ensure_work(c);
     if (st) return st;
-    if (o->precond == LES_PC_IC_A) {
-        st = ensure_stored_A(c);
-        if (st) return st;
-    }
+    if ((st = ic_ready(c, o))) return st;
     if (pcg64_coop_used(c, o)) {
         if ((st = pcg64_coop(c, o, row_form(c) == ROW_POW2, keep_tol))) return st;
         if ((st = wave_check(c))) return st;   // the exchanges' bounded waits
@@ -1048,11 +1053,8 @@ les_status les_precond_apply(les_ctx* c, const les_pcg_opts* o, int in, int out)
     if (!c || !o || in < 0 || in >= LES_NSLOTS || out < 0 || out >= LES_NSLOTS || in == out) return LES_BAD_ARG;
     cudaSetDevice(c->device);
     if (!c->stencil_mode && o->precond != LES_PC_IC) return fail(c, LES_BAD_ARG, "no matrix");
-    if (o->precond == LES_PC_IC_A) {
-        les_status st = ensure_stored_A(c);
-        if (st) return st;
-    }
-    les_status st = precond_dev(c, o, c->slot[in], c->slot[out], 0);
+    les_status st = ic_ready(c, o);
+    if (!st) st = precond_dev(c, o, c->slot[in], c->slot[out], 0);
     if (!st && (o->precond == LES_PC_IC || o->precond == LES_PC_IC_A))
         st = wave_check(c);   // waits for the wavefront: LES_TIMEOUT if a bounded wait gave up
     return st;

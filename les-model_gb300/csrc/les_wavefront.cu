@@ -11,22 +11,22 @@
 //
 // The substitution and the SOR sweep run as a pipelined wavefront with no
 // grid barrier inside a sweep.  The (j, k) plane is cut into tiles of TJ rows
-// by 32 columns; a block of TJ warps owns a tile and marches along i, warp w
-// on the tile's row w and lane l on column l, working at block step tau on
-// plane tau - l - w (lanes and warps skewed by one plane each).  So the k-1
+// by 32 columns; TJ warps of a block own a tile and march along i, warp w on
+// the tile's row w and lane l on column l, working at block step tau on plane
+// tau - l - w (lanes and warps skewed by one plane each).  So the k-1
 // neighbour of a cell is the previous lane's result of the step before (a
 // warp shuffle), the j-1 neighbour the previous warp's result of the step
-// before (shared memory, one block barrier per step), and the i-1 neighbour
-// the thread's own result of the step before.  The rows of a tile run on the
+// before (shared memory, one barrier per step), and the i-1 neighbour the
+// thread's own result of the step before.  The rows of a tile run on the
 // SM's four sub-partitions at once: a single warp would push all of them
 // through one sub-partition's FP64 unit.  Only a tile's first row and first
 // lane need other tiles' values: the tile below in j and the tile before in
-// k publish their progress (steps completed, one counter per tile, release
-// store after a fence) every WB steps, and a block waits (acquire load,
-// bounded by %globaltimer) for the progress its next WB steps need, then
-// reads those neighbours through L2.  The backward solve mirrors every
-// direction.  Tiles are handed out to the resident blocks in an order in
-// which each tile's producers come first, so the waits always end.
+// k publish their progress (steps completed, one counter per tile, a release
+// store) every few steps, and a block waits (acquire load, bounded by
+// %globaltimer) for the progress its next steps need, then reads those
+// neighbours through L2.  The backward solve mirrors every direction.  Tiles
+// are handed out to the resident blocks in an order in which each tile's
+// producers come first, so the waits always end.
 // The IC factorisation (set-up, once) keeps the simpler form: hyperplanes
 // i+j+k = s in order, one grid barrier between them.  Every wait is bounded
 // (about 2 s); a wait that gives up sets an error flag, every warp leaves,
@@ -95,7 +95,7 @@ __global__ void k_ic_build(Plane P, StencilView A, double* Lc, double* Lw, doubl
 #ifndef LES_WAVE_WD
 #define LES_WAVE_WD 8
 #endif
-constexpr int WB = LES_WAVE_WB;        // steps between progress publications
+constexpr int WB = LES_WAVE_WB;        // GS-SOR: steps between progress publications
 constexpr int WAVE_TJ = LES_WAVE_TJ;   // rows per tile = warps per block (one per SM sub-partition)
 constexpr int WT = 32 * WAVE_TJ;
 
@@ -215,128 +215,245 @@ __device__ __forceinline__ void cp_async(void* smem, const void* gmem)
     const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
     asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(s), "l"(gmem), "n"(BYTES) : "memory");
 }
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem)
+{
+    const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s), "l"(gmem) : "memory");
+}
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 __device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-// A tile: rows jb.. of TJ rows (the last tile in j may have fewer) by the 32
-// columns K*32..; warp w works on the tile's row w (in the sweep's order) and
-// lane l on column K*32 + l.  At block step tau, warp w lane l works on plane
-// tau - skew(l) - w (forward planes ascend, backward descend; skew(l) is l
-// forward, 31-l backward), so:
-//   the i-neighbour is the thread's own result of the step before,
-//   the k-neighbour the previous lane's result of the step before (shuffle),
-//   the j-neighbour the previous warp's result of the step before, handed
-//   over in shared memory (double-buffered by step parity, one block barrier
-//   per step); row 0 takes it from the tile before in j.
-template <typename T>
-struct IcStage {
-    T v[WD][5][WAVE_TJ][32];   // rhs (forward r, backward the cell's forward result), Lw, Ls, Lb, Lc
-    T xs[2][WAVE_TJ][32];      // each row's result of the last two steps
-    int flag;
+// Skewed arrays.  The lanes of a warp work on 32 different planes at a time, so
+// in the fields' own layout every lane's value lies in another sector.  A solve
+// therefore runs on copies in the order of the work: element (tile, step, warp,
+// lane) is the cell that this thread works on at that step.
+struct Skew {
+    int wj, steps;
+    __device__ __forceinline__ size_t at(int i, int j, int k) const   // interior coordinates
+    {
+        const int l = k & 31, w = j % WAVE_TJ, t = (k >> 5) * wj + j / WAVE_TJ;
+        return ((size_t)t * steps + (i + l + w)) * WT + w * 32 + l;
+    }
 };
 
-// IC(0) substitution of one tile, src/pressure.cpp:442-482.  DIR > 0: the
-// forward solve L y = r (z = y); DIR < 0: the backward solve L^T z = y.
+// IC(0) substitution, src/pressure.cpp:442-482.
+//
+// Work: a tile has TJ rows (the last in j may have fewer) by 32 columns.  In
+// the forward solve warp w works on row w and lane l on column l, at step tau
+// on plane tau - l - w.  The backward solve is its mirror image: warp w on row
+// TJ-1-w, lanes from the last column, at step tau on the cell of forward step
+// steps-1-tau.  So in both
+//   the i-neighbour is the thread's own result of the step before,
+//   the k-neighbour the adjacent lane's result of the step before (shuffle),
+//   the j-neighbour the previous warp's result of the step before, handed
+//   over in shared memory (double-buffered by step parity, one block barrier
+//   per step); warp 0 takes it from the next tile in j.
+//
+// Data: per tile and step one record of eight values for each of the 128 cells
+//   Lw Ls Lb | Lc 1/Lc | Lw(i+1) Ls(j+1) Lb(k+1)
+// of which the forward solve reads the first five and the backward solve the
+// last five, and the right-hand side, overwritten by the result: 6 KB per step
+// (FP64), contiguous, copied eight steps ahead in 16-byte pieces.  The records
+// are laid out once per solve (ic_records).
+//
+// Roles: four warps compute; a fifth waits for the producers and brings their
+// values into shared memory, up to RING batches ahead, and a sixth publishes
+// the tile's progress.  So a polled round trip, a load through L2 and a fence
+// (about a microsecond each) lengthen the distance between tiles, not each
+// batch of steps.
+//
+// Bound by the chain of a step: nine FP64 operations that hold a sub-partition's
+// unit about 64 cycles each (three for the division with the reciprocal at
+// hand, see div_by, instead of ten or more), the shuffle and the barrier.
+// Apply, 96x64x64: 960 -> 464 us; 256x128x128: 2930 -> 1616 us.
+constexpr int REC = 8;    // values of a record
+constexpr int IWB = 4;    // steps of a batch (1: 498, 2: 477, 4: 464 us for 96x64x64)
+constexpr int RING = 8;   // batches of neighbours' values in flight
+constexpr int IC_THREADS = WT + 64;
+template <typename T>
+struct IcStage {
+    T v[WD][6][WT];                // five factors and the right-hand side
+    T xs[2][WAVE_TJ][32];          // each row's result of the last two steps
+    T zj[RING][IWB][32];            // the row next to warp 0's
+    T zk[RING][IWB][WAVE_TJ];       // the column next to the near lane's
+    volatile int ready, done, fail;   // batches brought in, computed; a wait gave up
+    int go;
+};
+
+// The computing warps' barrier.
+__device__ __forceinline__ void compute_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(WT) : "memory"); }
+
+// One lane waits until *p has reached n; false once `fail` is set (the waits
+// on other blocks are the bounded ones) or after about 4 s.
+__device__ __forceinline__ bool wait_shared(const volatile int* p, int n, const volatile int* fail)
+{
+    unsigned spins = 0;
+    unsigned long long t0 = 0;
+    while (*p < n) {
+        if (*fail) return false;
+        if ((++spins & 1023u) == 0u) {
+            const unsigned long long t = globaltimer_ns();
+            if (t0 == 0) t0 = t;
+            if (t - t0 > 4000000000ull) return false;
+        }
+    }
+    __threadfence_block();
+    return true;
+}
+
+// sum / Lc with y = RN(1/Lc); y = 0 marks an Lc outside the range (see div_by)
+__device__ __forceinline__ double ic_divide(double sum, double lc, double y)
+{
+    const int hi = __double2hiint(sum), e = (hi >> 20) & 0x7ff;
+    const double q = sum * y;
+    if (y != 0.0) {
+        if (e > 1023 - 500 && e < 1023 + 500) return fma(fma(-q, lc, sum), y, q);
+        if (((hi << 1) | __double2loint(sum)) == 0) return q;   // 0 with its sign
+    }
+    return div_slow(sum, lc);
+}
+__device__ __forceinline__ float ic_divide(float sum, float lc, float) { return sum / lc; }
+
 template <typename T, int DIR>
-__device__ bool ic_tile(const Wave& W, int t, int base, const T* __restrict__ Lc, const T* __restrict__ Lw,
-                        const T* __restrict__ Ls, const T* __restrict__ Lb, const T* __restrict__ r, T* z,
-                        IcStage<T>& sg)
+__device__ bool ic_tile(const Wave& W, int t, int base, const T* __restrict__ rec, T* zs, IcStage<T>& sg)
 {
     constexpr unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int J = t % W.wj, K = t / W.wj;
-    const int jb = J * WAVE_TJ, rows = min(WAVE_TJ, W.ny - jb);
-    const int k = K * 32 + lane;
-    const bool kin = k < W.nz;
-    const int kc = min(k, W.nz - 1);                          // every address stays inside the grid
-    const int sk = DIR > 0 ? lane : 31 - lane;
+    const int rows = min(WAVE_TJ, W.ny - J * WAVE_TJ);
     const TileDeps d = tile_deps<DIR>(W, J, K, t);
-    const bool wact = w < rows;                               // this warp's row exists
-    // this warp's grid row (rows past the grid repeat the last one; dropped)
-    const int jr = DIR > 0 ? jb + min(w, rows - 1) : jb + rows - 1 - min(w, rows - 1);
-    const int rb = W.off + jr * W.sj + kc;
-    const bool jin = DIR > 0 ? jr > 0 : jr < W.ny - 1;        // the row has its j-neighbour
-    const bool kbn = DIR > 0 ? k > 0 : k < W.nz - 1;
-    // row 0's neighbour row in the tile before, the near lane's neighbour column
-    const int jn = DIR > 0 ? max(jb - 1, 0) : min(jb + rows, W.ny - 1);
-    const int kn = DIR > 0 ? max(K * 32 - 1, 0) : min(K * 32 + 32, W.nz - 1);
     const int near = DIR > 0 ? 0 : 31;
-    auto plane = [&](int tau, int skew) { return DIR > 0 ? tau - skew - w : W.nx - 1 - (tau - skew - w); };
-    auto clampi = [&](int i) { return min(max(i, 0), W.nx - 1); };
-    // the operands of step tau into slot tau % WD (one commit group per step);
-    // the factors of a missing neighbour are read from the cell and not used
-    auto stage = [&](int tau) {
-        const int i = clampi(plane(tau, sk));
-        const int sl = tau & (WD - 1);
-        const int id = rb + i * W.si;
-        const int ie = DIR > 0 ? 0 : (i < W.nx - 1 ? W.si : 0);
-        const int je = DIR > 0 ? 0 : (jin ? W.sj : 0);
-        const int ke = DIR > 0 ? 0 : (kbn ? 1 : 0);
-        cp_async<sizeof(T)>(&sg.v[sl][0][w][lane], (DIR > 0 ? r : z) + id);
-        cp_async<sizeof(T)>(&sg.v[sl][1][w][lane], Lw + id + ie);
-        cp_async<sizeof(T)>(&sg.v[sl][2][w][lane], Ls + id + je);
-        cp_async<sizeof(T)>(&sg.v[sl][3][w][lane], Lb + id + ke);
-        cp_async<sizeof(T)>(&sg.v[sl][4][w][lane], Lc + id);
-        cp_commit();
-    };
-    Watch watch = watch_producers(W.prog, d, base);
-    T prev = T(0), outp = T(0);
-    sg.xs[0][w][lane] = sg.xs[1][w][lane] = T(0);
+    const size_t tile = (size_t)W.steps * WT, tb = (size_t)t * tile;
+    const int batches = (W.steps + IWB - 1) / IWB;
+    auto fstep = [&](int tau) { return DIR > 0 ? tau : W.steps - 1 - tau; };   // the forward step of the same cells
+    if (threadIdx.x == 0) sg.ready = sg.done = sg.fail = 0;
+    __syncthreads();
+
+    if (w == WAVE_TJ) {   // the neighbours' values
+        Watch watch{nullptr, base, 0, base - (1 << 20)};
+        if (lane == 0 && d.dj >= 0) { watch.p = W.prog + d.dj; watch.ahead = WAVE_TJ - 1; }
+        if (lane == 1 && d.dk >= 0) { watch.p = W.prog + d.dk; watch.ahead = 31; }
+        // row 0 or TJ-1 of the tile next in j; column 0 or 31 of the tile next in k
+        const T* const zj_at = zs + (size_t)(DIR > 0 ? t - 1 : t + 1) * tile + (DIR > 0 ? 32 * (WAVE_TJ - 1) : 0) + lane;
+        const int q0 = lane & (IWB - 1), row0 = (lane / IWB) & (WAVE_TJ - 1);
+        const T* const zk_at = zs + (size_t)(DIR > 0 ? t - W.wj : t + W.wj) * tile + row0 * 32 + (DIR > 0 ? 31 : 0);
+        const int rj = DIR > 0 ? 0 : WAVE_TJ - 1;   // the row that needs the j-neighbour
+        for (int n = 0; n < batches; ++n) {
+            const int tau0 = n * IWB, tend = min(tau0 + IWB, W.steps);
+            bool ok = true;
+            if (watch.p) {
+                const int target = base + min(tend + watch.ahead, W.steps);
+                if (watch.seen - target < 0) ok = wait_progress(watch.p, target, W.err, watch.seen);
+            }
+            if (lane == 2) ok = wait_shared(&sg.done, n - RING + 1, &sg.fail);   // the ring's place is free
+            if (!__all_sync(FULL, ok)) {
+                sg.fail = 1;
+                break;
+            }
+            const int sl = n & (RING - 1);
+            T zj[IWB], zk = T(0);
 #pragma unroll
-    for (int q = 0; q < WD - 1; ++q) stage(q);
-    for (int tau0 = 0; tau0 < W.steps; tau0 += WB) {
-        const int tend = min(tau0 + WB, W.steps);
-        if (!wait_steps(W, watch, tend, &sg.flag)) {
-            cp_wait<0>();
-            return false;
-        }
-        // the batch's cross-tile neighbours through L2 (clamped loads,
-        // selected): row 0's j-neighbour for every step (own column), and the
-        // k-neighbours of this warp's near lane (lane q holds step tau0 + q's)
-        T zj[WB];
+            for (int q = 0; q < IWB; ++q) {
+                const int f = fstep(tau0 + q), i = f - lane - rj;
+                zj[q] = T(0);
+                if (d.dj >= 0 && i >= 0 && i < W.nx)
+                    zj[q] = __ldcg(zj_at + (size_t)(f + (DIR > 0 ? WAVE_TJ - 1 : 1 - WAVE_TJ)) * WT);
+            }
+            {
+                const int f = fstep(tau0 + q0), i = f - near - row0;
+                if (d.dk >= 0 && lane < IWB * WAVE_TJ && i >= 0 && i < W.nx)
+                    zk = __ldcg(zk_at + (size_t)(f + (DIR > 0 ? 31 : -31)) * WT);
+            }
 #pragma unroll
-        for (int q = 0; q < WB; ++q) {
-            const T v = __ldcg(z + W.off + clampi(plane(tau0 + q, sk)) * W.si + jn * W.sj + kc);
-            zj[q] = d.dj >= 0 ? v : T(0);
+            for (int q = 0; q < IWB; ++q) sg.zj[sl][q][lane] = zj[q];
+            if (lane < IWB * WAVE_TJ) sg.zk[sl][q0][row0] = zk;
+            __threadfence_block();
+            __syncwarp();
+            if (lane == 0) sg.ready = n + 1;
         }
-        T zk0;
-        {
-            const T v = __ldcg(z + W.off + clampi(plane(tau0 + (lane & (WB - 1)), 0)) * W.si + jr * W.sj + kn);
-            zk0 = d.dk >= 0 ? v : T(0);
-        }
+    } else if (w == WAVE_TJ + 1) {   // the tile's progress
+        if (lane == 0 && t != W.stall)
+            for (int n = 0; n < batches;) {
+                if (!wait_shared(&sg.done, n + 1, &sg.fail)) break;
+                n = sg.done;   // a release takes longer than a batch: the latest
+                __threadfence_block();
+                st_release(W.prog + t, base + min(n * IWB, W.steps));
+            }
+    } else {
+        const int row = DIR > 0 ? w : WAVE_TJ - 1 - w;
+        const int j = J * WAVE_TJ + row, k = K * 32 + lane, el = row * 32 + lane;
+        const bool cell = row < rows && k < W.nz;
+        const bool jin = DIR > 0 ? j > 0 : j < W.ny - 1, kin = DIR > 0 ? k > 0 : k < W.nz - 1;
+        constexpr int PER = 16 / sizeof(T), NREC = 5 * WT / PER, NALL = 6 * WT / PER;   // 16-byte pieces
+        auto stage = [&](int tau) {
+            if (tau < W.steps) {
+                const int f = fstep(tau), sl = tau & (WD - 1);
+                const T* const r = rec + ((size_t)t * W.steps + f) * (REC * WT) + (DIR > 0 ? 0 : 3 * WT);
+                const T* const z = zs + tb + (size_t)f * WT;
+                T* const to = &sg.v[sl][0][0];
 #pragma unroll
-        for (int q = 0; q < WB; ++q) {
-            const int tau = tau0 + q;
-            if (tau >= tend) break;   // block-uniform
-            stage(tau + WD - 1);      // past the last step: clamped copies, never used
-            cp_wait<WD - 1>();        // step tau's operands are in
-            const int i = plane(tau, sk);
-            const bool act = wact && kin && i >= 0 && i < W.nx;
-            const int sl = tau & (WD - 1);
-            const bool ib = DIR > 0 ? i > 0 : i < W.nx - 1;
-            T zk = DIR > 0 ? __shfl_up_sync(FULL, outp, 1) : __shfl_down_sync(FULL, outp, 1);
-            const T v0 = __shfl_sync(FULL, zk0, q);
-            zk = lane == near ? v0 : zk;
-            const T zjv = w == 0 ? zj[q] : sg.xs[(tau - 1) & 1][w - 1][lane];
-            // :451-463 / :469-481, the terms in the reference's order
-            T sum = sg.v[sl][0][w][lane];
-            T a = sum - sg.v[sl][1][w][lane] * prev;
-            sum = ib ? a : sum;
-            a = sum - sg.v[sl][2][w][lane] * zjv;
-            sum = jin ? a : sum;
-            a = sum - sg.v[sl][3][w][lane] * zk;
-            sum = kbn ? a : sum;
-            const T out = sum / sg.v[sl][4][w][lane];
-            if (act) z[rb + i * W.si] = out;
-            prev = outp = out;
-            sg.xs[tau & 1][w][lane] = out;
-            __syncthreads();          // the next step reads this step's rows
+                for (int c = threadIdx.x; c < NALL; c += WT)
+                    cp_async16(to + c * PER, c < NREC ? r + c * PER : z + (c - NREC) * PER);
+            }
+            cp_commit();
+        };
+        T prev = T(0);
+        sg.xs[0][w][lane] = sg.xs[1][w][lane] = T(0);
+#pragma unroll
+        for (int q = 0; q < WD - 1; ++q) stage(q);
+        cp_wait<WD - 2>();   // step 0
+        compute_barrier();
+        for (int n = 0; n < batches; ++n) {
+            const int tau0 = n * IWB, tend = min(tau0 + IWB, W.steps), nr = n & (RING - 1);
+            if (threadIdx.x == 0) {   // one thread decides, so that the warps leave together
+                sg.go = wait_shared(&sg.ready, n + 1, &sg.fail);
+                if (!sg.go) sg.fail = 1;
+            }
+            compute_barrier();
+            if (!sg.go) break;
+#pragma unroll
+            for (int q = 0; q < IWB; ++q) {
+                const int tau = tau0 + q;
+                if (tau >= tend) break;   // block-uniform
+                stage(tau + WD - 1);
+                const int i = fstep(tau) - lane - row, sl = tau & (WD - 1);
+                const bool act = cell && i >= 0 && i < W.nx;
+                const bool ib = DIR > 0 ? i > 0 : i < W.nx - 1;
+                T zk = DIR > 0 ? __shfl_up_sync(FULL, prev, 1) : __shfl_down_sync(FULL, prev, 1);
+                if (lane == near) zk = sg.zk[nr][q][row];
+                const T zj = w == 0 ? sg.zj[nr][q][lane] : sg.xs[(tau - 1) & 1][w - 1][lane];
+                // :451-463 / :469-481, the terms in the reference's order
+                constexpr int F = DIR > 0 ? 0 : 2, C = DIR > 0 ? 3 : 0;   // the factors', the diagonal's place
+                T sum = sg.v[sl][5][el];
+                T a = sum - sg.v[sl][F][el] * prev;
+                sum = ib ? a : sum;
+                a = sum - sg.v[sl][F + 1][el] * zj;
+                sum = jin ? a : sum;
+                a = sum - sg.v[sl][F + 2][el] * zk;
+                sum = kin ? a : sum;
+                // (the lanes outside the grid hold anything: not through the slow path)
+                T out = T(0);
+                if (act) {
+                    out = ic_divide(sum, sg.v[sl][C][el], sg.v[sl][C + 1][el]);
+                    zs[tb + (size_t)fstep(tau) * WT + el] = out;
+                }
+                prev = out;
+                sg.xs[tau & 1][w][lane] = out;
+                cp_wait<WD - 2>();        // this thread's pieces of the next step are in
+                compute_barrier();        // the next step reads this step's rows and others' pieces
+            }
+            if (threadIdx.x == 0) {
+                __threadfence_block();
+                sg.done = n + 1;
+            }
         }
-        if (t != W.stall) publish(W.prog + t, base + tend);   // block-uniform
+        cp_wait<0>();
     }
-    cp_wait<0>();
-    return true;
+    __syncthreads();
+    const bool good = sg.fail == 0;
+    __syncthreads();   // the next tile clears it
+    return good;
 }
 
 // apply_ic_preconditioner, src/pressure.cpp:442-482: the forward solve over
@@ -344,19 +461,52 @@ __device__ bool ic_tile(const Wave& W, int t, int base, const T* __restrict__ Lc
 // reference's arithmetic; T = float serves the FP32 inner solve of the
 // mixed-precision path (st == nullptr: never skipped).
 template <typename T>
-__global__ void __launch_bounds__(WT) k_ic_wave(Wave W, int base, const T* __restrict__ Lc, const T* __restrict__ Lw,
-                                                const T* __restrict__ Ls, const T* __restrict__ Lb,
-                                                const T* __restrict__ r, T* z, GridSync gs, const SolverState* st,
-                                                int skip_done)
+__global__ void __launch_bounds__(IC_THREADS) k_ic_wave(Wave W, int base, const T* __restrict__ rec, T* zs, GridSync gs,
+                                                const SolverState* st, int skip_done)
 {
     if (skip_done && st && st->done) return;   // uniform across blocks: no barrier is entered
-    __shared__ IcStage<T> sg;
+    extern __shared__ char ic_sm[];
+    IcStage<T>& sg = *reinterpret_cast<IcStage<T>*>(ic_sm);
     const int b = blockIdx.x, nb = gridDim.x;  // one tile per block at a time
     bool ok = true;
-    for (int t = b; t < W.ntiles && ok; t += nb) ok = ic_tile<T, 1>(W, t, base, Lc, Lw, Ls, Lb, r, z, sg);
+    for (int t = b; t < W.ntiles && ok; t += nb) ok = ic_tile<T, 1>(W, t, base, rec, zs, sg);
     if (!grid_barrier(gs) || !ok) return;
     for (int t = b; t < W.ntiles && ok; t += nb)
-        ok = ic_tile<T, -1>(W, W.ntiles - 1 - t, base + W.steps + 1, Lc, Lw, Ls, Lb, r, z, sg);
+        ok = ic_tile<T, -1>(W, W.ntiles - 1 - t, base + W.steps + 1, rec, zs, sg);
+}
+
+// The records of a factor (its FP64 diagonals).
+template <typename T>
+__global__ void k_ic_records(Geo g, Skew sk, const double* __restrict__ Lc, const double* __restrict__ Lw,
+                             const double* __restrict__ Ls, const double* __restrict__ Lb, T* __restrict__ rec)
+{
+    const int k = blockIdx.x * TBK + threadIdx.x, j = blockIdx.y * TBJ + threadIdx.y, i = blockIdx.z;
+    if (k >= g.nz || j >= g.ny) return;
+    const int id = i * g.si + j * g.sj + k;
+    const size_t at = sk.at(i, j, k);
+    T* const r = rec + at / WT * (REC * WT) + at % WT;
+    const T c = (T)Lc[id];
+    r[0] = (T)Lw[id];
+    r[WT] = (T)Ls[id];
+    r[2 * WT] = (T)Lb[id];
+    r[3 * WT] = c;
+    const int e = (__double2hiint((double)c) >> 20) & 0x7ff;
+    r[4 * WT] = e > 1023 - 400 && e < 1023 + 400 ? T(1) / c : T(0);
+    r[5 * WT] = i < g.nx - 1 ? (T)Lw[id + g.si] : T(0);
+    r[6 * WT] = j < g.ny - 1 ? (T)Ls[id + g.sj] : T(0);
+    r[7 * WT] = k < g.nz - 1 ? (T)Lb[id + 1] : T(0);
+}
+
+template <typename T, bool IN>
+__global__ void k_ic_skew(Geo g, Skew sk, const T* __restrict__ from, T* __restrict__ to, const SolverState* st,
+                          int skip_done)
+{
+    if (skip_done && st && st->done) return;
+    const int k = blockIdx.x * TBK + threadIdx.x, j = blockIdx.y * TBJ + threadIdx.y, i = blockIdx.z;
+    if (k >= g.nz || j >= g.ny) return;
+    const int id = i * g.si + j * g.sj + k;
+    if (IN) to[sk.at(i, j, k)] = from[id];
+    else to[id] = from[sk.at(i, j, k)];
 }
 
 // ---- GS-SOR, src/pressure.cpp:212-246 -------------------------------------------
@@ -396,24 +546,12 @@ __global__ void __launch_bounds__(WT) k_ic_wave(Wave W, int base, const T* __res
 // restored to the batch's start and exactly that many sweeps are run: the
 // result is that of testing after every sweep.
 //
-// Layout.  The lanes of a warp work on 32 different planes at a time, so in the
-// field's own layout every lane's 8 bytes lie in another sector (424 us per
-// sweep at 256x128x128, bound by those accesses).  The solve therefore runs on
-// skewed copies of p's interior and of the right-hand side: element (tile,
-// step, warp, lane) holds the cell that this thread works on at that step.
-// Every access of a step is then contiguous, and the old values of the east,
-// north and top neighbours are the next step's own elements of the same
-// thread, the next warp and the next lane: a step copies one new value per
-// cell instead of four.  Faces stay in p.
-struct Skew {
-    int wj, steps;
-    __device__ __forceinline__ size_t at(int i, int j, int k) const   // interior coordinates
-    {
-        const int l = k & 31, w = j % WAVE_TJ, t = (k >> 5) * wj + j / WAVE_TJ;
-        return ((size_t)t * steps + (i + l + w)) * WT + w * 32 + l;
-    }
-};
-
+// Layout.  The solve runs on skewed copies of p's interior and of the
+// right-hand side: every access of a step is then contiguous (in the field's
+// own layout: 424 us per sweep at 256x128x128, bound by those accesses), and
+// the old values of the east, north and top neighbours are the next step's own
+// elements of the same thread, the next warp and the next lane: a step copies
+// one new value per cell instead of four.  Faces stay in p.
 struct GsArgs {
     Wave W;
     int Q, nb;                  // sweeps in flight, blocks per sweep
@@ -583,8 +721,9 @@ __device__ bool gs_tile(const GsArgs& A, int t, int s, int num, int base, double
             pb = lane == 0 ? v0 : pb;
             const double ps = w == 0 ? ps0[q] : sg.xs[(tau - 1) & 1][w - 1][lane];
             const double ew = pe + pw, ns = pn + ps, tb2 = pt + pb;
-            double x;
-            if (FORM == GS_EQUAL) x = fma((ew + ns) + tb2, A.dx.y, -rh);
+            double x = 0.0;   // (the lanes outside the grid hold anything: not through the slow path)
+            if (!act) {
+            } else if (FORM == GS_EQUAL) x = fma((ew + ns) + tb2, A.dx.y, -rh);
             else if (FORM == GS_POW2) x = fma(tb2, A.dz.y, fma(ns, A.dy.y, ew * A.dx.y)) - rh;
             else x = ((div_by(ew, A.dx) + div_by(ns, A.dy)) + div_by(tb2, A.dz)) - rh;
             const double v = one_m_omega * po + omega_coef * x;
@@ -907,24 +1046,24 @@ les_status wave_setup(les_ctx* c, int nx, int ny, int nz, int off, long long spa
 // as tiles but no more than can be resident at once (the tiles are handed out
 // in producer-first order, so any resident count finishes).
 // grid: blocks, no more than wave_resident.
-les_status wave_resident(les_ctx* c, const void* fn, int* blocks)
+les_status wave_resident(les_ctx* c, const void* fn, int threads, size_t smem, int* blocks)
 {
     int per_sm = 0;
-    les_status st = check_cuda(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, WT, 0), "occupancy");
+    les_status st = check_cuda(c, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, threads, smem), "occupancy");
     if (st) return st;
     if (per_sm < 1) return fail(c, LES_CUDA_ERROR, "wavefront kernel cannot be resident");
     *blocks = per_sm * c->sms;
     return LES_OK;
 }
 
-les_status wave_launch(les_ctx* c, const void* fn, void** args, int grid, int pid)
+les_status wave_launch(les_ctx* c, const void* fn, void** args, int grid, int threads, size_t smem, int pid)
 {
     // count and generation only: the error word stays set until the host reads it
     les_status st = check_cuda(c, cudaMemsetAsync(c->gsync, 0, sizeof(unsigned) * 2, c->stream), "reset barrier");
     if (st) return st;
     cudaEvent_t e1 = nullptr;
     if (pid >= 0 && c->prof_on) prof_begin(c, pid, &e1);
-    st = check_cuda(c, cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(WT), args, 0, c->stream),
+    st = check_cuda(c, cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(threads), args, smem, c->stream),
                     "cooperative launch");
     ++c->launches;
     if (e1) cudaEventRecord(e1, c->stream);
@@ -938,45 +1077,79 @@ namespace les {
 // LES_TIMEOUT (and the flag cleared) if a wavefront wait gave up since the last check.
 les_status wave_check(les_ctx* c) { return check_barrier(c); }
 
-les_status ic_apply_dev(les_ctx* c, const double* r, double* z, const double* const* Lsrc, int skip_done)
+// The skewed arrays, kept from solve to solve.
+static les_status skew_buffer(les_ctx* c, size_t doubles)
 {
-    const double* const* L = Lsrc ? Lsrc : (const double* const*)c->L;
+    if (c->skew_len >= doubles) return LES_OK;
+    cudaFree(c->skew_buf);
+    c->skew_buf = nullptr;
+    c->skew_len = 0;
+    les_status st = check_cuda(c, cudaMalloc(&c->skew_buf, sizeof(double) * doubles), "cudaMalloc(skewed arrays)");
+    if (!st) c->skew_len = doubles;
+    return st;
+}
+
+static Skew ic_skew(const les_ctx* c, size_t* len)
+{
+    const Geo& g = c->g;
+    const Skew sk{(g.ny + WAVE_TJ - 1) / WAVE_TJ, g.nx + 31 + WAVE_TJ - 1};
+    *len = (size_t)sk.wj * ((g.nz + 31) / 32) * sk.steps * WT;
+    return sk;
+}
+
+// Lays out the records of the factor L (c, n, s, e, w, t, b) for the applies
+// that follow.
+template <typename T>
+static les_status ic_records(les_ctx* c, const double* const* L)
+{
+    size_t len;
+    const Skew sk = ic_skew(c, &len);
+    les_status st = skew_buffer(c, (REC + 1) * len);   // records, then the vector (FP32 takes half)
+    if (st) return st;
+    launch(c, k_ic_records<T>, cell_grid(c->g), cell_block(), c->g, sk, L[0], L[4], L[2], L[6],
+           reinterpret_cast<T*>(c->skew_buf));
+    return check_launch(c, "ic records");
+}
+
+les_status ic_records64(les_ctx* c, const double* const* L) { return ic_records<double>(c, L); }
+les_status ic_records32(les_ctx* c, const double* const* L) { return ic_records<float>(c, L); }
+
+// z = M^-1 r with the records laid out last.
+template <typename T>
+static les_status ic_apply(les_ctx* c, const T* r, T* z, const SolverState* state, int skip_done)
+{
+    size_t len;
+    const Skew sk = ic_skew(c, &len);
+    if (c->skew_len < (REC + 1) * len) return fail(c, LES_BAD_ARG, "internal: no IC records");
+    const T* rec = reinterpret_cast<const T*>(c->skew_buf);
+    T* zs = reinterpret_cast<T*>(c->skew_buf) + REC * len;
     Wave W;
     int base = 0;
     les_status st = wave_setup(c, c->g.nx, c->g.ny, c->g.nz, 0, 2 * (c->g.nx + 32 + WAVE_TJ), 1, W, base);
     if (st) return st;
-    const double *Lc = L[0], *Lw = L[4], *Ls = L[2], *Lb = L[6];
-    const void* fn = (const void*)k_ic_wave<double>;
-    int resident = 0;
-    st = wave_resident(c, fn, &resident);
+    const void* fn = (const void*)k_ic_wave<T>;
+    const size_t smem = sizeof(IcStage<T>);
+    st = check_cuda(c, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "smem attribute");
     if (st) return st;
+    int resident = 0;
+    if ((st = wave_resident(c, fn, IC_THREADS, smem, &resident))) return st;
     const int grid = W.ntiles < resident ? W.ntiles : resident;
     GridSync gs = grid_sync(c, grid);
-    const SolverState* stp = c->state;
-    int skip = skip_done;
-    void* args[] = {&W, &base, (void*)&Lc, (void*)&Lw, (void*)&Ls, (void*)&Lb, (void*)&r, (void*)&z, &gs,
-                    (void*)&stp, &skip};
-    return wave_launch(c, fn, args, grid, PROF_IC);
+    launch(c, k_ic_skew<T, true>, cell_grid(c->g), cell_block(), c->g, sk, r, zs, state, skip_done);
+    void* args[] = {&W, &base, (void*)&rec, (void*)&zs, &gs, (void*)&state, &skip_done};
+    if ((st = wave_launch(c, fn, args, grid, IC_THREADS, smem, PROF_IC))) return st;
+    launch(c, k_ic_skew<T, false>, cell_grid(c->g), cell_block(), c->g, sk, (const T*)zs, z, state, skip_done);
+    return check_launch(c, "ic apply");
 }
 
-les_status ic_apply_dev32(les_ctx* c, const float* r, float* z, const float* const* L, SolverState* st)
+les_status ic_apply_dev(les_ctx* c, const double* r, double* z, int skip_done)
 {
-    Wave W;
-    int base = 0;
-    les_status s2 = wave_setup(c, c->g.nx, c->g.ny, c->g.nz, 0, 2 * (c->g.nx + 32 + WAVE_TJ), 1, W, base);
-    if (s2) return s2;
-    const float *Lc = L[0], *Lw = L[4], *Ls = L[2], *Lb = L[6];
-    const void* fn = (const void*)k_ic_wave<float>;
-    int resident = 0;
-    s2 = wave_resident(c, fn, &resident);
-    if (s2) return s2;
-    const int grid = W.ntiles < resident ? W.ntiles : resident;
-    GridSync gs = grid_sync(c, grid);
-    const SolverState* stp = st;
-    int skip = st ? 1 : 0;
-    void* args[] = {&W, &base, (void*)&Lc, (void*)&Lw, (void*)&Ls, (void*)&Lb, (void*)&r, (void*)&z, &gs,
-                    (void*)&stp, &skip};
-    return wave_launch(c, fn, args, grid, PROF_IC);
+    return ic_apply<double>(c, r, z, c->state, skip_done);
+}
+
+les_status ic_apply_dev32(les_ctx* c, const float* r, float* z, SolverState* st)
+{
+    return ic_apply<float>(c, r, z, st, st ? 1 : 0);
 }
 
 les_status build_ic_dev(les_ctx* c)
@@ -1017,7 +1190,7 @@ les_status solve_gs_dev(les_ctx* c, double dt, double rho, int max_iter, double 
     const void* fn = !p2 ? (const void*)k_gs_wave<GS_DIV>
                          : (dx2 == dy2 && dy2 == dz2 ? (const void*)k_gs_wave<GS_EQUAL> : (const void*)k_gs_wave<GS_POW2>);
     int resident = 0;
-    st = wave_resident(c, fn, &resident);
+    st = wave_resident(c, fn, WT, 0, &resident);
     if (st) return st;
     // Sweeps in flight: as many as there are resident blocks for, up to what a
     // sweep's length has room for (a sweep starts about 20 steps behind the
@@ -1037,14 +1210,7 @@ les_status solve_gs_dev(les_ctx* c, double dt, double rho, int max_iter, double 
                     batches * GS_BATCH * (long long)(g.nx - 2 + 32 + WAVE_TJ), Q, a.W, base);
     if (st) return st;
     a.len = (size_t)a.W.ntiles * a.W.steps * WT;
-    if (c->gs_len < 5 * a.len) {   // the skewed arrays, kept for the next solve
-        cudaFree(c->gs_buf);
-        c->gs_buf = nullptr;
-        c->gs_len = 0;
-        st = check_cuda(c, cudaMalloc(&c->gs_buf, sizeof(double) * 5 * a.len), "cudaMalloc(skewed sweeps)");
-        if (st) return st;
-        c->gs_len = 5 * a.len;
-    }
+    if ((st = skew_buffer(c, 5 * a.len))) return st;
     const int words = (g.nx + 31) / 32;
     a.Q = Q;
     a.nb = ntiles < resident ? ntiles : resident;
@@ -1056,12 +1222,12 @@ les_status solve_gs_dev(les_ctx* c, double dt, double rho, int max_iter, double 
     a.tol = tol;
     a.max_iter = max_iter;
     a.p = c->slot[LES_P];
-    a.ps = c->gs_buf;
-    double* const rhs = c->gs_buf + a.len;
+    a.ps = c->skew_buf;
+    double* const rhs = c->skew_buf + a.len;
     a.rhs = rhs;
-    a.ps_back = c->gs_buf + 2 * a.len;
-    a.rep[0] = c->gs_buf + 3 * a.len;
-    a.rep[1] = c->gs_buf + 4 * a.len;
+    a.ps_back = c->skew_buf + 2 * a.len;
+    a.rep[0] = c->skew_buf + 3 * a.len;
+    a.rep[1] = c->skew_buf + 4 * a.len;
     a.face_back = c->w[0];
     a.rep_back = c->w[1];
     unsigned* const rd = reinterpret_cast<unsigned*>(c->w[2]);   // two words per column and 32 planes: n doubles hold them
@@ -1088,7 +1254,7 @@ les_status solve_gs_dev(les_ctx* c, double dt, double rho, int max_iter, double 
     if ((st = check_launch(c, "gs set-up"))) return st;
     void* args[] = {&a, &base};
     if (max_iter > 0) {
-        st = wave_launch(c, fn, args, grid, -1);
+        st = wave_launch(c, fn, args, grid, WT, 0, -1);
         if (st) return st;
         launch(c, k_gs_unskew, cell_grid(g), cell_block(), g, sk, (const double*)a.ps, a.p);
         if ((st = pressure_bcs_dev(c, a.p))) return st;   // of the last sweep
