@@ -18,8 +18,8 @@
 // by the block, loads and stores are 16 bytes wide, the arithmetic is packed
 // (two cells per instruction) and 12 warps instead of 8 run on an SM.
 // Microseconds per inner iteration, strips -> plane marches (GB300):
-//   64x32x32 degree 4     22.6 -> 13.2     256x128x128 degree 4   46.4 -> 40.1
-//   161x93x75 degree 5    36.5 -> 26.4     256x128x128 degree 7    138 -> 72
+//   64x32x32 degree 4     22.6 -> 11.1     256x128x128 degree 4   46.4 -> 37.7
+//   161x93x75 degree 5    36.5 -> 25.0     256x128x128 degree 7    138 -> 72
 //   128x96x96 degree 4    28.3 -> 20.6     512x256x256 degree 4    335 -> 252
 //   200x90x90 Jacobi      19.4 -> 15.4     384x200x257 degree 5    302 -> 220
 // What bounds them: pass A at 512x256x256 the HBM rate (24 B per cell, 126 us:
@@ -56,7 +56,7 @@ constexpr int PR = 2;   // rows per thread
 // registers spill 0.5 KB, and pass B of 512x256x256 takes 282 instead of
 // 124 us; at 384 threads none).
 __host__ __device__ constexpr int plane_threads_b(int S) { return S <= 2 ? 512 : (S == 3 ? 384 : 256); }
-__host__ __device__ constexpr int plane_threads_a() { return 512; }
+__host__ __device__ constexpr int plane_threads_a() { return 448; }
 
 // A published vector's levels lie side by side, an odd number of 16-byte
 // slots apart from the next vector's (no bank conflicts); a buffer has the
@@ -403,22 +403,24 @@ __device__ __forceinline__ void plane_a(const PlaneArgsA& a, int blk, int nblk)
     const TilePos t = tile_pos<1>(g, m, blk);
     const unsigned si = 4u * (unsigned)g.si;
     const int is = t.i0 > 0 ? t.i0 - 1 : 0;
-    Vec vz[PR], vp[PR], ve[PR];
-    // planes past the outlet read the outlet plane (weight 0), planes that are
-    // not owned some e (not used)
-    auto fetch = [&](int P) {
+    // two planes ahead (one ahead in 512 threads: 20.8 us at 256x128x128, two in
+    // 448: 19.7); planes past the outlet read the outlet plane (weight 0),
+    // planes that are not owned some e (not used)
+    Vec fz[2][PR], fp[2][PR], fe[2][PR];
+    auto fetch = [&](int P, int s) {
         const unsigned at = (unsigned)min(P, g.nx - 1) * si;
 #pragma unroll
         for (int r = 0; r < PR; ++r) {
-            vz[r] = ldv(a.z, at + t.off[r]);
+            fz[s][r] = ldv(a.z, at + t.off[r]);
             if (!FIRST) {
-                vp[r] = ldv(a.pold, at + t.off[r]);
-                ve[r] = ldv(a.e, at + t.off[r]);
+                fp[s][r] = ldv(a.pold, at + t.off[r]);
+                fe[s][r] = ldv(a.e, at + t.off[r]);
             }
         }
     };
     dep_wait();
-    fetch(is);   // on its way while the head sums
+    fetch(is, 0);   // on their way while the head sums
+    fetch(is + 1, 1);
     const HeadOut h = plane_head_a<FIRST>(a.df.pin, a.df.nb_in, a.st, a.outer, a.total_cap, a.pslot, blk);
     if (h.end) return;
     const float beta = h.coef, aprev = FIRST ? 0.f : (float)a.st->alpha;
@@ -438,6 +440,7 @@ __device__ __forceinline__ void plane_a(const PlaneArgsA& a, int blk, int nblk)
             if (P > t.i1) break;
             constexpr int BUF = TMAX * PR;
             const int put = (u & 1) * BUF, got = ((u & 1) ^ 1) * BUF;
+            Vec(&vz)[PR] = fz[u & 1], (&vp)[PR] = fp[u & 1], (&ve)[PR] = fe[u & 1];
             Vec(&p0)[PR] = p[u], (&p1)[PR] = p[(u + 3) & 3], (&p2)[PR] = p[(u + 2) & 3];
             const unsigned at = (unsigned)P * si;
 #pragma unroll
@@ -454,7 +457,7 @@ __device__ __forceinline__ void plane_a(const PlaneArgsA& a, int blk, int nblk)
                         stv(a.e, at + t.off[r], FIRST ? vzero() : vfma(aprev, vp[r], ve[r]));
                     }
             }
-            if (P < t.i1) fetch(P + 1);
+            if (P + 1 < t.i1) fetch(P + 2, u & 1);
             const int C = P - 1;
             if (C >= t.i0) {
                 const bool ident = C == g.nx - 1;
