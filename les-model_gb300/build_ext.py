@@ -37,6 +37,7 @@ UNITS = {
     "les_plane.cu": [],
     "les_plane_lo.cu": [],
     "les_plane_hi.cu": [],
+    "les_cluster.cu": [],
     "les_ensemble.cu": [],
     "les_tune.cu": [],
     "les_adjoint.cu": ["-fmad=false"],

@@ -230,6 +230,7 @@ les_status col_plan(les_ctx* c, const les_pcg_opts* o, ViewF A, SolverState* in,
     if (P.plane) {
         les_status st = plane_maps(c, o, P);
         if (st) return st;
+        P.cluster = cluster_used(c, o, P.S);
         if ((size_t)2 * P.blocks_b + (size_t)P.blocks_a > c->partials_len)
             return fail(c, LES_BAD_ARG, "plane march grid exceeds the reduction scratch");
         return LES_OK;

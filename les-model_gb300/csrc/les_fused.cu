@@ -908,6 +908,10 @@ les_status inner_solve_fused(les_ctx* c, const les_pcg_opts* o, ViewF A, SolverS
     FusedPlan P;
     les_status st = fused_plan(c, o, A, in, out, P);
     if (st) return st;
+    if (P.col && P.cp.cluster) {
+        st = cluster_solve(c, P.cp);
+        return st ? st : read_state(c);
+    }
     st = emit_pass_b(c, P, true, 0, 0);   // z = M^-1 r, rho, e = 0
     if (st) return st;
     int rc = 1, pc = 0, launched = 0, batch = 4;
@@ -982,6 +986,11 @@ les_status capture_mixed_fused(les_ctx* c, const les_pcg_opts* o, ViewF A, int k
     return capture_while(c, set_outer, [&](cudaGraphConditionalHandle ho) -> les_status {
         les_status s2;
         if ((s2 = emit_inner_start(c, o, inner_cap))) return s2;     // inner state from the outer residual
+        if (P.col && P.cp.cluster) {
+            if ((s2 = cluster_solve(c, P.cp))) return s2;
+            if ((s2 = emit_outer_update(c, o, P.col))) return s2;
+            return set_outer(ho);
+        }
         if ((s2 = emit_pass_b(c, P, true, 0, 0))) return s2;          // z = M^-1 r, rho, e = 0
         if ((s2 = emit_pass_a(c, P, true, 0))) return s2;             // iteration 1: p1 = z
         if ((s2 = emit_pass_b(c, P, false, 1, 1))) return s2;         //   r1 -> r0

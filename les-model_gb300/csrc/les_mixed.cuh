@@ -149,6 +149,7 @@ struct PlaneMap {
 struct ColPlan {
     bool plane = false;    // the plane marches (pa, pb) instead of the strips (ma, mb)
     PlaneMap pa{}, pb{};
+    bool cluster = false;  // the whole inner solve in one cluster (les_cluster.cu)
     int S = 0;             // Chebyshev levels (degree - 1); 0 = Jacobi
     ColCheb c3{};
     float inv_c0 = 1.f;
@@ -164,6 +165,8 @@ struct ColPlan {
 constexpr int plane_pitch(int nz) { return (nz + 3) / 4 * 4; }
 bool plane_used(const les_ctx* c, const les_pcg_opts* o);   // the plane marches serve this solve
 les_status plane_maps(les_ctx* c, const les_pcg_opts* o, ColPlan& P);
+bool cluster_used(les_ctx* c, const les_pcg_opts* o, int S);
+les_status cluster_solve(les_ctx* c, const ColPlan& P);   // f[0] -> e, the last p and alpha
 les_status plane_pass_a(les_ctx* c, const ColPlan& P, bool first, int pc);
 les_status plane_pass_b(les_ctx* c, const ColPlan& P, bool first, int rin);
 // row length of the inner vectors of this solve

@@ -106,7 +106,7 @@ Geo padded(const Geo& g)
 
 namespace les {
 
-static ChebPairs cheb_pairs(const ColCheb& c, int S)
+ChebPairs cheb_pairs(const ColCheb& c, int S)
 {
     ChebPairs p{};
     auto two = [](double v) { return make_float2((float)v, (float)v); };

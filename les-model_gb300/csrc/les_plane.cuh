@@ -77,6 +77,8 @@ struct ChebPairs {
     float2 zs;              // s_S: the last level's z
 };
 
+ChebPairs cheb_pairs(const ColCheb& c, int S);
+
 struct PlaneArgsA {
     Geo g;            // strides of the padded layout
     PlaneMap m;

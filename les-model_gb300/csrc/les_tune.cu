@@ -218,7 +218,8 @@ les_status tune(std::vector<Case>& cs, cudaStream_t main, double base, double* b
     if (!st && plane) st = time_round(cs, main, &up);
     plane = plane && !st && up < ub;
     for (auto& q : cs) {
-        q.c->tune_plane = plane;
+        // the cluster solve stands on the plane marches and beats both
+        q.c->tune_plane = plane || (!st && cluster_used(q.c, &q.o, q.S));
         ++q.c->version;
     }
     if (plane) ub = up;
