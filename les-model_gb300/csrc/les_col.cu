@@ -44,6 +44,8 @@
 // planes need plane-uniform coefficients.  Halo cells of a strip are
 // recomputed by every strip that needs them (values of lanes and rows past
 // the shrinking halo are never used).
+#include <algorithm>
+
 #include "les_col_march.cuh"
 
 namespace {
@@ -151,9 +153,9 @@ ColMap col_map(les_ctx* c, const void* fn, int threads, int halo, int tj, int ci
 {
     const Geo& g = c->g;
     ColMap m{};
-    m.tk = 32 - 2 * halo;
     m.tj = tj;
-    m.tiles_k = (g.nz + m.tk - 1) / m.tk;
+    // the tiles at the two walls have a halo on one side (a single tile none)
+    m.tiles_k = g.nz <= 32 ? 1 : 2 + std::max(0, (g.nz - 2 * (32 - halo) + 31 - 2 * halo) / (32 - 2 * halo));
     m.tiles_j = (g.ny + tj - 1) / tj;
     const int tiles = m.tiles_k * m.tiles_j;
     int ci = ci_force;

@@ -68,7 +68,8 @@ constexpr unsigned FULL = 0xffffffffu;
 struct StripPos {
     int j0;        // j of row 0
     int i0, i1;    // owned planes [i0, i1)
-    int kl;        // this lane's k after reflection at the walls
+    int kl;        // this lane's k (after reflection at the walls)
+    int lo, hi;    // lanes of the k neighbours (a wall's mirrored neighbour is the one inside)
     unsigned own;  // bit r: cell of row r owned by this lane
     int rows;      // row pattern (RowsMode) of the strip
     bool kown;     // this lane's k is owned
@@ -124,7 +125,11 @@ __device__ __forceinline__ StripPos strip_pos(const Geo& g, const ColMap& m, int
     StripPos s;
     const int kt = item % m.tiles_k, rest = item / m.tiles_k;
     const int jt = rest % m.tiles_j, ch = rest / m.tiles_j;
-    const int kg = kt * m.tk - HALO + lane;
+    // a tile at a wall has its edge lane there and needs no halo on that side
+    const bool last = kt == m.tiles_k - 1;
+    const int own0 = kt == 0 ? 0 : 32 - HALO + (kt - 1) * (32 - 2 * HALO);
+    const int own1 = last ? g.nz : own0 + (kt == 0 ? 32 - HALO : 32 - 2 * HALO);
+    const int kg = (kt == 0 ? 0 : (last ? g.nz - 32 : own0 - HALO)) + lane;
     s.j0 = jt * TJ - HALO;
     constexpr int H = TJ + 2 * HALO;
     if (s.j0 >= 0 && s.j0 + H <= g.ny) s.rows = ROWS_PLAIN;
@@ -135,7 +140,9 @@ __device__ __forceinline__ StripPos strip_pos(const Geo& g, const ColMap& m, int
     s.i1 = min(g.nx, s.i0 + m.ci);
     // lanes past one reflection are never used; they read any cell of the grid
     s.kl = max(reflect(kg, g.nz), 0);
-    const bool kown = kg >= 0 && kg < g.nz && lane >= HALO && lane < HALO + m.tk;
+    const bool kown = kg >= own0 && kg < own1;
+    s.lo = kg == 0 ? lane + 1 : max(lane - 1, 0);
+    s.hi = kg == g.nz - 1 ? lane - 1 : min(lane + 1, 31);
     s.kown = kown;
     s.allrows = s.j0 + HALO + TJ <= g.ny;
     s.own = 0u;
@@ -473,8 +480,8 @@ __device__ __forceinline__ void col_a(const Geo& g, const ColMap& m, const Coef&
 #pragma unroll
                 for (int r = 1; r <= TJ; ++r) {
                     const float pc = p1[r];
-                    const float pb = __shfl_up_sync(FULL, pc, 1);
-                    const float pt = __shfl_down_sync(FULL, pc, 1);
+                    const float pb = __shfl_sync(FULL, pc, s.lo);
+                    const float pt = __shfl_sync(FULL, pc, s.hi);
                     qv[r] = cc * pc + cx * p2[r] + ce * p0[r] + cy * (p1[r - 1] + p1[r + 1]) + cz * (pb + pt);
                 }
                 auto outq = [&](auto all) {
@@ -684,8 +691,8 @@ __device__ __forceinline__ void col_b(const Geo& g, const ColMap& m, const ColCh
                         zc = zr[LV - 2][1][r]; zw = zr[LV - 2][2][r]; ze = zr[LV - 2][0][r];
                         zs = zr[LV - 2][1][r - 1]; zn = zr[LV - 2][1][r + 1];
                     }
-                    const float zb = __shfl_up_sync(FULL, zc, 1);
-                    const float zt = __shfl_down_sync(FULL, zc, 1);
+                    const float zb = __shfl_sync(FULL, zc, s.lo);
+                    const float zt = __shfl_sync(FULL, zc, s.hi);
                     float zk = cc * zc + cx * zw + ce * ze + cy * (zs + zn) + cz * (zb + zt);
                     if (LV == 2) zk = fmaf(cr, rp[2][r], zk);   // r' and z_0 = a0 r'
                     if (LV >= 3) zk = fmaf(cr, rp[LV][r], fmaf(cg, zr[LV - 3][2][r], zk));

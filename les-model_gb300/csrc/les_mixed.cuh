@@ -128,7 +128,6 @@ bool fused_supported(const les_pcg_opts* o);
 // Work split of one pass: warp `item` owns k-strip item % tiles_k, row strip
 // (item / tiles_k) % tiles_j and plane chunk item / (tiles_k * tiles_j).
 struct ColMap {
-    int tk;        // output cells of a strip along k (32 minus twice the halo)
     int tj;        // output rows of a strip along j
     int tiles_k, tiles_j;
     int ci;        // planes per chunk
