@@ -521,12 +521,13 @@ def run_adjoint(args):
     return 0
 
 
-# FP64 operations per cell of the FP64 PCG kernels (each multiply and add
-# counted; the reference-order kernels run without FMA): the 7-point row is
-# 7 multiplies + 6 adds
-FP64_OPS_PER_CELL = {"spmv_f64": 15.0,     # row + p.q term
-                     "update_f64": 6.0,    # x += a p, r -= a q, r.r term (Chebyshev/IC form)
-                     "cheb_f64": 18.0}     # row + r - Az + beta p + z + alpha p
+# FP64 operations per cell of the FP64 PCG kernels as they execute for the
+# power-of-two coefficients of these grids (a multiply and an add whose product
+# is exact are one fused operation, counted once): the 7-point row is a multiply
+# and 6 fused operations
+FP64_OPS_PER_CELL = {"spmv_f64": 8.0,      # row + p.q term
+                     "update_f64": 6.0,    # x += a p, r -= a q, r.r term, z_0 = a0 r
+                     "cheb_f64": 13.0}     # row + r - Az + beta p + z + alpha p}     # row + r - Az + beta p + z + alpha p
 
 
 def rel_err(a, b, tmp=None):

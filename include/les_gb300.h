@@ -353,14 +353,17 @@ les_status les_ensemble_set_batched(les_ensemble* ens, int on);
 /* ---- options (no reference counterpart) --------------------------------- */
 typedef enum les_option {
     LES_OPT_FUSED = 0,  /* mixed-precision inner iteration (Jacobi, Chebyshev degree
-                           2..7) as two fused passes: 1 (default) register-column
-                           marches (device-built matrix; stored matrices use 2);
+                           2..7) as two fused passes: 1 (default) plane marches, on
+                           small grids the whole inner solve in one thread-block
+                           cluster, in batched ensembles register-column strips
+                           (device-built matrix; stored matrices use 2);
                            2 shared-memory tiles; 0: one kernel per vector operation */
     LES_OPT_TMA = 1,    /* 1: the shared-memory tile passes, with their planes staged
                            by TMA when nz % 16 == 0 and the matrix is device-built;
                            0 (default): no TMA */
-    /* shape of the register-column passes (0 = built-in choice; les_autotune
-       sets them by timing): */
+    /* shape of the register-column strips (0 = built-in choice; les_autotune
+       sets them by timing).  Setting one makes a single case's solve run as
+       strips instead of plane marches: */
     LES_OPT_ROWS_A = 2,   /* rows per strip of pass A: 8 or 16 */
     LES_OPT_ROWS_B = 3,   /* rows per strip of pass B: 16 (Jacobi), 4 or 8
                              (Chebyshev degree 2..4), 4 (degree 5..7) */
@@ -370,8 +373,8 @@ typedef enum les_option {
                              runs as one CUDA graph launch (captured per velocity
                              buffer parity, both solver loops as conditional nodes;
                              not while les_profile records); 0: launch by launch */
-    LES_OPT_PDL = 7,      /* 1 (default; 0 for ensemble cases): the register-column
-                             passes are launched as programmatic dependents of the
+    LES_OPT_PDL = 7,      /* 1 (default; 0 for ensemble cases): the passes of the
+                             inner iteration are launched as programmatic dependents of the
                              kernel before them (their blocks become resident while it
                              drains); 0: plain stream order */
     LES_OPT_PHYS32 = 8,   /* 1 (default): a les_step whose pressure solve is the
@@ -384,7 +387,7 @@ typedef enum les_option {
                              (about 2 s) gives up; the solve then returns LES_TIMEOUT
                              and the context stays usable.  For testing the failure
                              path only. */
-    LES_OPT_COL_STRIDE = 10 /* 1 (default): the register-column passes of a grid with
+    LES_OPT_COL_STRIDE = 10 /* 1 (default): the register-column strips of a grid with
                              nz = 32, 64, 128 or 256 run kernels compiled for that row
                              stride (row offsets as immediates); 0: the kernels that
                              read the stride at run time.  Same results either way. */

@@ -1,6 +1,11 @@
 // les_col.cu -- the FP32 inner PCG iteration of the mixed-precision solve as
 // two register-resident column marches (Jacobi or Chebyshev preconditioner).
 //
+// The strips of this file serve batched ensembles, solves with a forced strip
+// shape and vectors of 4 GB and more; the others run the same two passes as
+// plane marches (les_plane.cuh) or, on small grids, in one cluster
+// (les_cluster.cu).
+//
 // Each warp owns a strip of the grid, 32 consecutive cells along k (one per
 // lane) by H rows along j, and marches along i over a chunk of planes.  A lane
 // keeps its own column of values in registers for the planes a stencil needs:

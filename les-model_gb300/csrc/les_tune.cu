@@ -8,7 +8,9 @@
 // GPU the case gets (alone, or beside other cases of an ensemble), so they are
 // measured: each candidate runs a few launches of the pass on the context's
 // own matrix and work vectors, timed with CUDA events, cases of an ensemble
-// concurrently as in a step.
+// concurrently as in a step.  The best strips then compete with the plane
+// marches (les_plane.cuh), which choose their own tiles; where the cluster
+// solve (les_cluster.cu) applies it stays in use.
 #include <algorithm>
 #include <vector>
 

@@ -524,8 +524,8 @@ __global__ void k_ic_skew(Geo g, Skew sk, const T* __restrict__ from, T* __restr
 // sweep.  One sweep at a time spends 700 of its 1000 steps filling and
 // draining the wavefront with one warp per SM sub-partition (256x128x128: 1.18
 // ms per sweep, FP64 pipe idle); in flight the sweeps keep several blocks on
-// every SM busy.  256x128x128: 1180 -> 195 us per sweep (the FP64 pipe alone
-// needs about 95); h = 1/161, 191x161x115: 2070 -> 370 us; 67x46x53: 570 -> 80.
+// every SM busy.  256x128x128: 1180 -> 190 us per sweep (the FP64 pipe alone
+// needs about 95); h = 1/161, 191x161x115: 2070 -> 318 us; 67x46x53: 570 -> 80.
 //
 // Boundary conditions inside a run of sweeps.  Faces: the value that
 // apply_pressure_BCs leaves on the face next to an interior cell is that
