@@ -181,8 +181,8 @@ struct ClusterSolve {
             const float4 x = lane < nw ? warp_part[lane] : make_float4(0.f, 0.f, 0.f, 0.f);
             s0 = Acc{x.x, x.y};
             s1 = Acc{x.z, x.w};
-            lane_sum<32>(s0);
-            if (which == 1) lane_sum<32>(s1);
+            lane_sum<PER == 2 ? 16 : 32>(s0);   // PER = 2: at most 16 warps
+            if (which == 1) lane_sum<PER == 2 ? 16 : 32>(s1);
             if (lane < NB) peer_store(peer_addr(smem_addr(part[which] + rank), lane), make_float4(s0.hi, s0.lo, s1.hi, s1.lo));
         }
     }
