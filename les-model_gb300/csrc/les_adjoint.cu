@@ -35,6 +35,7 @@
 #include <vector>
 
 #include "les_internal.cuh"
+#include "les_mixed.cuh"
 
 using namespace les;
 
@@ -44,6 +45,15 @@ les_status velocity_bcs_dev(les_ctx* c);
 les_status pcg_fp64(les_ctx* c, const les_pcg_opts* o, les_pcg_result* res, int keep_tol);
 les_status pcg_mixed_impl(les_ctx* c, const les_pcg_opts* o, les_pcg_result* res, int keep_tol);
 les_status dot_dev(les_ctx* c, const double* a, const double* b, double* out_host);
+
+// A captured mixed solve of one solution and right-hand side (its tolerance is
+// set on the device before each launch).
+struct SolveGraph {
+    double *rhs = nullptr, *sol = nullptr;
+    les_pcg_opts o{};
+    unsigned long long version = 0, captured = 0;
+    cudaGraphExec_t exec = nullptr;
+};
 
 struct AdjWork {
     les_adjoint_params prm{};
@@ -60,6 +70,7 @@ struct AdjWork {
     double* grad_in = nullptr;     // ny*nz
     double* acc = nullptr;         // [0] J, [1] dJ/dCs
     bool forward_done = false;
+    SolveGraph sg[2];              // the forward steps' solve, the adjoint's
 };
 
 void adj_work_free(AdjWork* a)
@@ -75,6 +86,8 @@ void adj_work_free(AdjWork* a)
     cudaFree(a->lb);
     cudaFree(a->grad_in);
     cudaFree(a->acc);
+    for (auto& g : a->sg)
+        if (g.exec) cudaGraphExecDestroy(g.exec);
     delete a;
 }
 }  // namespace les
@@ -558,6 +571,54 @@ les_status fwd_step(les_ctx* c, const les_step_params* prm)
     return LES_OK;
 }
 
+__global__ void k_solve_tol(SolverState* st, double tol) { st->tol = tol; }
+
+// The mixed solve as one graph launch, both solver loops on the device.  Driven
+// from the host it waits for the state every 32 iterations and starts up to 31
+// that find the solve ended: 128x64x64 to 1e-12, 592 iterations, 9.07 -> 8.25 ms.
+les_status solve_graph(les_ctx* c, AdjWork& a, const les_pcg_opts& opts, les_pcg_result* r)
+{
+    les_status st = ensure_work(c);
+    if (!st) st = ensure_work32(c);
+    if (st) return st;
+    double *rhs = c->slot[LES_B], *sol = c->slot[LES_P];
+    les_pcg_opts o = opts;
+    o.tol = 0.0;
+    SolveGraph& g = a.sg[sol == a.lb ? 1 : 0];
+    if (!g.exec || g.version != c->version || g.rhs != rhs || g.sol != sol || std::memcmp(&g.o, &o, sizeof o)) {
+        if (g.exec) cudaGraphExecDestroy(g.exec);
+        g = SolveGraph{};
+        const unsigned long long l0 = c->launches;
+        cudaGraph_t graph = nullptr;
+        st = check_cuda(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeRelaxed), "begin solve capture");
+        if (st) return st;
+        les_status st1 = capture_mixed_fused(c, &o, view32_of(c), 1);
+        st = check_cuda(c, cudaStreamEndCapture(c->stream, &graph), "end solve capture");
+        if (st1) st = st1;
+        if (!st) st = check_cuda(c, cudaGraphInstantiate(&g.exec, graph, 0), "instantiate solve graph");
+        if (graph) cudaGraphDestroy(graph);
+        if (st) {
+            c->launches = l0;
+            g = SolveGraph{};
+            return st;
+        }
+        g.captured = c->launches - l0;
+        c->launches = l0;
+        g.rhs = rhs;
+        g.sol = sol;
+        g.o = o;
+        g.version = c->version;
+    }
+    launch(c, k_solve_tol, 1, 1, c->state, opts.tol);
+    if ((st = check_cuda(c, cudaGraphLaunch(g.exec, c->stream), "launch solve graph")) || (st = read_state(c))) return st;
+    c->launches += g.captured;   // one pass of each loop
+    const SolverState& h = c->h_state[0];
+    r->iters = h.iters;
+    r->outer = h.k;
+    r->residual = h.err;
+    return h.done ? (les_status)h.status : LES_NOT_CONVERGED;
+}
+
 // sol = A^-1 rhs with the step's PCG to adj_rel_tol * ||rhs|| (sol holds the
 // warm start on entry)
 les_status solve_linear(les_ctx* c, AdjWork& a, double* rhs, double* sol, const char* what)
@@ -580,7 +641,11 @@ les_status solve_linear(les_ctx* c, AdjWork& a, double* rhs, double* sol, const 
     c->slot[LES_B] = rhs;
     c->slot[LES_P] = sol;
     les_pcg_result r{};
-    st = o.precision == LES_MIXED ? pcg_mixed_impl(c, &o, &r, 0) : pcg_fp64(c, &o, &r, 0);
+    if (o.precision == LES_MIXED && c->graph_on && !c->prof_on && c->stencil_mode == 1 && c->fused && fused_supported(&o) &&
+        o.max_iter > 0)
+        st = solve_graph(c, a, o, &r);
+    else
+        st = o.precision == LES_MIXED ? pcg_mixed_impl(c, &o, &r, 0) : pcg_fp64(c, &o, &r, 0);
     c->slot[LES_B] = sb;
     c->slot[LES_P] = sp;
     if (st == LES_NOT_CONVERGED) return fail(c, st, std::string(what) + ": a pressure solve did not converge");
