@@ -252,12 +252,28 @@ __device__ __forceinline__ void zero_pads(Vec& v, const TilePos& t)
 // together.  64x32x32: 12.6 -> 11.5 us per iteration, 128x64x64:
 // 16.4 -> 15.0, 256x128x128: 40.1 -> 38.7.
 
-// num / den to FP32 precision from pairs
+// The quotient of two pairs on the FP64 pipe: out of line, for df_quotient's rare
+// operands.
+__device__ __noinline__ static float pair_divide(float nh, float nl, float dh, float dl)
+{
+    return (float)(((double)nh + (double)nl) / ((double)dh + (double)dl));
+}
+
+// num / den of pairs, rounded to FP32: the quotient of the high parts and one
+// correction by the remainder, within 2^-46 of the exact quotient before the
+// rounding.  That wants normal numbers all along -- the reciprocal of a d.hi
+// below 2^-128 is infinite, and the remainder of a small n.hi is lost below
+// 2^-126 -- so operands outside 2^-64 .. 2^64 take FP64, as do zeros, infinities
+// and NaN.  (The residual's square leaves that range for right-hand sides of
+// about 1e-10 and smaller.)
 __device__ __forceinline__ float df_quotient(const Acc& n, const Acc& d)
 {
+    auto inside = [](float x) { return ((__float_as_uint(x) >> 23) & 0xffu) - (127u - 64u) <= 128u; };
     const float q = __fdiv_rn(n.hi, d.hi);
     const float r = __fadd_rn(fmaf(-q, d.hi, n.hi), fmaf(-q, d.lo, n.lo));
-    return fmaf(r, __frcp_rn(d.hi), q);
+    float v = fmaf(r, __frcp_rn(d.hi), q);
+    if (!inside(n.hi) | !inside(d.hi)) v = pair_divide(n.hi, n.lo, d.hi, d.lo);
+    return v;
 }
 
 // Sums NV vectors of nb partials, the totals in thread 0.
