@@ -3,6 +3,7 @@
 #include "les_plane.cuh"
 
 #include <algorithm>
+#include <cmath>
 
 namespace {
 
@@ -130,6 +131,34 @@ ChebPairs cheb_pairs(const ColCheb& c, int S)
     return p;
 }
 
+// The scaled levels are larger than r': a bound of their growth, from the sums
+// of the weights' magnitudes.
+static double level_growth(const ChebPairs& p, int S)
+{
+    double before = 0.0, g = 1.0, most = 1.0;   // levels k-2, k-1
+    for (int k = 0; k < S; ++k) {
+        const double cc = std::max(std::fabs(p.cc[k].x), std::fabs(p.ci[k].x));
+        const double v = (cc + 2.0 + 2.0 * std::fabs(p.wy.x) + 2.0 * std::fabs(p.wz.x)) * g + std::fabs(p.rr[k].x) +
+                         std::fabs(p.gg[k].x) * before;
+        before = g;
+        g = v;
+        if (!(g <= most)) most = g;
+    }
+    return most;
+}
+
+// Growth 2^60 at most: the square of r' is an FP32 number, so |r'| < 2^64 and the
+// levels stay below 2^124; and with the last weight normal nothing is lost at the
+// lower end.  Cubes have 2^24 at degree 7 and 2^12 at degree 4; the line lies at
+// about dx / dy = 10 for degree 7, 300 for degree 4.  (The strips do not scale
+// their levels.)
+static bool levels_fit(const les_ctx* c, const les_pcg_opts* o, int S)
+{
+    if (S < 1) return true;
+    const ChebPairs p = cheb_pairs(col_cheb(o, (float)c->coef.c0, (float)c->coef.x1, (float)c->coef.y1, (float)c->coef.z1), S);
+    return level_growth(p, S) <= 0x1p60 && std::fabs(p.zs.x) >= 0x1p-126f;
+}
+
 static bool plane_plan(const les_ctx* c, const les_pcg_opts* o, int S, PlaneMap& a, PlaneMap& b)
 {
     const Geo& g = c->g;
@@ -149,15 +178,17 @@ static bool plane_plan(const les_ctx* c, const les_pcg_opts* o, int S, PlaneMap&
 // faster on every grid measured, 24x16x16 to 512x256x256, rows of 16 to 512
 // cells, Jacobi and degrees 3 to 7 (1.10 to 2.07 times, les_plane.cuh).  The
 // strips run where a caller asked for a strip shape or the autotuner found
-// one faster, in batched ensembles, and for vectors of 4 GB and more (32-bit
-// byte offsets).
+// one faster, in batched ensembles, for vectors of 4 GB and more (32-bit byte
+// offsets) and for spacings whose scaled levels would leave FP32 (levels_fit).
 bool plane_used(const les_ctx* c, const les_pcg_opts* o)
 {
     if (!col_supported(c, o)) return false;
     if ((unsigned long long)c->g.nx * c->g.ny * plane_pitch(c->g.nz) >= (1ull << 30)) return false;
     if ((c->tune_tja || c->tune_tjb || c->tune_cia || c->tune_cib) && !c->tune_plane) return false;
+    const int S = o->precond == LES_PC_JACOBI ? 0 : o->degree - 1;
+    if (!levels_fit(c, o, S)) return false;
     PlaneMap a, b;
-    return plane_plan(c, o, o->precond == LES_PC_JACOBI ? 0 : o->degree - 1, a, b);
+    return plane_plan(c, o, S, a, b);
 }
 
 les_status plane_maps(les_ctx* c, const les_pcg_opts* o, ColPlan& P)
