@@ -351,6 +351,7 @@ __device__ bool ic_tile(const Wave& W, int t, int base, const T* __restrict__ re
                 sg.fail = 1;
                 break;
             }
+            __syncwarp();   // the lanes that waited order the others' loads and stores (a vote orders nothing)
             const int sl = n & (RING - 1);
             T zj[IWB], zk = T(0);
 #pragma unroll
