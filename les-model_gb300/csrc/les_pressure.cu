@@ -440,13 +440,14 @@ __global__ void k_cheb_step(Geo g, StencilView A, int ci, double alpha, double b
 // [1, n-2] and g(i, j', k') = P(1, j', k') for i == 0, 0 for i == nx-1,
 // P(i, j', k') otherwise (P: the values before the call).  `in` may equal
 // `out` (faces read interior cells only).
+// (One-dimensional blocks: GS-SOR ends here on grids of any number of planes.)
 __global__ void k_pbc_faces(Geo g, const double* in, double* out)
 {
-    int i, j, k;
-    if (!cell_coords(g, i, j, k)) return;
+    const int id = blockIdx.x * blockDim.x + threadIdx.x;
+    if (id >= g.n) return;
+    const int i = id / g.si, r = id - i * g.si, j = r / g.sj, k = r - j * g.sj;
     bool jk_in = j >= 1 && j <= g.ny - 2 && k >= 1 && k <= g.nz - 2;
     if (jk_in && i > 0 && i < g.nx - 1) return;
-    const int id = i * g.si + j * g.sj + k;
     if (i == g.nx - 1) { out[id] = 0.0; return; }
     int jj = j < 1 ? 1 : (j > g.ny - 2 ? g.ny - 2 : j);
     int kk = k < 1 ? 1 : (k > g.nz - 2 ? g.nz - 2 : k);
@@ -702,7 +703,7 @@ les_status div_b_dev(les_ctx* c, double dt, double rho, double rel_tol, const do
 
 les_status pressure_bcs_dev(les_ctx* c, double* p)
 {
-    launch(c, k_pbc_faces, cell_grid(c->g), cell_block(), c->g, p, p);
+    launch(c, k_pbc_faces, (c->g.n + 255) / 256, 256, c->g, p, p);
     if (c->n_solid)
         launch(c, k_pbc_obstacle, (c->n_solid + 255) / 256, 256, c->g, c->solid_list, c->n_solid,
                                                                           c->mask, p);

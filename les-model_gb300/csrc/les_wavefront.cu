@@ -476,14 +476,32 @@ __global__ void __launch_bounds__(IC_THREADS) k_ic_wave(Wave W, int base, const 
         ok = ic_tile<T, -1>(W, W.ntiles - 1 - t, base + W.steps + 1, rec, zs, sg);
 }
 
+// One thread per cell of the grid, in a one-dimensional grid of blocks (the
+// other dimensions end at 65535 blocks, a wavefront's planes need not).
+constexpr int FLAT = 256;
+inline unsigned flat_grid(const Geo& g) { return (unsigned)((g.n + FLAT - 1) / FLAT); }
+struct CellAt {
+    int id, i, j, k;
+};
+__device__ __forceinline__ bool flat_cell(const Geo& g, CellAt& c)
+{
+    c.id = blockIdx.x * FLAT + threadIdx.x;
+    if (c.id >= g.n) return false;
+    c.i = c.id / g.si;
+    const int r = c.id - c.i * g.si;
+    c.j = r / g.sj;
+    c.k = r - c.j * g.sj;
+    return true;
+}
+
 // The records of a factor (its FP64 diagonals).
 template <typename T>
 __global__ void k_ic_records(Geo g, Skew sk, const double* __restrict__ Lc, const double* __restrict__ Lw,
                              const double* __restrict__ Ls, const double* __restrict__ Lb, T* __restrict__ rec)
 {
-    const int k = blockIdx.x * TBK + threadIdx.x, j = blockIdx.y * TBJ + threadIdx.y, i = blockIdx.z;
-    if (k >= g.nz || j >= g.ny) return;
-    const int id = i * g.si + j * g.sj + k;
+    CellAt q;
+    if (!flat_cell(g, q)) return;
+    const int id = q.id, i = q.i, j = q.j, k = q.k;
     const size_t at = sk.at(i, j, k);
     T* const r = rec + at / WT * (REC * WT) + at % WT;
     const T c = (T)Lc[id];
@@ -503,9 +521,9 @@ __global__ void k_ic_skew(Geo g, Skew sk, const T* __restrict__ from, T* __restr
                           int skip_done)
 {
     if (skip_done && st && st->done) return;
-    const int k = blockIdx.x * TBK + threadIdx.x, j = blockIdx.y * TBJ + threadIdx.y, i = blockIdx.z;
-    if (k >= g.nz || j >= g.ny) return;
-    const int id = i * g.si + j * g.sj + k;
+    CellAt q;
+    if (!flat_cell(g, q)) return;
+    const int id = q.id, i = q.i, j = q.j, k = q.k;
     if (IN) to[sk.at(i, j, k)] = from[id];
     else to[id] = from[sk.at(i, j, k)];
 }
@@ -785,45 +803,47 @@ __device__ __forceinline__ int first_fluid(const uint8_t* solid, int id, int si,
     return 6;
 }
 
-// One thread per column and word of 32 planes.
+// One thread per column, its words of 32 planes shared out along y.
 __global__ void k_gs_flags(int nx, int ny, int nz, const uint8_t* __restrict__ solid, unsigned* __restrict__ rd,
                            unsigned* __restrict__ wr, uint8_t* __restrict__ fl)
 {
     const int si = ny * nz, sj = nz;
-    const int col = blockIdx.x * blockDim.x + threadIdx.x, wi = blockIdx.y;
+    const int col = blockIdx.x * blockDim.x + threadIdx.x;
     if (col >= si) return;
     const int j = col / nz, k = col - j * nz;
-    unsigned r = 0u, w = 0u;
     auto interior = [&](int i, int jj, int kk) {
         return i >= 1 && i <= nx - 2 && jj >= 1 && jj <= ny - 2 && kk >= 1 && kk <= nz - 2;
     };
-    for (int b = 0; b < 32; ++b) {
-        const int i = wi * 32 + b;
-        if (i >= nx) break;
-        const int id = i * si + col;
-        unsigned f = 0u;
-        if (interior(i, j, k)) {
-            if (solid[id]) {
-                const int q = first_fluid(solid, id, si, sj);
-                const int di[7] = {1, -1, 0, 0, 0, 0, 0}, dj[7] = {0, 0, 1, -1, 0, 0, 0}, dk[7] = {0, 0, 0, 0, 1, -1, 0};
-                if (q < 6) {
-                    if (interior(i + di[q], j + dj[q], k + dk[q])) r |= 1u << b;
-                    else if (q == 0) { r |= 1u << b; f = 128u; }   // the outlet face
+    for (int wi = blockIdx.y; wi * 32 < nx; wi += gridDim.y) {
+        unsigned r = 0u, w = 0u;
+        for (int b = 0; b < 32; ++b) {
+            const int i = wi * 32 + b;
+            if (i >= nx) break;
+            const int id = i * si + col;
+            unsigned f = 0u;
+            if (interior(i, j, k)) {
+                if (solid[id]) {
+                    const int q = first_fluid(solid, id, si, sj);
+                    const int di[7] = {1, -1, 0, 0, 0, 0, 0}, dj[7] = {0, 0, 1, -1, 0, 0, 0}, dk[7] = {0, 0, 0, 0, 1, -1, 0};
+                    if (q < 6) {
+                        if (interior(i + di[q], j + dj[q], k + dk[q])) r |= 1u << b;
+                        else if (q == 0) { r |= 1u << b; f = 128u; }   // the outlet face
+                    }
+                } else {   // the solid neighbours this cell is the first fluid neighbour of
+                    if (interior(i + 1, j, k) && solid[id + si] && first_fluid(solid, id + si, si, sj) == 1) f |= 1u;
+                    if (interior(i - 1, j, k) && solid[id - si] && first_fluid(solid, id - si, si, sj) == 0) f |= 2u;
+                    if (interior(i, j + 1, k) && solid[id + sj] && first_fluid(solid, id + sj, si, sj) == 3) f |= 4u;
+                    if (interior(i, j - 1, k) && solid[id - sj] && first_fluid(solid, id - sj, si, sj) == 2) f |= 8u;
+                    if (interior(i, j, k + 1) && solid[id + 1] && first_fluid(solid, id + 1, si, sj) == 5) f |= 16u;
+                    if (interior(i, j, k - 1) && solid[id - 1] && first_fluid(solid, id - 1, si, sj) == 4) f |= 32u;
                 }
-            } else {   // the solid neighbours this cell is the first fluid neighbour of
-                if (interior(i + 1, j, k) && solid[id + si] && first_fluid(solid, id + si, si, sj) == 1) f |= 1u;
-                if (interior(i - 1, j, k) && solid[id - si] && first_fluid(solid, id - si, si, sj) == 0) f |= 2u;
-                if (interior(i, j + 1, k) && solid[id + sj] && first_fluid(solid, id + sj, si, sj) == 3) f |= 4u;
-                if (interior(i, j - 1, k) && solid[id - sj] && first_fluid(solid, id - sj, si, sj) == 2) f |= 8u;
-                if (interior(i, j, k + 1) && solid[id + 1] && first_fluid(solid, id + 1, si, sj) == 5) f |= 16u;
-                if (interior(i, j, k - 1) && solid[id - 1] && first_fluid(solid, id - 1, si, sj) == 4) f |= 32u;
             }
+            if (f) w |= 1u << b;
+            fl[id] = (uint8_t)f;
         }
-        if (f) w |= 1u << b;
-        fl[id] = (uint8_t)f;
+        rd[(size_t)wi * si + col] = r;
+        wr[(size_t)wi * si + col] = w;
     }
-    rd[(size_t)wi * si + col] = r;
-    wr[(size_t)wi * si + col] = w;
 }
 
 // Skewed copies: p's interior and the right-hand side, src/pressure.cpp:197-210.
@@ -831,9 +851,10 @@ __global__ void k_gs_skew(Geo g, Skew sk, double coef, DivBy two_dx, DivBy two_d
                           const double* __restrict__ u, const double* __restrict__ v, const double* __restrict__ w,
                           const double* __restrict__ p, double* __restrict__ ps, double* __restrict__ rhs)
 {
-    const int k = blockIdx.x * TBK + threadIdx.x, j = blockIdx.y * TBJ + threadIdx.y, i = blockIdx.z;
+    CellAt q;
+    if (!flat_cell(g, q)) return;
+    const int id = q.id, i = q.i, j = q.j, k = q.k;
     if (i < 1 || i > g.nx - 2 || j < 1 || j > g.ny - 2 || k < 1 || k > g.nz - 2) return;
-    const int id = i * g.si + j * g.sj + k;
     const size_t at = sk.at(i - 1, j - 1, k - 1);
     const double div = div_by(u[id + g.si] - u[id - g.si], two_dx) + div_by(v[id + g.sj] - v[id - g.sj], two_dy) +
                        div_by(w[id + 1] - w[id - 1], two_dz);
@@ -843,9 +864,11 @@ __global__ void k_gs_skew(Geo g, Skew sk, double coef, DivBy two_dx, DivBy two_d
 
 __global__ void k_gs_unskew(Geo g, Skew sk, const double* __restrict__ ps, double* __restrict__ p)
 {
-    const int k = blockIdx.x * TBK + threadIdx.x, j = blockIdx.y * TBJ + threadIdx.y, i = blockIdx.z;
+    CellAt q;
+    if (!flat_cell(g, q)) return;
+    const int i = q.i, j = q.j, k = q.k;
     if (i < 1 || i > g.nx - 2 || j < 1 || j > g.ny - 2 || k < 1 || k > g.nz - 2) return;
-    p[i * g.si + j * g.sj + k] = ps[sk.at(i - 1, j - 1, k - 1)];
+    p[q.id] = ps[sk.at(i - 1, j - 1, k - 1)];
 }
 
 // What a batch may have to go back to: p's interior and faces, and the old
@@ -1107,7 +1130,7 @@ static les_status ic_records(les_ctx* c, const double* const* L)
     const Skew sk = ic_skew(c, &len);
     les_status st = skew_buffer(c, (REC + 1) * len);   // records, then the vector (FP32 takes half)
     if (st) return st;
-    launch(c, k_ic_records<T>, cell_grid(c->g), cell_block(), c->g, sk, L[0], L[4], L[2], L[6],
+    launch(c, k_ic_records<T>, flat_grid(c->g), FLAT, c->g, sk, L[0], L[4], L[2], L[6],
            reinterpret_cast<T*>(c->skew_buf));
     return check_launch(c, "ic records");
 }
@@ -1136,10 +1159,10 @@ static les_status ic_apply(les_ctx* c, const T* r, T* z, const SolverState* stat
     if ((st = wave_resident(c, fn, IC_THREADS, smem, &resident))) return st;
     const int grid = W.ntiles < resident ? W.ntiles : resident;
     GridSync gs = grid_sync(c, grid);
-    launch(c, k_ic_skew<T, true>, cell_grid(c->g), cell_block(), c->g, sk, r, zs, state, skip_done);
+    launch(c, k_ic_skew<T, true>, flat_grid(c->g), FLAT, c->g, sk, r, zs, state, skip_done);
     void* args[] = {&W, &base, (void*)&rec, (void*)&zs, &gs, (void*)&state, &skip_done};
     if ((st = wave_launch(c, fn, args, grid, IC_THREADS, smem, PROF_IC))) return st;
-    launch(c, k_ic_skew<T, false>, cell_grid(c->g), cell_block(), c->g, sk, (const T*)zs, z, state, skip_done);
+    launch(c, k_ic_skew<T, false>, flat_grid(c->g), FLAT, c->g, sk, (const T*)zs, z, state, skip_done);
     return check_launch(c, "ic apply");
 }
 
@@ -1246,18 +1269,18 @@ les_status solve_gs_dev(les_ctx* c, double dt, double rho, int max_iter, double 
     const int grid = a.nb * Q;
     a.gs = grid_sync(c, grid);
     const Skew sk{a.W.wj, a.W.steps};
-    launch(c, k_gs_skew, cell_grid(g), cell_block(), g, sk, rho / dt, div_by_const(2 * m.dx), div_by_const(2 * m.dy),
+    launch(c, k_gs_skew, flat_grid(g), FLAT, g, sk, rho / dt, div_by_const(2 * m.dx), div_by_const(2 * m.dy),
            div_by_const(2 * m.dz), (const double*)c->slot[LES_U], (const double*)c->slot[LES_V],
            (const double*)c->slot[LES_W], (const double*)a.p, a.ps, rhs);
     if (c->n_solid)
-        launch(c, k_gs_flags, dim3((g.si + 255) / 256, words), 256, g.nx, g.ny, g.nz, (const uint8_t*)c->mask, rd,
+        launch(c, k_gs_flags, dim3((g.si + 255) / 256, words < 65535 ? words : 65535), 256, g.nx, g.ny, g.nz, (const uint8_t*)c->mask, rd,
                rd + (size_t)words * g.si, fl);
     if ((st = check_launch(c, "gs set-up"))) return st;
     void* args[] = {&a, &base};
     if (max_iter > 0) {
         st = wave_launch(c, fn, args, grid, WT, 0, -1);
         if (st) return st;
-        launch(c, k_gs_unskew, cell_grid(g), cell_block(), g, sk, (const double*)a.ps, a.p);
+        launch(c, k_gs_unskew, flat_grid(g), FLAT, g, sk, (const double*)a.ps, a.p);
         if ((st = pressure_bcs_dev(c, a.p))) return st;   // of the last sweep
     }
     st = check_barrier(c);
