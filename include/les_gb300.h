@@ -387,10 +387,18 @@ typedef enum les_option {
                              (about 2 s) gives up; the solve then returns LES_TIMEOUT
                              and the context stays usable.  For testing the failure
                              path only. */
-    LES_OPT_COL_STRIDE = 10 /* 1 (default): the register-column strips of a grid with
+    LES_OPT_COL_STRIDE = 10, /* 1 (default): the register-column strips of a grid with
                              nz = 32, 64, 128 or 256 run kernels compiled for that row
                              stride (row offsets as immediates); 0: the kernels that
                              read the stride at run time.  Same results either way. */
+    LES_OPT_WAVE_COPIES = 11 /* 1 (default): GS-SOR and the IC(0) applies run on copies of
+                             their operands in the order of the wavefront: five FP64
+                             arrays for GS-SOR, nine for IC(0) (FP32 in a mixed solve),
+                             each padded to whole tiles.  Up to 1 GB of them stays with
+                             the context from solve to solve.  0, and whenever the
+                             memory cannot be had: on the fields' own arrays, slower
+                             (IC(0) 1.25 to 1.5 times, GS-SOR 5 times).  Same results
+                             either way. */
 } les_option;
 les_status les_set_option(les_ctx* ctx, int option, int value);
 /* The current value of an option: the last one set, the default, or for the

@@ -382,7 +382,7 @@ __global__ void k_adj_sgs_gather(Geo g, Dx d, const double* __restrict__ hxx, co
 les_status alloc(les_ctx* c, double** p, size_t n)
 {
     if (*p) return LES_OK;
-    return check_cuda(c, cudaMalloc(p, sizeof(double) * n), "cudaMalloc(adjoint)");
+    return check_cuda(c, dev_malloc(c, p, sizeof(double) * n), "cudaMalloc(adjoint)");
 }
 
 les_status copy(les_ctx* c, double* dst, const double* src)

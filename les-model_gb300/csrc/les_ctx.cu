@@ -47,11 +47,22 @@ int reduction_blocks(const Geo& g)
     return (int)(gr.x * gr.y * gr.z);
 }
 
+cudaError_t dev_malloc_bytes(les_ctx* c, void** p, size_t bytes)
+{
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation && c->skew_buf) {
+        cudaGetLastError();
+        skew_free(c);
+        e = cudaMalloc(p, bytes);
+    }
+    return e;
+}
+
 les_status ensure_work(les_ctx* c)
 {
     if (c->w[0]) return LES_OK;
     for (int q = 0; q < 8; ++q) {
-        cudaError_t e = cudaMalloc(&c->w[q], sizeof(double) * (size_t)c->g.n);
+        cudaError_t e = dev_malloc(c, &c->w[q], sizeof(double) * (size_t)c->g.n);
         if (e != cudaSuccess) return check_cuda(c, e, "cudaMalloc(work)");
         cudaMemsetAsync(c->w[q], 0, sizeof(double) * (size_t)c->g.n, c->stream);
     }
@@ -63,7 +74,7 @@ les_status ensure_work32(les_ctx* c)
     if (c->f[0]) return LES_OK;
     for (int q = 0; q < 8; ++q) {
         const size_t bytes = sizeof(float) * (size_t)c->g.nx * c->g.ny * plane_pitch(c->g.nz);   // rows may be padded
-        cudaError_t e = cudaMalloc(&c->f[q], bytes);
+        cudaError_t e = dev_malloc(c, &c->f[q], bytes);
         if (e != cudaSuccess) return check_cuda(c, e, "cudaMalloc(work32)");
         cudaMemsetAsync(c->f[q], 0, bytes, c->stream);
     }
@@ -373,7 +384,7 @@ static les_status put_diag7(les_ctx* c, double** dst, const double* const* src)
     const size_t nb = sizeof(double) * (size_t)c->g.n;
     for (int q = 0; q < 7; ++q) {
         if (!dst[q]) {
-            les_status st = check_cuda(c, cudaMalloc(&dst[q], nb), "cudaMalloc(diag)");
+            les_status st = check_cuda(c, dev_malloc(c, &dst[q], nb), "cudaMalloc(diag)");
             if (st) return st;
         }
         les_status st = check_cuda(c, cudaMemcpyAsync(dst[q], src[q], nb, cudaMemcpyHostToDevice, c->stream),
@@ -421,6 +432,10 @@ les_status les_set_option(les_ctx* c, int option, int value)
     case LES_OPT_PHYS32: c->phys32 = value ? 1 : 0; return LES_OK;
     case LES_OPT_TEST_STALL: c->test_stall = value ? 1 : 0; return LES_OK;
     case LES_OPT_COL_STRIDE: c->col_stride = value ? 1 : 0; return LES_OK;
+    case LES_OPT_WAVE_COPIES:
+        c->wave_copies = value ? 1 : 0;
+        if (!value) skew_free(c);
+        return LES_OK;
     case LES_OPT_FUSED: c->fused = value == 2 ? 2 : (value ? 1 : 0); return LES_OK;
     case LES_OPT_TMA: c->opt_tma = value ? 1 : 0; return LES_OK;
     case LES_OPT_ROWS_A: c->tune_tja = value; c->tune_plane = 0; return LES_OK;
@@ -439,6 +454,7 @@ les_status les_get_option(const les_ctx* c, int option, int* value)
     case LES_OPT_PDL: *value = c->pdl; return LES_OK;
     case LES_OPT_PHYS32: *value = c->phys32; return LES_OK;
     case LES_OPT_TEST_STALL: *value = c->test_stall; return LES_OK;
+    case LES_OPT_WAVE_COPIES: *value = c->wave_copies; return LES_OK;
     case LES_OPT_COL_STRIDE: *value = c->col_stride; return LES_OK;
     case LES_OPT_FUSED: *value = c->fused; return LES_OK;
     case LES_OPT_TMA: *value = c->opt_tma; return LES_OK;

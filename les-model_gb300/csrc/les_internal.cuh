@@ -355,6 +355,7 @@ struct les_ctx {
     int wave_epoch = 0;
     double* skew_buf = nullptr;   // skewed arrays (les_wavefront.cu): GS-SOR's vectors, the IC records
     size_t skew_len = 0;
+    int wave_copies = 1;          // LES_OPT_WAVE_COPIES
     std::string err;
     // accounting: kernel launches issued by this context, and optional CUDA
     // event timing of the solver's hot kernels (les_profile)
@@ -473,6 +474,19 @@ unsigned long long graph_step_stats(les_ctx* c, const les_step_params* prm, unsi
                                     les_step_stats* stats);
 les_status read_state(les_ctx* c);
 int reduction_blocks(const Geo& g);
+
+// the wavefronts' skewed arrays (les_wavefront.cu): freed; freed if large
+void skew_free(les_ctx* c);
+void skew_trim(les_ctx* c);
+// cudaMalloc that gives those arrays up before it fails: for what a context
+// allocates outside an IC(0) solve (its records live from ic_records to the last
+// apply)
+cudaError_t dev_malloc_bytes(les_ctx* c, void** p, size_t bytes);
+template <class T>
+cudaError_t dev_malloc(les_ctx* c, T** p, size_t bytes)
+{
+    return dev_malloc_bytes(c, reinterpret_cast<void**>(p), bytes);
+}
 
 // kernels shared across translation units (les_pressure.cu)
 les_status spmv_dev(les_ctx* c, const double* in, double* out);

@@ -31,7 +31,7 @@ using namespace les;
 namespace les {
 les_status ensure_stored_A(les_ctx* c);
 les_status ic_records32(les_ctx* c, const double* const* L);
-les_status ic_apply_dev32(les_ctx* c, const float* r, float* z, SolverState* st);
+les_status ic_apply_dev32(les_ctx* c, const double* const* L, const float* r, float* z, SolverState* st);
 les_status wave_check(les_ctx* c);
 }
 
@@ -352,7 +352,7 @@ les_status ensure_f32_copy(les_ctx* c, float** dst, double* const* src)
     for (int q = 0; q < 7; ++q) {
         if (!src[q]) continue;
         if (!dst[q]) {
-            les_status st = check_cuda(c, cudaMalloc(&dst[q], sizeof(float) * (size_t)n), "cudaMalloc(f32 copy)");
+            les_status st = check_cuda(c, dev_malloc(c, &dst[q], sizeof(float) * (size_t)n), "cudaMalloc(f32 copy)");
             if (st) return st;
         }
         launch(c, k_to_f, (n + 255) / 256, 256, n, src[q], dst[q]);
@@ -393,7 +393,8 @@ static les_status inner_precond(les_ctx* c, const les_pcg_opts* o, ViewF A, floa
         return check_launch(c, "inner chebyshev");
     }
     // IC: wavefront solve in FP32, then r.z
-    les_status st = ic_apply_dev32(c, r, z, skip_done ? in : nullptr);
+    les_status st = ic_apply_dev32(c, (const double* const*)(o->precond == LES_PC_IC ? c->L : c->A), r, z,
+                                   skip_done ? in : nullptr);
     if (st) return st;
     launch(c, k_in_dot_beta, gr, bl, g, r, z, c->partials, c->counters + 13, in, init);
     return check_launch(c, "inner ic");
@@ -501,6 +502,7 @@ les_status pcg_mixed_impl(les_ctx* c, const les_pcg_opts* o, les_pcg_result* res
     }
     if (mode == 2) {   // the IC wavefront's bounded waits
         st = wave_check(c);
+        skew_trim(c);
         if (st) return st;
     }
     const SolverState& h = c->h_state[0];

@@ -374,7 +374,7 @@ les_status sgs_nut_dev(les_ctx* c, double cs, int want_tau)
 {
     const Geo& g = c->g;
     if (want_tau && !c->tau) {
-        les_status st = check_cuda(c, cudaMalloc(&c->tau, sizeof(double) * 6 * (size_t)g.n), "cudaMalloc(tau)");
+        les_status st = check_cuda(c, dev_malloc(c, &c->tau, sizeof(double) * 6 * (size_t)g.n), "cudaMalloc(tau)");
         if (st) return st;
         cudaMemsetAsync(c->tau, 0, sizeof(double) * 6 * (size_t)g.n, c->stream);
     }
@@ -451,7 +451,7 @@ les_status les_sgs(les_ctx* c, double cs, int want_tau)
     cudaSetDevice(c->device);
     const Geo& g = c->g;
     if (want_tau && !c->tau) {
-        les_status st = check_cuda(c, cudaMalloc(&c->tau, sizeof(double) * 6 * (size_t)g.n), "cudaMalloc(tau)");
+        les_status st = check_cuda(c, dev_malloc(c, &c->tau, sizeof(double) * 6 * (size_t)g.n), "cudaMalloc(tau)");
         if (st) return st;
         cudaMemsetAsync(c->tau, 0, sizeof(double) * 6 * (size_t)g.n, c->stream);
     }

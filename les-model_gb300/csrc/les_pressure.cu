@@ -21,7 +21,7 @@ using namespace les;
 
 namespace les {
 les_status ic_records64(les_ctx* c, const double* const* L);
-les_status ic_apply_dev(les_ctx* c, const double* r, double* z, int skip_done);
+les_status ic_apply_dev(les_ctx* c, const double* const* L, const double* r, double* z, int skip_done);
 les_status wave_check(les_ctx* c);
 les_status build_ic_dev(les_ctx* c);
 les_status pcg_mixed(les_ctx* c, const les_pcg_opts* o, les_pcg_result* res);
@@ -761,7 +761,8 @@ static les_status precond_dot(les_ctx* c, const les_pcg_opts* o, const double* r
     }
     case LES_PC_IC:
     case LES_PC_IC_A:
-        st = ic_apply_dev(c, r, z, skip_done);   // with the records of ic_ready
+        // with the records of ic_ready
+        st = ic_apply_dev(c, (const double* const*)(o->precond == LES_PC_IC ? c->L : c->A), r, z, skip_done);
         break;
     default:
         return fail(c, LES_BAD_ARG, "unknown preconditioner");
@@ -782,7 +783,7 @@ les_status ensure_stored_A(les_ctx* c)
     const size_t nb = sizeof(double) * (size_t)c->g.n;
     for (int q = 0; q < 7; ++q)
         if (!c->A[q]) {
-            les_status st = check_cuda(c, cudaMalloc(&c->A[q], nb), "cudaMalloc(A)");
+            les_status st = check_cuda(c, dev_malloc(c, &c->A[q], nb), "cudaMalloc(A)");
             if (st) return st;
         }
     launch(c, k_expand_stencil, cell_grid(c->g), cell_block(), 
@@ -878,6 +879,7 @@ les_status pcg_fp64(les_ctx* c, const les_pcg_opts* o, les_pcg_result* res, int 
     }
     if (o->precond == LES_PC_IC || o->precond == LES_PC_IC_A) {   // the wavefront's bounded waits
         st = wave_check(c);
+        skew_trim(c);
         if (st) return st;
     }
     const SolverState& h = *c->h_state;
@@ -979,7 +981,7 @@ les_status les_build_stencil(les_ctx* c)
     if (!c) return LES_BAD_ARG;
     cudaSetDevice(c->device);
     if (!c->code) {
-        les_status st = check_cuda(c, cudaMalloc(&c->code, (size_t)c->g.n), "cudaMalloc(code)");
+        les_status st = check_cuda(c, dev_malloc(c, &c->code, (size_t)c->g.n), "cudaMalloc(code)");
         if (st) return st;
     }
     const les_mesh& m = c->mesh;
@@ -1014,7 +1016,7 @@ les_status les_get_stencil(les_ctx* c, double* const* diag7)
     const size_t nb = sizeof(double) * (size_t)c->g.n;
     double* tmp[7];
     for (int q = 0; q < 7; ++q) {
-        st = check_cuda(c, cudaMalloc(&tmp[q], nb), "cudaMalloc(tmp)");
+        st = check_cuda(c, dev_malloc(c, &tmp[q], nb), "cudaMalloc(tmp)");
         if (st) return st;
     }
     launch(c, k_expand_stencil, cell_grid(c->g), cell_block(), c->g, stencil_view(c), tmp[0], tmp[1],
@@ -1057,8 +1059,10 @@ les_status les_precond_apply(les_ctx* c, const les_pcg_opts* o, int in, int out)
     if (!c->stencil_mode && o->precond != LES_PC_IC) return fail(c, LES_BAD_ARG, "no matrix");
     les_status st = ic_ready(c, o);
     if (!st) st = precond_dev(c, o, c->slot[in], c->slot[out], 0);
-    if (!st && (o->precond == LES_PC_IC || o->precond == LES_PC_IC_A))
-        st = wave_check(c);   // waits for the wavefront: LES_TIMEOUT if a bounded wait gave up
+    if (o->precond == LES_PC_IC || o->precond == LES_PC_IC_A) {
+        if (!st) st = wave_check(c);   // waits for the wavefront: LES_TIMEOUT if a bounded wait gave up
+        skew_trim(c);
+    }
     return st;
 }
 

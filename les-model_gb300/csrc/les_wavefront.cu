@@ -255,7 +255,10 @@ struct Skew {
 // of which the forward solve reads the first five and the backward solve the
 // last five, and the right-hand side, overwritten by the result: 6 KB per step
 // (FP64), contiguous, copied eight steps ahead in 16-byte pieces.  The records
-// are laid out once per solve (ic_records).
+// are laid out once per solve (ic_records).  COPY = false: no records; the
+// operands are read from the factor's and the vectors' own arrays, cell by cell
+// (a context without the memory for the copies): 96x64x64 694 us an apply,
+// 256x128x128 2015.
 //
 // Roles: four warps compute; a fifth waits for the producers and brings their
 // values into shared memory, up to RING batches ahead, and a sixth publishes
@@ -315,8 +318,19 @@ __device__ __forceinline__ double ic_divide(double sum, double lc, double y)
 }
 __device__ __forceinline__ float ic_divide(float sum, float lc, float) { return sum / lc; }
 
-template <typename T, int DIR>
-__device__ bool ic_tile(const Wave& W, int t, int base, const T* __restrict__ rec, T* zs, IcStage<T>& sg)
+// A factor's own arrays (COPY = false)
+struct IcFactor {
+    const double *Lc, *Lw, *Ls, *Lb;
+};
+__device__ __forceinline__ void copy_in(double* smem, const double* gmem) { cp_async<8>(smem, gmem); }
+__device__ __forceinline__ void copy_in(float* smem, const float* gmem) { cp_async<4>(smem, gmem); }
+__device__ __forceinline__ void copy_in(float* smem, const double* gmem) { *smem = (float)__ldg(gmem); }
+
+// zs: the right-hand side, overwritten by the result, in the records' order;
+// COPY = false: the result z, and r the right-hand side of the forward solve.
+template <typename T, int DIR, bool COPY>
+__device__ bool ic_tile(const Wave& W, int t, int base, const T* __restrict__ rec, const IcFactor& L,
+                        const T* __restrict__ r_in, T* zs, IcStage<T>& sg)
 {
     constexpr unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -339,6 +353,8 @@ __device__ bool ic_tile(const Wave& W, int t, int base, const T* __restrict__ re
         const int q0 = lane & (IWB - 1), row0 = (lane / IWB) & (WAVE_TJ - 1);
         const T* const zk_at = zs + (size_t)(DIR > 0 ? t - W.wj : t + W.wj) * tile + row0 * 32 + (DIR > 0 ? 31 : 0);
         const int rj = DIR > 0 ? 0 : WAVE_TJ - 1;   // the row that needs the j-neighbour
+        // the same row and column of the grid
+        const int jn = J * WAVE_TJ + (DIR > 0 ? -1 : WAVE_TJ), kj = K * 32 + lane, kn = K * 32 + (DIR > 0 ? -1 : 32);
         for (int n = 0; n < batches; ++n) {
             const int tau0 = n * IWB, tend = min(tau0 + IWB, W.steps);
             bool ok = true;
@@ -358,13 +374,15 @@ __device__ bool ic_tile(const Wave& W, int t, int base, const T* __restrict__ re
             for (int q = 0; q < IWB; ++q) {
                 const int f = fstep(tau0 + q), i = f - lane - rj;
                 zj[q] = T(0);
-                if (d.dj >= 0 && i >= 0 && i < W.nx)
-                    zj[q] = __ldcg(zj_at + (size_t)(f + (DIR > 0 ? WAVE_TJ - 1 : 1 - WAVE_TJ)) * WT);
+                if (d.dj >= 0 && i >= 0 && i < W.nx && (COPY || kj < W.nz))
+                    zj[q] = __ldcg(COPY ? zj_at + (size_t)(f + (DIR > 0 ? WAVE_TJ - 1 : 1 - WAVE_TJ)) * WT
+                                        : zs + i * W.si + jn * W.sj + kj);
             }
             {
                 const int f = fstep(tau0 + q0), i = f - near - row0;
-                if (d.dk >= 0 && lane < IWB * WAVE_TJ && i >= 0 && i < W.nx)
-                    zk = __ldcg(zk_at + (size_t)(f + (DIR > 0 ? 31 : -31)) * WT);
+                if (d.dk >= 0 && lane < IWB * WAVE_TJ && i >= 0 && i < W.nx && (COPY || row0 < rows))
+                    zk = __ldcg(COPY ? zk_at + (size_t)(f + (DIR > 0 ? 31 : -31)) * WT
+                                     : zs + i * W.si + (J * WAVE_TJ + row0) * W.sj + kn);
             }
 #pragma unroll
             for (int q = 0; q < IWB; ++q) sg.zj[sl][q][lane] = zj[q];
@@ -388,7 +406,21 @@ __device__ bool ic_tile(const Wave& W, int t, int base, const T* __restrict__ re
         const bool jin = DIR > 0 ? j > 0 : j < W.ny - 1, kin = DIR > 0 ? k > 0 : k < W.nz - 1;
         constexpr int PER = 16 / sizeof(T), NREC = 5 * WT / PER, NALL = 6 * WT / PER;   // 16-byte pieces
         auto stage = [&](int tau) {
-            if (tau < W.steps) {
+            if (!COPY) {
+                const int i = fstep(tau) - lane - row;
+                if (tau < W.steps && cell && i >= 0 && i < W.nx) {
+                    const int id = i * W.si + j * W.sj + k;
+                    T* const to = &sg.v[tau & (WD - 1)][0][el];
+                    constexpr int F = DIR > 0 ? 0 : 2, C = DIR > 0 ? 3 : 0;
+                    // (factors of a missing neighbour are not used)
+                    copy_in(to + F * WT, L.Lw + id + (DIR > 0 || i == W.nx - 1 ? 0 : W.si));
+                    copy_in(to + (F + 1) * WT, L.Ls + id + (DIR > 0 || !jin ? 0 : W.sj));
+                    copy_in(to + (F + 2) * WT, L.Lb + id + (DIR > 0 || !kin ? 0 : 1));
+                    copy_in(to + C * WT, L.Lc + id);
+                    to[(C + 1) * WT] = T(0);   // no reciprocal: a division
+                    copy_in(to + 5 * WT, (DIR > 0 ? r_in : zs) + id);
+                }
+            } else if (tau < W.steps) {
                 const int f = fstep(tau), sl = tau & (WD - 1);
                 const T* const r = rec + ((size_t)t * W.steps + f) * (REC * WT) + (DIR > 0 ? 0 : 3 * WT);
                 const T* const z = zs + tb + (size_t)f * WT;
@@ -437,7 +469,7 @@ __device__ bool ic_tile(const Wave& W, int t, int base, const T* __restrict__ re
                 T out = T(0);
                 if (act) {
                     out = ic_divide(sum, sg.v[sl][C][el], sg.v[sl][C + 1][el]);
-                    zs[tb + (size_t)fstep(tau) * WT + el] = out;
+                    zs[COPY ? tb + (size_t)fstep(tau) * WT + el : (size_t)(i * W.si + j * W.sj + k)] = out;
                 }
                 prev = out;
                 sg.xs[tau & 1][w][lane] = out;
@@ -461,19 +493,20 @@ __device__ bool ic_tile(const Wave& W, int t, int base, const T* __restrict__ re
 // all tiles, one grid barrier, the backward solve.  T = double is the
 // reference's arithmetic; T = float serves the FP32 inner solve of the
 // mixed-precision path (st == nullptr: never skipped).
-template <typename T>
-__global__ void __launch_bounds__(IC_THREADS) k_ic_wave(Wave W, int base, const T* __restrict__ rec, T* zs, GridSync gs,
-                                                const SolverState* st, int skip_done)
+template <typename T, bool COPY>
+__global__ void __launch_bounds__(IC_THREADS) k_ic_wave(Wave W, int base, const T* __restrict__ rec, IcFactor L,
+                                                        const T* __restrict__ r, T* zs, GridSync gs,
+                                                        const SolverState* st, int skip_done)
 {
     if (skip_done && st && st->done) return;   // uniform across blocks: no barrier is entered
     extern __shared__ char ic_sm[];
     IcStage<T>& sg = *reinterpret_cast<IcStage<T>*>(ic_sm);
     const int b = blockIdx.x, nb = gridDim.x;  // one tile per block at a time
     bool ok = true;
-    for (int t = b; t < W.ntiles && ok; t += nb) ok = ic_tile<T, 1>(W, t, base, rec, zs, sg);
+    for (int t = b; t < W.ntiles && ok; t += nb) ok = ic_tile<T, 1, COPY>(W, t, base, rec, L, r, zs, sg);
     if (!grid_barrier(gs) || !ok) return;
     for (int t = b; t < W.ntiles && ok; t += nb)
-        ok = ic_tile<T, -1>(W, W.ntiles - 1 - t, base + W.steps + 1, rec, zs, sg);
+        ok = ic_tile<T, -1, COPY>(W, W.ntiles - 1 - t, base + W.steps + 1, rec, L, r, zs, sg);
 }
 
 // One thread per cell of the grid, in a one-dimensional grid of blocks (the
@@ -629,7 +662,11 @@ __device__ __forceinline__ void watch_old(Watch& w, const Wave& W, const int* pr
 
 // Sweep `s` of a batch over tile t, the solve's sweep number `num`.  base:
 // progress value of this sweep's start (the one before: base - steps - 1).
-template <int FORM>
+//
+// COPY = false: no copies (a context without the memory for them): ps is the
+// field itself and rhs, rep lie in the fields' layout; one sweep at a time, with
+// the divisions that serve any spacing.  256x128x128: 954 us per sweep.
+template <int FORM, bool COPY>
 __device__ bool gs_tile(const GsArgs& A, int t, int s, int num, int base, double one_m_omega, double omega_coef,
                         unsigned long long& maxr, GsStage& sg)
 {
@@ -677,11 +714,14 @@ __device__ bool gs_tile(const GsArgs& A, int t, int s, int num, int base, double
                 if ((rn >> (gi & 31)) & 1u) pn = rep_old;
                 if ((rt >> (gi & 31)) & 1u) pt = rep_old;
             }
-            const size_t at = tb + (size_t)tau * WT;
+            const int id = rb + i * ssi;
+            const size_t at = COPY ? tb + (size_t)tau * WT : (size_t)id;
             cp_async<8>(&sg.own[sl][w][lane], po + at);
             cp_async<8>(&sg.rhs[sl][w][lane], A.rhs + at);
-            if (last_row) cp_async<8>(&sg.north[sl][lane], wall_n ? p + rb + i * ssi + ssj : pn + nb + (size_t)(tau - w) * WT);
-            if (last_col) cp_async<8>(&sg.top[sl][w], wall_t ? p + rb + i * ssi + 1 : pt + ob + (size_t)(tau - lane) * WT);
+            if (last_row)
+                cp_async<8>(&sg.north[sl][lane], wall_n ? p + id + ssj : pn + (COPY ? nb + (size_t)(tau - w) * WT : id + ssj));
+            if (last_col)
+                cp_async<8>(&sg.top[sl][w], wall_t ? p + id + 1 : pt + (COPY ? ob + (size_t)(tau - lane) * WT : id + 1));
             if (i == 0) cp_async<8>(&sg.inlet[w][lane], p + rb - ssi);
         }
         cp_commit();
@@ -713,14 +753,14 @@ __device__ bool gs_tile(const GsArgs& A, int t, int s, int num, int base, double
             const int i = tau0 + q - lane;
             ps0[q] = 0.0;
             if (w == 0 && cell && i >= 0 && i < W.nx)
-                ps0[q] = __ldcg(d.dj >= 0 ? A.ps + (t - 1) * tile + (size_t)(tau0 + q + WAVE_TJ - 1) * WT + 32 * (WAVE_TJ - 1) + lane
+                ps0[q] = __ldcg(COPY && d.dj >= 0 ? A.ps + (t - 1) * tile + (size_t)(tau0 + q + WAVE_TJ - 1) * WT + 32 * (WAVE_TJ - 1) + lane
                                           : p + rb + i * ssi - ssj);
         }
         {
             const int q = lane & (WB - 1), i = tau0 + q - w;
             if (w < rows && i >= 0 && i < W.nx)
-                pb0 = __ldcg(d.dk >= 0 ? A.ps + (t - W.wj) * tile + (size_t)(tau0 + q + 31) * WT + w * 32 + 31
-                                       : p + W.off + jr * ssj + i * ssi - 1);
+                pb0 = __ldcg(COPY && d.dk >= 0 ? A.ps + (t - W.wj) * tile + (size_t)(tau0 + q + 31) * WT + w * 32 + 31
+                                       : p + W.off + jr * ssj + i * ssi + kb - 1);
         }
 #pragma unroll
         for (int q = 0; q < WB; ++q) {
@@ -747,9 +787,9 @@ __device__ bool gs_tile(const GsArgs& A, int t, int s, int num, int base, double
             else x = ((div_by(ew, A.dx) + div_by(ns, A.dy)) + div_by(tb2, A.dz)) - rh;
             const double v = one_m_omega * po + omega_coef * x;
             if (act) {
-                A.ps[tb + (size_t)tau * WT] = v;
-                // the faces next to this cell, src/pressure.cpp:14-72
                 const int id = rb + i * ssi;
+                A.ps[COPY ? tb + (size_t)tau * WT : (size_t)id] = v;
+                // the faces next to this cell, src/pressure.cpp:14-72
                 if (i == 0) p[id - ssi] = v;
                 if (i == W.nx - 1) p[id + ssi] = 0.0;
                 if (jr == 0) p[id - ssj] = v;
@@ -764,13 +804,16 @@ __device__ bool gs_tile(const GsArgs& A, int t, int s, int num, int base, double
                     }
                     if ((wo >> (gi & 31)) & 1u) {   // the source of solid cells, or solid next to the outlet
                         const unsigned f = A.fl[id];
-                        if (f & 1u) rep_new[sk.at(i + 1, jr, k)] = v;
-                        if (f & 2u) rep_new[sk.at(i - 1, jr, k)] = v;
-                        if (f & 4u) rep_new[sk.at(i, jr + 1, k)] = v;
-                        if (f & 8u) rep_new[sk.at(i, jr - 1, k)] = v;
-                        if (f & 16u) rep_new[sk.at(i, jr, k + 1)] = v;
-                        if (f & 32u) rep_new[sk.at(i, jr, k - 1)] = v;
-                        if (f & 128u) rep_new[sk.at(i, jr, k)] = 0.0;
+                        auto rep = [&](int di, int dj, int dk) -> double& {
+                            return rep_new[COPY ? sk.at(i + di, jr + dj, k + dk) : (size_t)(id + di * ssi + dj * ssj + dk)];
+                        };
+                        if (f & 1u) rep(1, 0, 0) = v;
+                        if (f & 2u) rep(-1, 0, 0) = v;
+                        if (f & 4u) rep(0, 1, 0) = v;
+                        if (f & 8u) rep(0, -1, 0) = v;
+                        if (f & 16u) rep(0, 0, 1) = v;
+                        if (f & 32u) rep(0, 0, -1) = v;
+                        if (f & 128u) rep(0, 0, 0) = 0.0;
                     }
                 }
                 // max over non-negative doubles by their bit patterns; NaN is not selected
@@ -846,7 +889,8 @@ __global__ void k_gs_flags(int nx, int ny, int nz, const uint8_t* __restrict__ s
     }
 }
 
-// Skewed copies: p's interior and the right-hand side, src/pressure.cpp:197-210.
+// p's interior (COPY) and the right-hand side, src/pressure.cpp:197-210.
+template <bool COPY>
 __global__ void k_gs_skew(Geo g, Skew sk, double coef, DivBy two_dx, DivBy two_dy, DivBy two_dz,
                           const double* __restrict__ u, const double* __restrict__ v, const double* __restrict__ w,
                           const double* __restrict__ p, double* __restrict__ ps, double* __restrict__ rhs)
@@ -855,10 +899,10 @@ __global__ void k_gs_skew(Geo g, Skew sk, double coef, DivBy two_dx, DivBy two_d
     if (!flat_cell(g, q)) return;
     const int id = q.id, i = q.i, j = q.j, k = q.k;
     if (i < 1 || i > g.nx - 2 || j < 1 || j > g.ny - 2 || k < 1 || k > g.nz - 2) return;
-    const size_t at = sk.at(i - 1, j - 1, k - 1);
+    const size_t at = COPY ? sk.at(i - 1, j - 1, k - 1) : (size_t)id;
     const double div = div_by(u[id + g.si] - u[id - g.si], two_dx) + div_by(v[id + g.sj] - v[id - g.sj], two_dy) +
                        div_by(w[id + 1] - w[id - 1], two_dz);
-    ps[at] = p[id];
+    if (COPY) ps[at] = p[id];
     rhs[at] = coef * div;
 }
 
@@ -911,7 +955,7 @@ __device__ void gs_backup(const GsArgs& A, int num, bool to, int gt, int gn)
     }
 }
 
-template <int FORM>
+template <int FORM, bool COPY>
 __global__ void __launch_bounds__(WT, FORM == GS_DIV ? 5 : 6) k_gs_wave(const __grid_constant__ GsArgs A, int base)
 {
     __shared__ GsStage sg;
@@ -926,7 +970,7 @@ __global__ void __launch_bounds__(WT, FORM == GS_DIV ? 5 : 6) k_gs_wave(const __
     while (done < A.max_iter && !converged) {
         if (!redo) {
             run = min(run, A.max_iter - done);
-            if (run > 1) gs_backup(A, done, true, gt, gn);
+            if (COPY && run > 1) gs_backup(A, done, true, gt, gn);
         }
         if (gt < GS_BATCH) A.gmax[gt] = 0ull;
         if (!grid_barrier(A.gs)) return;
@@ -934,7 +978,7 @@ __global__ void __launch_bounds__(WT, FORM == GS_DIV ? 5 : 6) k_gs_wave(const __
         for (int s = q0; s < run && ok; s += A.Q) {
             unsigned long long maxr = 0ull;
             for (int t = blk; t < W.ntiles && ok; t += A.nb)
-                ok = gs_tile<FORM>(A, t, s, done + s, epoch + s * (W.steps + 1), one_m_omega, omega_coef, maxr, sg);
+                ok = gs_tile<FORM, COPY>(A, t, s, done + s, epoch + s * (W.steps + 1), one_m_omega, omega_coef, maxr, sg);
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) {
                 const unsigned long long x = __shfl_xor_sync(0xffffffffu, maxr, o);
@@ -949,12 +993,12 @@ __global__ void __launch_bounds__(WT, FORM == GS_DIV ? 5 : 6) k_gs_wave(const __
             __syncthreads();
         }
         if (!grid_barrier(A.gs) || !ok) return;
-        epoch += GS_BATCH * (W.steps + 1);
+        epoch += (COPY ? GS_BATCH : 1) * (W.steps + 1);
         // the first sweep whose max|dp| is below tol (the same in every thread)
         int hit = run;
         for (int s = 0; s < run && hit == run; ++s)
             if (__longlong_as_double((long long)__ldcg(A.gmax + s)) < A.tol) hit = s;
-        if (hit < run - 1) {   // before the batch's last: run that many again from its start
+        if (COPY && hit < run - 1) {   // before the batch's last: run that many again from its start
             run = hit + 1;
             redo = true;
             gs_backup(A, done, false, gt, gn);
@@ -962,7 +1006,7 @@ __global__ void __launch_bounds__(WT, FORM == GS_DIV ? 5 : 6) k_gs_wave(const __
             done += run;
             converged = hit < run;
             redo = false;
-            run = min(2 * run, GS_BATCH);
+            if (COPY) run = min(2 * run, GS_BATCH);
         }
         if (!grid_barrier(A.gs)) return;   // every thread has read gmax; restored values are in place
     }
@@ -1101,16 +1145,36 @@ namespace les {
 // LES_TIMEOUT (and the flag cleared) if a wavefront wait gave up since the last check.
 les_status wave_check(les_ctx* c) { return check_barrier(c); }
 
-// The skewed arrays, kept from solve to solve.
-static les_status skew_buffer(les_ctx* c, size_t doubles)
+// The skewed arrays.  false: the context works without them (LES_OPT_WAVE_COPIES)
+// or the memory cannot be had; the solve then runs on the fields' own layout.
+// Arrays of up to SKEW_KEEP are kept from solve to solve, larger ones given back
+// at its end: cudaMalloc and cudaFree of 0.34 GB take 0.25 ms, of 1.3 GB 1.0 ms.
+constexpr size_t SKEW_KEEP = size_t(1) << 30;
+
+static bool skew_buffer(les_ctx* c, size_t doubles)
 {
-    if (c->skew_len >= doubles) return LES_OK;
+    if (!c->wave_copies) return false;
+    if (c->skew_len >= doubles) return true;
+    skew_free(c);
+    if (cudaMalloc(&c->skew_buf, sizeof(double) * doubles) != cudaSuccess) {
+        cudaGetLastError();
+        c->skew_buf = nullptr;
+        return false;
+    }
+    c->skew_len = doubles;
+    return true;
+}
+
+void skew_free(les_ctx* c)
+{
     cudaFree(c->skew_buf);
     c->skew_buf = nullptr;
     c->skew_len = 0;
-    les_status st = check_cuda(c, cudaMalloc(&c->skew_buf, sizeof(double) * doubles), "cudaMalloc(skewed arrays)");
-    if (!st) c->skew_len = doubles;
-    return st;
+}
+
+void skew_trim(les_ctx* c)
+{
+    if (sizeof(double) * c->skew_len > SKEW_KEEP) skew_free(c);
 }
 
 static Skew ic_skew(const les_ctx* c, size_t* len)
@@ -1121,6 +1185,13 @@ static Skew ic_skew(const les_ctx* c, size_t* len)
     return sk;
 }
 
+// doubles that hold the records and the vector
+template <typename T>
+static size_t ic_doubles(size_t len)
+{
+    return ((REC + 1) * len * sizeof(T) + sizeof(double) - 1) / sizeof(double);
+}
+
 // Lays out the records of the factor L (c, n, s, e, w, t, b) for the applies
 // that follow.
 template <typename T>
@@ -1128,8 +1199,7 @@ static les_status ic_records(les_ctx* c, const double* const* L)
 {
     size_t len;
     const Skew sk = ic_skew(c, &len);
-    les_status st = skew_buffer(c, (REC + 1) * len);   // records, then the vector (FP32 takes half)
-    if (st) return st;
+    if (!skew_buffer(c, ic_doubles<T>(len))) return LES_OK;
     launch(c, k_ic_records<T>, flat_grid(c->g), FLAT, c->g, sk, L[0], L[4], L[2], L[6],
            reinterpret_cast<T*>(c->skew_buf));
     return check_launch(c, "ic records");
@@ -1138,20 +1208,21 @@ static les_status ic_records(les_ctx* c, const double* const* L)
 les_status ic_records64(les_ctx* c, const double* const* L) { return ic_records<double>(c, L); }
 les_status ic_records32(les_ctx* c, const double* const* L) { return ic_records<float>(c, L); }
 
-// z = M^-1 r with the records laid out last.
+// z = M^-1 r with the factor L whose records were laid out last.
 template <typename T>
-static les_status ic_apply(les_ctx* c, const T* r, T* z, const SolverState* state, int skip_done)
+static les_status ic_apply(les_ctx* c, const double* const* L, const T* r, T* z, const SolverState* state, int skip_done)
 {
     size_t len;
     const Skew sk = ic_skew(c, &len);
-    if (c->skew_len < (REC + 1) * len) return fail(c, LES_BAD_ARG, "internal: no IC records");
+    const bool copy = c->wave_copies && c->skew_len >= ic_doubles<T>(len);
     const T* rec = reinterpret_cast<const T*>(c->skew_buf);
-    T* zs = reinterpret_cast<T*>(c->skew_buf) + REC * len;
+    T* zs = copy ? reinterpret_cast<T*>(c->skew_buf) + REC * len : z;
+    IcFactor F{L[0], L[4], L[2], L[6]};
     Wave W;
     int base = 0;
     les_status st = wave_setup(c, c->g.nx, c->g.ny, c->g.nz, 0, 2 * (c->g.nx + 32 + WAVE_TJ), 1, W, base);
     if (st) return st;
-    const void* fn = (const void*)k_ic_wave<T>;
+    const void* fn = copy ? (const void*)k_ic_wave<T, true> : (const void*)k_ic_wave<T, false>;
     const size_t smem = sizeof(IcStage<T>);
     st = check_cuda(c, cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "smem attribute");
     if (st) return st;
@@ -1159,21 +1230,21 @@ static les_status ic_apply(les_ctx* c, const T* r, T* z, const SolverState* stat
     if ((st = wave_resident(c, fn, IC_THREADS, smem, &resident))) return st;
     const int grid = W.ntiles < resident ? W.ntiles : resident;
     GridSync gs = grid_sync(c, grid);
-    launch(c, k_ic_skew<T, true>, flat_grid(c->g), FLAT, c->g, sk, r, zs, state, skip_done);
-    void* args[] = {&W, &base, (void*)&rec, (void*)&zs, &gs, (void*)&state, &skip_done};
+    if (copy) launch(c, k_ic_skew<T, true>, flat_grid(c->g), FLAT, c->g, sk, r, zs, state, skip_done);
+    void* args[] = {&W, &base, (void*)&rec, &F, (void*)&r, (void*)&zs, &gs, (void*)&state, &skip_done};
     if ((st = wave_launch(c, fn, args, grid, IC_THREADS, smem, PROF_IC))) return st;
-    launch(c, k_ic_skew<T, false>, flat_grid(c->g), FLAT, c->g, sk, (const T*)zs, z, state, skip_done);
+    if (copy) launch(c, k_ic_skew<T, false>, flat_grid(c->g), FLAT, c->g, sk, (const T*)zs, z, state, skip_done);
     return check_launch(c, "ic apply");
 }
 
-les_status ic_apply_dev(les_ctx* c, const double* r, double* z, int skip_done)
+les_status ic_apply_dev(les_ctx* c, const double* const* L, const double* r, double* z, int skip_done)
 {
-    return ic_apply<double>(c, r, z, c->state, skip_done);
+    return ic_apply<double>(c, L, r, z, c->state, skip_done);
 }
 
-les_status ic_apply_dev32(les_ctx* c, const float* r, float* z, SolverState* st)
+les_status ic_apply_dev32(les_ctx* c, const double* const* L, const float* r, float* z, SolverState* st)
 {
-    return ic_apply<float>(c, r, z, st, st ? 1 : 0);
+    return ic_apply<float>(c, L, r, z, st, st ? 1 : 0);
 }
 
 les_status build_ic_dev(les_ctx* c)
@@ -1181,7 +1252,7 @@ les_status build_ic_dev(les_ctx* c)
     const size_t nb = sizeof(double) * (size_t)c->g.n;
     for (int q = 0; q < 7; ++q) {
         if (!c->L[q]) {
-            les_status st = check_cuda(c, cudaMalloc(&c->L[q], nb), "cudaMalloc(L)");
+            les_status st = check_cuda(c, dev_malloc(c, &c->L[q], nb), "cudaMalloc(L)");
             if (st) return st;
         }
         cudaMemsetAsync(c->L[q], 0, nb, c->stream);
@@ -1211,30 +1282,35 @@ les_status solve_gs_dev(les_ctx* c, double dt, double rho, int max_iter, double 
     // x / d2 for a power of two d2 is exactly x * (1 / d2)
     auto pow2 = [](double v) { int e; return std::frexp(v, &e) == 0.5; };
     const bool p2 = pow2(dx2) && pow2(dy2) && pow2(dz2);
-    const void* fn = !p2 ? (const void*)k_gs_wave<GS_DIV>
-                         : (dx2 == dy2 && dy2 == dz2 ? (const void*)k_gs_wave<GS_EQUAL> : (const void*)k_gs_wave<GS_POW2>);
+    // the skewed arrays first: the work is split for the form that runs
+    const Skew sk{(g.ny - 2 + WAVE_TJ - 1) / WAVE_TJ, g.nx - 2 + 31 + WAVE_TJ - 1};
+    const int ntiles = sk.wj * ((g.nz - 2 + 31) / 32);
+    const size_t len = (size_t)ntiles * sk.steps * WT;
+    const bool copy = skew_buffer(c, 5 * len);
+    const void* fn = !copy ? (const void*)k_gs_wave<GS_DIV, false>
+                   : !p2   ? (const void*)k_gs_wave<GS_DIV, true>
+                   : (dx2 == dy2 && dy2 == dz2 ? (const void*)k_gs_wave<GS_EQUAL, true> : (const void*)k_gs_wave<GS_POW2, true>);
     int resident = 0;
     st = wave_resident(c, fn, WT, 0, &resident);
     if (st) return st;
     // Sweeps in flight: as many as there are resident blocks for, up to what a
     // sweep's length has room for (a sweep starts about 20 steps behind the
     // one before: the staging depth, the waits' granularity).
-    const int ntiles = ((g.ny - 2 + WAVE_TJ - 1) / WAVE_TJ) * ((g.nz - 2 + 31) / 32);
-    const int room = (g.nx - 2 + 31 + WAVE_TJ - 1) / 20 + 1;
-    int Q = resident / ntiles;
+    const int room = sk.steps / 20 + 1;
+    int Q = copy ? resident / ntiles : 1;
     Q = Q < 1 ? 1 : (Q > room ? room : Q);
     if (Q > GS_MAX_FLIGHT) Q = GS_MAX_FLIGHT;
     if (Q > max_iter && max_iter > 0) Q = max_iter;
     GsArgs a{};
     int base = 0;
     // progress values: every batch (about max_iter / GS_BATCH and the doubling
-    // ones before, one run again) takes GS_BATCH sweeps' worth
-    const long long batches = max_iter / GS_BATCH + 8;
-    st = wave_setup(c, g.nx - 2, g.ny - 2, g.nz - 2, g.si + g.sj + 1,
-                    batches * GS_BATCH * (long long)(g.nx - 2 + 32 + WAVE_TJ), Q, a.W, base);
+    // ones before, one run again) takes GS_BATCH sweeps' worth; without the
+    // copies a sweep takes its own
+    const long long sweeps_worth = copy ? (long long)(max_iter / GS_BATCH + 8) * GS_BATCH : max_iter;
+    st = wave_setup(c, g.nx - 2, g.ny - 2, g.nz - 2, g.si + g.sj + 1, sweeps_worth * (g.nx - 2 + 32 + WAVE_TJ), Q, a.W,
+                    base);
     if (st) return st;
-    a.len = (size_t)a.W.ntiles * a.W.steps * WT;
-    if ((st = skew_buffer(c, 5 * a.len))) return st;
+    a.len = len;
     const int words = (g.nx + 31) / 32;
     a.Q = Q;
     a.nb = ntiles < resident ? ntiles : resident;
@@ -1246,12 +1322,12 @@ les_status solve_gs_dev(les_ctx* c, double dt, double rho, int max_iter, double 
     a.tol = tol;
     a.max_iter = max_iter;
     a.p = c->slot[LES_P];
-    a.ps = c->skew_buf;
-    double* const rhs = c->skew_buf + a.len;
+    a.ps = copy ? c->skew_buf : a.p;
+    double* const rhs = copy ? c->skew_buf + len : c->w[4];
     a.rhs = rhs;
-    a.ps_back = c->skew_buf + 2 * a.len;
-    a.rep[0] = c->skew_buf + 3 * a.len;
-    a.rep[1] = c->skew_buf + 4 * a.len;
+    a.ps_back = copy ? c->skew_buf + 2 * len : nullptr;
+    a.rep[0] = copy ? c->skew_buf + 3 * len : c->w[5];
+    a.rep[1] = copy ? c->skew_buf + 4 * len : c->w[6];
     a.face_back = c->w[0];
     a.rep_back = c->w[1];
     unsigned* const rd = reinterpret_cast<unsigned*>(c->w[2]);   // two words per column and 32 planes: n doubles hold them
@@ -1268,8 +1344,7 @@ les_status solve_gs_dev(les_ctx* c, double dt, double rho, int max_iter, double 
     a.nz = g.nz;
     const int grid = a.nb * Q;
     a.gs = grid_sync(c, grid);
-    const Skew sk{a.W.wj, a.W.steps};
-    launch(c, k_gs_skew, flat_grid(g), FLAT, g, sk, rho / dt, div_by_const(2 * m.dx), div_by_const(2 * m.dy),
+    launch(c, copy ? k_gs_skew<true> : k_gs_skew<false>, flat_grid(g), FLAT, g, sk, rho / dt, div_by_const(2 * m.dx), div_by_const(2 * m.dy),
            div_by_const(2 * m.dz), (const double*)c->slot[LES_U], (const double*)c->slot[LES_V],
            (const double*)c->slot[LES_W], (const double*)a.p, a.ps, rhs);
     if (c->n_solid)
@@ -1280,13 +1355,14 @@ les_status solve_gs_dev(les_ctx* c, double dt, double rho, int max_iter, double 
     if (max_iter > 0) {
         st = wave_launch(c, fn, args, grid, WT, 0, -1);
         if (st) return st;
-        launch(c, k_gs_unskew, flat_grid(g), FLAT, g, sk, (const double*)a.ps, a.p);
+        if (copy) launch(c, k_gs_unskew, flat_grid(g), FLAT, g, sk, (const double*)a.ps, a.p);
         if ((st = pressure_bcs_dev(c, a.p))) return st;   // of the last sweep
     }
     st = check_barrier(c);
     if (st) return st;
     st = read_state(c);
     if (st) return st;
+    skew_trim(c);
     if (sweeps) *sweeps = max_iter > 0 ? c->h_state->iters : 0;
     return LES_OK;
 }
