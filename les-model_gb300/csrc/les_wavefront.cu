@@ -1095,7 +1095,7 @@ les_status wave_setup(les_ctx* c, int nx, int ny, int nz, int off, long long spa
         st = check_cuda(c, cudaMemsetAsync(c->wave_prog, 0, sizeof(int) * (size_t)len, c->stream), "memset");
         if (st) return st;
     }
-    if (span < 0 || span > (1 << 29)) return fail(c, LES_BAD_ARG, "wavefront: too many sweeps in one launch");
+    if (span < 0 || span > (1 << 30)) return fail(c, LES_BAD_ARG, "wavefront: too many sweeps in one launch");
     if (c->wave_epoch > (1 << 30) - (int)span) {   // restart the counters well before the int range ends
         les_status st = check_cuda(c, cudaMemsetAsync(c->wave_prog, 0, sizeof(int) * (size_t)c->wave_prog_len,
                                                       c->stream), "memset");
@@ -1282,11 +1282,14 @@ les_status solve_gs_dev(les_ctx* c, double dt, double rho, int max_iter, double 
     // x / d2 for a power of two d2 is exactly x * (1 / d2)
     auto pow2 = [](double v) { int e; return std::frexp(v, &e) == 0.5; };
     const bool p2 = pow2(dx2) && pow2(dy2) && pow2(dz2);
+    // progress values of a sweep, and the most sweeps of a solve
+    const long long per = g.nx - 2 + 32 + WAVE_TJ;
+    if (max_iter * per > (1 << 29)) return fail(c, LES_BAD_ARG, "wavefront: too many sweeps in one launch");
     // the skewed arrays first: the work is split for the form that runs
     const Skew sk{(g.ny - 2 + WAVE_TJ - 1) / WAVE_TJ, g.nx - 2 + 31 + WAVE_TJ - 1};
     const int ntiles = sk.wj * ((g.nz - 2 + 31) / 32);
     const size_t len = (size_t)ntiles * sk.steps * WT;
-    const bool copy = skew_buffer(c, 5 * len);
+    const bool copy = 8 * GS_BATCH * per <= (1 << 29) && skew_buffer(c, 5 * len);   // (room for the batches below)
     const void* fn = !copy ? (const void*)k_gs_wave<GS_DIV, false>
                    : !p2   ? (const void*)k_gs_wave<GS_DIV, true>
                    : (dx2 == dy2 && dy2 == dz2 ? (const void*)k_gs_wave<GS_EQUAL, true> : (const void*)k_gs_wave<GS_POW2, true>);
@@ -1307,8 +1310,7 @@ les_status solve_gs_dev(les_ctx* c, double dt, double rho, int max_iter, double 
     // ones before, one run again) takes GS_BATCH sweeps' worth; without the
     // copies a sweep takes its own
     const long long sweeps_worth = copy ? (long long)(max_iter / GS_BATCH + 8) * GS_BATCH : max_iter;
-    st = wave_setup(c, g.nx - 2, g.ny - 2, g.nz - 2, g.si + g.sj + 1, sweeps_worth * (g.nx - 2 + 32 + WAVE_TJ), Q, a.W,
-                    base);
+    st = wave_setup(c, g.nx - 2, g.ny - 2, g.nz - 2, g.si + g.sj + 1, sweeps_worth * per, Q, a.W, base);
     if (st) return st;
     a.len = len;
     const int words = (g.nx + 31) / 32;
