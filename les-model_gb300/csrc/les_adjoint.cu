@@ -641,8 +641,9 @@ les_status solve_linear(les_ctx* c, AdjWork& a, double* rhs, double* sol, const 
     c->slot[LES_B] = rhs;
     c->slot[LES_P] = sol;
     les_pcg_result r{};
-    if (o.precision == LES_MIXED && c->graph_on && !c->prof_on && c->stencil_mode == 1 && c->fused && fused_supported(&o) &&
-        o.max_iter > 0)
+    // (the TMA passes' waits may give up, which the host looks for after each inner solve)
+    if (o.precision == LES_MIXED && c->graph_on && !c->prof_on && c->stencil_mode == 1 && c->fused && !c->opt_tma &&
+        fused_supported(&o) && o.max_iter > 0)
         st = solve_graph(c, a, o, &r);
     else
         st = o.precision == LES_MIXED ? pcg_mixed_impl(c, &o, &r, 0) : pcg_fp64(c, &o, &r, 0);
