@@ -46,8 +46,9 @@ les_status pcg_fp64(les_ctx* c, const les_pcg_opts* o, les_pcg_result* res, int 
 les_status pcg_mixed_impl(les_ctx* c, const les_pcg_opts* o, les_pcg_result* res, int keep_tol);
 les_status dot_dev(les_ctx* c, const double* a, const double* b, double* out_host);
 
-// A captured mixed solve of one solution and right-hand side (its tolerance is
-// set on the device before each launch).
+// The captured mixed solve of the adjoint and tangent systems (its tolerance is
+// set on the device before each launch; the forward steps' solves are part of
+// les_step's own graph).
 struct SolveGraph {
     double *rhs = nullptr, *sol = nullptr;
     les_pcg_opts o{};
@@ -70,7 +71,7 @@ struct AdjWork {
     double* grad_in = nullptr;     // ny*nz
     double* acc = nullptr;         // [0] J, [1] dJ/dCs
     bool forward_done = false;
-    SolveGraph sg[2];              // the forward steps' solve, the adjoint's
+    SolveGraph sg;
 };
 
 void adj_work_free(AdjWork* a)
@@ -86,8 +87,7 @@ void adj_work_free(AdjWork* a)
     cudaFree(a->lb);
     cudaFree(a->grad_in);
     cudaFree(a->acc);
-    for (auto& g : a->sg)
-        if (g.exec) cudaGraphExecDestroy(g.exec);
+    if (a->sg.exec) cudaGraphExecDestroy(a->sg.exec);
     delete a;
 }
 }  // namespace les
@@ -584,7 +584,7 @@ les_status solve_graph(les_ctx* c, AdjWork& a, const les_pcg_opts& opts, les_pcg
     double *rhs = c->slot[LES_B], *sol = c->slot[LES_P];
     les_pcg_opts o = opts;
     o.tol = 0.0;
-    SolveGraph& g = a.sg[sol == a.lb ? 1 : 0];
+    SolveGraph& g = a.sg;
     if (!g.exec || g.version != c->version || g.rhs != rhs || g.sol != sol || std::memcmp(&g.o, &o, sizeof o)) {
         if (g.exec) cudaGraphExecDestroy(g.exec);
         g = SolveGraph{};
