@@ -382,11 +382,12 @@ typedef enum les_option {
                              in FP32 (FP64 fields, FP64 velocity update; not with
                              want_tau); 0: the reference-order FP64 kernels */
     LES_OPT_TEST_STALL = 9, /* test hook, 0 (default) off.  1: the first tile of the
-                             IC(0) and GS-SOR wavefronts withholds its progress, so
-                             the tiles after it wait in vain until their bounded wait
-                             (about 2 s) gives up; the solve then returns LES_TIMEOUT
-                             and the context stays usable.  For testing the failure
-                             path only. */
+                             IC(0) and GS-SOR wavefronts withholds its progress, and
+                             the first block of a cooperative FP64 PCG never arrives
+                             at the others' exchange, so the ones that wait for it
+                             wait in vain until their bounded wait (about 2 s) gives
+                             up; the solve then returns LES_TIMEOUT and the context
+                             stays usable.  For testing the failure path only. */
     LES_OPT_COL_STRIDE = 10, /* 1 (default): the register-column strips of a grid with
                              nz = 32, 64, 128 or 256 run kernels compiled for that row
                              stride (row offsets as immediates); 0: the kernels that

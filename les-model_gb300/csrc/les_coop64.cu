@@ -30,6 +30,7 @@ struct Meet {
     double* part;
     unsigned* count;
     int* err;
+    int stall;   // this block never arrives (LES_OPT_TEST_STALL)
     unsigned nb, number;
 };
 
@@ -84,7 +85,7 @@ __device__ __forceinline__ int meet(Meet& m, double (&v)[NV], double (*sm)[CT], 
 #pragma unroll
             for (int q = 0; q < NV; ++q) __stcg(s + q * m.nb + blockIdx.x, v[q]);
         __threadfence();   // the block's stores before the arrival
-        atomicAdd(m.count, 1u);
+        if (!m.stall) atomicAdd(m.count, 1u);
         const unsigned target = e * m.nb;
         unsigned spins = 0;
         unsigned long long t0 = 0;
@@ -160,6 +161,7 @@ struct Args {
     double* part;
     unsigned* count;
     int* err;
+    int stall;
     double tol;
     int keep_tol, max_iter, degree;        // degree 0: Jacobi
     double alpha0, alpha[MAX_STEPS], beta[MAX_STEPS];   // Chebyshev's coefficients, :878-899
@@ -172,7 +174,7 @@ __global__ void __launch_bounds__(CT, 1) k_pcg64(const __grid_constant__ Args a)
     __shared__ double sm[2][CT];
     __shared__ Scalars sc;
     const Geo& g = a.g;
-    Meet m{a.part, a.count, a.err, gridDim.x, 0};
+    Meet m{a.part, a.count, a.err, a.stall && blockIdx.x == 0, gridDim.x, 0};
     const int per = (g.n + (int)gridDim.x - 1) / (int)gridDim.x;
     const int c0 = (int)blockIdx.x * per + (int)threadIdx.x, c1 = min(g.n, ((int)blockIdx.x + 1) * per);
     const double tol = a.keep_tol ? a.st->tol : a.tol;
@@ -335,6 +337,7 @@ les_status pcg64_coop(les_ctx* c, const les_pcg_opts* o, bool pow2, int keep_tol
     a.pc = c->w[7];
     a.st = c->state;
     a.err = (int*)(c->gsync + 2);
+    a.stall = c->test_stall;
     a.tol = o->tol;
     a.keep_tol = keep_tol;
     a.max_iter = o->max_iter;
