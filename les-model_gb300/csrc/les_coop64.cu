@@ -308,10 +308,14 @@ const void* pick(bool plain, bool pow2)
 namespace les {
 
 // Cells up to which the cooperative form is taken.  Microseconds per iteration,
-// launch by launch and cooperative (GB300): Jacobi 64x32x32 26.5 / 13.3,
-// 96x48x48 47.9 / 21.4, 111x65x73 74.7 / 37.4, 128x128x64 71.0 / 51.6; Chebyshev
-// degree 4 64x32x32 48.0 / 28.0, 96x48x48 107 / 58, 111x65x73 188 / 113, degree 3
-// 128x128x64 133 / 123.  Beyond that the FP64 pipe bounds both.
+// launch by launch and cooperative (GB300), of Jacobi / Chebyshev degree 4:
+//   64x32x32     26.5 / 13.3     48 / 28      111x65x73   74.7 / 37.4   188 / 113
+//   80x80x80     65.6 / 36.6    155 / 111     (h = 0.01: no power of two, rows of
+//   100x100x100   102 / 61      269 / 195     thirteen operations instead of the
+//                                             launched kernels' eight to ten)
+//   128x128x64   71.0 / 51.5    162 / 154     degree 7 254 / 244, h = 0.01 363 / 337
+// It was also ahead at 160x128x100 (132 / 89, 342 / 283), the largest timed; the
+// line stays at the size up to which every degree and spacing was.
 constexpr long long COOP_CELLS = 1 << 20;
 
 bool pcg64_coop_used(const les_ctx* c, const les_pcg_opts* o)
