@@ -127,16 +127,18 @@ __device__ __forceinline__ void march_rows(const StencilView& A, const double* _
         const double pe = c.x1 * xe;
         __syncthreads();   // one barrier per plane: the planes alternate between two tiles
         if (in) {
+            // code 0: an identity row, every multiplier 0 (and 0 times an infinity NaN)
             const unsigned code = A.code[id];
-            const unsigned cd = code ? code - 1u : 0u, xs = cd % 5u, r = cd / 5u, ys = r & 3u, zs = r >> 2;
-            double val = c.c0 * xc;
+            const unsigned cd = code ? code - 1u : 3u, xs = cd % 5u, r = cd / 5u, ys = r & 3u, zs = r >> 2;
+            const unsigned lo = code ? YL_PACK : 0u, hi = code ? YH_PACK : 0u;
+            double val = (code ? c.c0 : 1.0) * xc;
             if (i > 0) val = fma(mult(XW_PACK, xs), pw, val);
             if (i < g.nx - 1) val = fma(mult(XE_PACK, xs), pe, val);
-            if (j > 0) val = fma(mult(YL_PACK, ys), ty[tj - 1][tk], val);
-            if (j < g.ny - 1) val = fma(mult(YH_PACK, ys), ty[tj + 1][tk], val);
-            if (k > 0) val = fma(mult(YL_PACK, zs), tz[tj][tk - 1], val);
-            if (k < g.nz - 1) val = fma(mult(YH_PACK, zs), tz[tj][tk + 1], val);
-            f(i, id, xc, code ? val : xc);   // code 0: identity row
+            if (j > 0) val = fma(mult(lo, ys), ty[tj - 1][tk], val);
+            if (j < g.ny - 1) val = fma(mult(hi, ys), ty[tj + 1][tk], val);
+            if (k > 0) val = fma(mult(lo, zs), tz[tj][tk - 1], val);
+            if (k < g.nz - 1) val = fma(mult(hi, zs), tz[tj][tk + 1], val);
+            f(i, id, xc, val);
         }
         xc = xe;
         pw = pc;
