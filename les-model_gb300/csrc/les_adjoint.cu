@@ -592,7 +592,7 @@ les_status solve_graph(les_ctx* c, AdjWork& a, const les_pcg_opts& opts, les_pcg
         cudaGraph_t graph = nullptr;
         st = check_cuda(c, cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeRelaxed), "begin solve capture");
         if (st) return st;
-        les_status st1 = capture_mixed_fused(c, &o, view32_of(c), 1);
+        les_status st1 = capture_mixed_fused(c, &o, view32_of(c), 1, true);
         st = check_cuda(c, cudaStreamEndCapture(c->stream, &graph), "end solve capture");
         if (st1) st = st1;
         if (!st) st = check_cuda(c, cudaGraphInstantiate(&g.exec, graph, 0), "instantiate solve graph");
@@ -613,6 +613,9 @@ les_status solve_graph(les_ctx* c, AdjWork& a, const les_pcg_opts& opts, les_pcg
     if ((st = check_cuda(c, cudaGraphLaunch(g.exec, c->stream), "launch solve graph")) || (st = read_state(c))) return st;
     c->launches += g.captured;   // one pass of each loop
     const SolverState& h = c->h_state[0];
+    // (without a correction the inner state is an earlier solve's)
+    if (h.k > 0 && c->h_state[1].status == LES_TIMEOUT)
+        return fail(c, LES_TIMEOUT, "a TMA wait in the inner solve timed out");
     r->iters = h.iters;
     r->outer = h.k;
     r->residual = h.err;
@@ -641,9 +644,8 @@ les_status solve_linear(les_ctx* c, AdjWork& a, double* rhs, double* sol, const 
     c->slot[LES_B] = rhs;
     c->slot[LES_P] = sol;
     les_pcg_result r{};
-    // (the TMA passes' waits may give up, which the host looks for after each inner solve)
-    if (o.precision == LES_MIXED && c->graph_on && !c->prof_on && c->stencil_mode == 1 && c->fused && !c->opt_tma &&
-        fused_supported(&o) && o.max_iter > 0)
+    if (o.precision == LES_MIXED && c->graph_on && !c->prof_on && c->stencil_mode == 1 && c->fused && fused_supported(&o) &&
+        o.max_iter > 0)
         st = solve_graph(c, a, o, &r);
     else
         st = o.precision == LES_MIXED ? pcg_mixed_impl(c, &o, &r, 0) : pcg_fp64(c, &o, &r, 0);

@@ -945,9 +945,12 @@ __global__ void k_cond_inner(const SolverState* in, cudaGraphConditionalHandle h
     cudaGraphSetConditional(h, (!in->done && in->k < cap) ? 1u : 0u);
 }
 
-__global__ void k_cond_outer(const SolverState* out, cudaGraphConditionalHandle h, int max_outer, int cap)
+// in != nullptr: no correction follows an inner solve that broke down
+__global__ void k_cond_outer(const SolverState* out, const SolverState* in, cudaGraphConditionalHandle h, int max_outer,
+                             int cap)
 {
-    cudaGraphSetConditional(h, (!out->done && out->k < max_outer && out->iters < cap) ? 1u : 0u);
+    const bool broke = in && (in->status == LES_NONFINITE || in->status == LES_TIMEOUT);
+    cudaGraphSetConditional(h, (!out->done && !broke && out->k < max_outer && out->iters < cap) ? 1u : 0u);
 }
 
 // Adds a `while` loop at the current capture point of c->stream: creates the
@@ -964,8 +967,9 @@ static les_status capture_while(les_ctx* c, Entry entry, Body body)
 }
 
 // Emits the mixed solve of les_mixed.cu (outer FP64 defect correction, inner
-// fused FP32 PCG) into the capture in progress on c->stream.
-les_status capture_mixed_fused(les_ctx* c, const les_pcg_opts* o, ViewF A, int keep_tol)
+// fused FP32 PCG) into the capture in progress on c->stream.  end_broken: an
+// inner solve that broke down ends it, as it ends the loop driven from the host.
+les_status capture_mixed_fused(les_ctx* c, const les_pcg_opts* o, ViewF A, int keep_tol, bool end_broken)
 {
     SolverState* out = c->state;
     SolverState* in = c->state + 1;
@@ -975,21 +979,23 @@ les_status capture_mixed_fused(les_ctx* c, const les_pcg_opts* o, ViewF A, int k
     les_status st = fused_plan(c, o, A, in, out, P);
     if (st) return st;
     if ((st = emit_outer_start(c, o, keep_tol, inner_pitch(c, o)))) return st;   // tol, r = b - A x, ||r||
-    auto set_outer = [&](cudaGraphConditionalHandle h) -> les_status {
-        launch(c, k_cond_outer, 1, 1, (const SolverState*)out, h, max_outer, o->max_iter);
+    auto set_outer = [&](cudaGraphConditionalHandle h, const SolverState* solved) -> les_status {
+        launch(c, k_cond_outer, 1, 1, (const SolverState*)out, solved, h, max_outer, o->max_iter);
         return check_launch(c, "outer condition");
     };
+    const SolverState* const solved = end_broken ? in : nullptr;
     auto set_inner = [&](cudaGraphConditionalHandle h) -> les_status {
         launch(c, k_cond_inner, 1, 1, (const SolverState*)in, h, inner_cap);
         return check_launch(c, "inner condition");
     };
-    return capture_while(c, set_outer, [&](cudaGraphConditionalHandle ho) -> les_status {
+    return capture_while(c, [&](cudaGraphConditionalHandle ho) { return set_outer(ho, nullptr); },
+                         [&](cudaGraphConditionalHandle ho) -> les_status {
         les_status s2;
         if ((s2 = emit_inner_start(c, o, inner_cap))) return s2;     // inner state from the outer residual
         if (P.col && P.cp.cluster) {
             if ((s2 = cluster_solve(c, P.cp))) return s2;
             if ((s2 = emit_outer_update(c, o, P.col))) return s2;
-            return set_outer(ho);
+            return set_outer(ho, solved);
         }
         if ((s2 = emit_pass_b(c, P, true, 0, 0))) return s2;          // z = M^-1 r, rho, e = 0
         if ((s2 = emit_pass_a(c, P, true, 0))) return s2;             // iteration 1: p1 = z
@@ -1006,7 +1012,7 @@ les_status capture_mixed_fused(les_ctx* c, const les_pcg_opts* o, ViewF A, int k
         });
         if (s2) return s2;
         if ((s2 = emit_outer_update(c, o, P.col))) return s2;                   // x += e, r = b - A x, ||r||
-        return set_outer(ho);
+        return set_outer(ho, solved);
     });
 }
 

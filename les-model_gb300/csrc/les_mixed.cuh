@@ -302,7 +302,7 @@ les_status capture_while_on(cudaStream_t* stream, Check check, Entry entry, Body
 les_status emit_outer_start(les_ctx* c, const les_pcg_opts* o, int keep_tol, int pitch);
 les_status emit_inner_start(les_ctx* c, const les_pcg_opts* o, int inner_cap);
 les_status emit_outer_update(les_ctx* c, const les_pcg_opts* o, bool deferred);
-les_status capture_mixed_fused(les_ctx* c, const les_pcg_opts* o, ViewF A, int keep_tol);
+les_status capture_mixed_fused(les_ctx* c, const les_pcg_opts* o, ViewF A, int keep_tol, bool end_broken);
 ViewF view32_of(les_ctx* c);
 
 }  // namespace les

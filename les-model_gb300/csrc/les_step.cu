@@ -154,7 +154,7 @@ les_status les::emit_step(les_ctx* c, const les_step_params* prm)
     if (c->ev_pre && (st = check_cuda(c, cudaEventRecordWithFlags(c->ev_pre, c->stream, cudaEventRecordExternal),
                                       "step event")))
         return st;
-    if ((st = capture_mixed_fused(c, &prm->pcg, view32_of(c), prm->rel_tol > 0 ? 1 : 0))) return st;
+    if ((st = capture_mixed_fused(c, &prm->pcg, view32_of(c), prm->rel_tol > 0 ? 1 : 0, false))) return st;
     return emit_step_post(c, prm);
 }
 
