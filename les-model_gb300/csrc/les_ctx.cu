@@ -60,8 +60,9 @@ cudaError_t dev_malloc_bytes(les_ctx* c, void** p, size_t bytes)
 
 les_status ensure_work(les_ctx* c)
 {
-    if (c->w[0]) return LES_OK;
+    if (c->w[7]) return LES_OK;
     for (int q = 0; q < 8; ++q) {
+        if (c->w[q]) continue;   // an earlier call that ran out of memory got this far
         cudaError_t e = dev_malloc(c, &c->w[q], sizeof(double) * (size_t)c->g.n);
         if (e != cudaSuccess) return check_cuda(c, e, "cudaMalloc(work)");
         cudaMemsetAsync(c->w[q], 0, sizeof(double) * (size_t)c->g.n, c->stream);
@@ -71,8 +72,9 @@ les_status ensure_work(les_ctx* c)
 
 les_status ensure_work32(les_ctx* c)
 {
-    if (c->f[0]) return LES_OK;
+    if (c->f[7]) return LES_OK;
     for (int q = 0; q < 8; ++q) {
+        if (c->f[q]) continue;
         const size_t bytes = sizeof(float) * (size_t)c->g.nx * c->g.ny * plane_pitch(c->g.nz);   // rows may be padded
         cudaError_t e = dev_malloc(c, &c->f[q], bytes);
         if (e != cudaSuccess) return check_cuda(c, e, "cudaMalloc(work32)");
