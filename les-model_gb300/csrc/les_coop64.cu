@@ -30,7 +30,7 @@ struct Meet {
     double* part;
     unsigned* count;
     int* err;
-    int stall;   // this block never arrives (LES_OPT_TEST_STALL)
+    unsigned arrive;   // 1; 0: this block never arrives (LES_OPT_TEST_STALL)
     unsigned nb, number;
 };
 
@@ -85,7 +85,7 @@ __device__ __forceinline__ int meet(Meet& m, double (&v)[NV], double (*sm)[CT], 
 #pragma unroll
             for (int q = 0; q < NV; ++q) __stcg(s + q * m.nb + blockIdx.x, v[q]);
         __threadfence();   // the block's stores before the arrival
-        if (!m.stall) atomicAdd(m.count, 1u);
+        atomicAdd(m.count, m.arrive);
         const unsigned target = e * m.nb;
         unsigned spins = 0;
         unsigned long long t0 = 0;
@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(CT, 1) k_pcg64(const __grid_constant__ Args a)
     __shared__ double sm[2][CT];
     __shared__ Scalars sc;
     const Geo& g = a.g;
-    Meet m{a.part, a.count, a.err, a.stall && blockIdx.x == 0, gridDim.x, 0};
+    Meet m{a.part, a.count, a.err, a.stall && blockIdx.x == 0 ? 0u : 1u, gridDim.x, 0};
     const int per = (g.n + (int)gridDim.x - 1) / (int)gridDim.x;
     const int c0 = (int)blockIdx.x * per + (int)threadIdx.x, c1 = min(g.n, ((int)blockIdx.x + 1) * per);
     const double tol = a.keep_tol ? a.st->tol : a.tol;
@@ -209,7 +209,7 @@ __global__ void __launch_bounds__(CT, 1) k_pcg64(const __grid_constant__ Args a)
     // M^-1 r of the pointwise preconditioners (Jacobi, src/pressure.cpp:420-428;
     // Chebyshev's step 0), formed where r is
     auto point = [&](int c, double rv) {
-        const double zv = a.degree == 0 ? (a.A.code ? (a.A.code[c] ? div_by(rv, a.by_c0) : rv) : rv / a.A.d[0][c])
+        const double zv = a.degree == 0 ? (PLAIN || a.A.code ? (a.A.code[c] ? div_by(rv, a.by_c0) : rv) : rv / a.A.d[0][c])
                                         : fma(a.alpha0, rv, 0.0);
         if (steps <= 0) a.z[c] = zv;
         return zv;
