@@ -527,7 +527,7 @@ def run_adjoint(args):
 # and 6 fused operations
 FP64_OPS_PER_CELL = {"spmv_f64": 8.0,      # row + p.q term
                      "update_f64": 6.0,    # x += a p, r -= a q, r.r term, z_0 = a0 r
-                     "cheb_f64": 13.0}     # row + r - Az + beta p + z + alpha p}     # row + r - Az + beta p + z + alpha p
+                     "cheb_f64": 13.0}     # row, r - A z, + beta p, z + alpha p, r.z' (formed in every step)
 
 
 def rel_err(a, b, tmp=None):
@@ -570,6 +570,8 @@ def run_ours(args):
     if (not gs and args.tune and args.fused == 1 and args.rows == "0,0" and args.chunks == "0,0"
             and args.precond != "ic"):
         tune_us = ctx.autotune(prm.pcg)
+    # the strips' shape: what a solve that runs as strips uses (forced rows or chunks, or the
+    # autotuner found strips faster than the plane marches)
     shape_used = {k: ctx.get_option(o) for k, o in (("rows_a", G.OPT_ROWS_A), ("rows_b", G.OPT_ROWS_B),
                                                     ("chunk_a", G.OPT_CHUNK_A), ("chunk_b", G.OPT_CHUNK_B))}
     ctx64 = ctxT = None

@@ -411,7 +411,11 @@ les_status les_get_option(const les_ctx* ctx, int option, int* value);
 /* Number of kernels this context has launched so far. */
 unsigned long long les_launch_count(const les_ctx* ctx);
 /* CUDA-event timing of the solver's hot kernels: enable=1 starts a fresh
- * record, 0 stops recording. */
+ * record, 0 stops recording.  Kernels are timed launch by launch: while a record
+ * runs, steps are not captured, and the solves that otherwise run in one launch --
+ * mixed solves of small grids (one thread-block cluster), FP64 Jacobi and
+ * Chebyshev PCG up to 2^20 cells (one cooperative launch) -- run as the launches
+ * that serve the larger grids.  Those are the kernels the times are of. */
 les_status les_profile(les_ctx* ctx, int enable);
 /* Launch count and summed device time (ms) of one profiled kernel id
  * (0..7, names from les_profile_name). */

@@ -16,7 +16,7 @@
 // (les_plane.cuh); the sums differ by reassociation.
 //
 // Microseconds per inner iteration, plane marches -> cluster (GB300, degree 4):
-//     16x32x32 10.0 -> 3.8    64x32x32 10.3 -> 5.2
+//     16x32x32 10.0 -> 3.8    64x32x32 10.3 -> 5.3
 //     48x48x32 10.6 -> 6.4    60x40x40 12.1 -> 8.7
 // (Jacobi at 64x32x32 7.4 -> 3.4, degree 7 16.8 -> 8.3).
 // What bounds it: a barrier with the stores before it takes 0.35 us (the

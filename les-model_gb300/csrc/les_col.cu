@@ -2,9 +2,9 @@
 // two register-resident column marches (Jacobi or Chebyshev preconditioner).
 //
 // The strips of this file serve batched ensembles, solves with a forced strip
-// shape and vectors of 4 GB and more; the others run the same two passes as
-// plane marches (les_plane.cuh) or, on small grids, in one cluster
-// (les_cluster.cu).
+// shape, vectors of 4 GB and more and cells very long along i; the others run the
+// same two passes as plane marches (les_plane.cuh) or, on small grids, in one
+// cluster (les_cluster.cu).
 //
 // Each warp owns a strip of the grid, 32 consecutive cells along k (one per
 // lane) by H rows along j, and marches along i over a chunk of planes.  A lane

@@ -51,7 +51,9 @@ inline dim3 cell_block() { return dim3(TBK, TBJ, 1); }
 // the ghost-doubling of src/pressure.cpp:663-696:
 //   x (w,e): 0:(1,1) 1:(0,2) 2:(1,0) 3:(0,0) 4:(2,0)
 //   y (s,n) and z (b,t): 0:(1,1) 1:(0,2) 2:(2,0) 3:(1,0)
-// Multipliers are packed two bits per state.
+// Multipliers are packed two bits per state.  A fluid cell between a wall and a
+// solid cell keeps the multiplier 1 for the neighbour in the wall: a row has to
+// leave neighbours outside the grid out (:721-744), whatever their multiplier.
 constexpr unsigned XW_PACK = 1u | (0u << 2) | (1u << 4) | (0u << 6) | (2u << 8);
 constexpr unsigned XE_PACK = 1u | (2u << 2) | (0u << 4) | (0u << 6) | (0u << 8);
 constexpr unsigned YL_PACK = 1u | (0u << 2) | (2u << 4) | (1u << 6);  // s / b
