@@ -527,7 +527,7 @@ def run_adjoint(args):
 # and 6 fused operations
 FP64_OPS_PER_CELL = {"spmv_f64": 8.0,      # row + p.q term
                      "update_f64": 6.0,    # x += a p, r -= a q, r.r term, z_0 = a0 r
-                     "cheb_f64": 13.0}     # row, r - A z, + beta p, z + alpha p, r.z' (formed in every step)
+                     "cheb_f64": 37.0 / 3}  # row, r - A z, + beta p, z + alpha p; r.z' in the last of three steps
 
 
 def rel_err(a, b, tmp=None):

@@ -309,19 +309,24 @@ namespace les {
 
 // Cells up to which the cooperative form is taken.  Microseconds per iteration,
 // launch by launch and cooperative (GB300), of Jacobi / Chebyshev degree 4:
-//   64x32x32     26.5 / 13.3     48 / 28      111x65x73   74.7 / 37.4   188 / 113
-//   80x80x80     65.6 / 36.6    155 / 111     (h = 0.01: no power of two, rows of
-//   100x100x100   102 / 61      269 / 195     thirteen operations instead of the
-//                                             launched kernels' eight to ten)
-//   128x128x64   71.0 / 51.5    162 / 154     degree 7 254 / 244, h = 0.01 363 / 337
-// It was also ahead at 160x128x100 (132 / 89, 342 / 283), the largest timed; the
-// line stays at the size up to which every degree and spacing was.
-constexpr long long COOP_CELLS = 1 << 20;
+//   64x32x32     26.5 / 13.2     48 / 28      90x90x90    70.3 / 48.2    164 / 149
+//   80x80x80     60.3 / 37.4    133 / 111     100x100x100 93.3 / 62.2    228 / 196
+//   128x128x64   71.0 / 51.4    157 / 153     degree 7 243 / 244
+// (h = 0.01 but for the first and the last).  It was also ahead at 160x128x100,
+// the largest timed (132 / 90, 330 / 284; h = 0.01 155 / 116, 420 / 387); the line
+// stays at the size up to which every degree was.
+// A spacing that is no power of two has rows of thirteen operations here and of
+// eight to ten in the launched kernels, which come out ahead from degree 3 where
+// their tiles of 8 x 32 cells fill the plane: 128x128x64, h = 0.01, degree 3 155 /
+// 161, degree 7 303 / 336; 128x80x64 degree 3 117 / 106, degree 7 219 / 219.
+constexpr long long COOP_CELLS = 1 << 20, COOP_CELLS_WHOLE = 5 << 17;
 
-bool pcg64_coop_used(const les_ctx* c, const les_pcg_opts* o)
+bool pcg64_coop_used(const les_ctx* c, const les_pcg_opts* o, bool pow2)
 {
-    return (o->precond == LES_PC_JACOBI || (o->precond == LES_PC_CHEBYSHEV && o->degree >= 1 && o->degree <= MAX_STEPS + 1)) && o->max_iter > 0 &&
-           !c->prof_on && c->g.n <= COOP_CELLS;
+    const bool cheb = o->precond == LES_PC_CHEBYSHEV;
+    if (!(o->precond == LES_PC_JACOBI || (cheb && o->degree >= 1 && o->degree <= MAX_STEPS + 1))) return false;
+    const bool whole = c->stencil_mode == 1 && !pow2 && cheb && o->degree > 2 && c->g.ny % TBJ == 0 && c->g.nz % TBK == 0;
+    return o->max_iter > 0 && !c->prof_on && c->g.n <= (whole ? COOP_CELLS_WHOLE : COOP_CELLS);
 }
 
 // The whole solve in one launch; the state is read back (and a wait that gave

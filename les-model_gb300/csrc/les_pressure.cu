@@ -25,7 +25,7 @@ les_status ic_apply_dev(les_ctx* c, const double* const* L, const double* r, dou
 les_status wave_check(les_ctx* c);
 les_status build_ic_dev(les_ctx* c);
 les_status pcg_mixed(les_ctx* c, const les_pcg_opts* o, les_pcg_result* res);
-bool pcg64_coop_used(const les_ctx* c, const les_pcg_opts* o);   // les_coop64.cu
+bool pcg64_coop_used(const les_ctx* c, const les_pcg_opts* o, bool pow2);   // les_coop64.cu
 les_status pcg64_coop(les_ctx* c, const les_pcg_opts* o, bool pow2, int keep_tol);
 }
 
@@ -71,19 +71,21 @@ __device__ __forceinline__ double apply_row(const StencilView& A, const double* 
 //            is formed once per cell and handed on -- along i in registers as
 //            the block marches, along j and k in shared memory; one product
 //            serves all axes whose spacings are equal
-// An FP64 Chebyshev(4)-PCG step of 256x128x128 (POW2, with step 0 and r.z in
-// the kernels next to them): 586 -> 415 ms.
+// 256x128x128, general rows of one cell per thread -> POW2 / SHARED: SpMV
+// 125 -> 58 / 91 us (with p.q 64 / 99); Chebyshev(4)-PCG iteration, with step 0
+// and r.z in the kernels next to them, 735 -> 495 / 639 us (a matrix of the
+// caller 735 -> 706).
 enum RowForm { ROW_GENERAL = 0, ROW_POW2 = 1, ROW_SHARED = 2 };
 
 struct RowTile {
     double v[2][2][TBJ + 2][TBK + 2];   // [plane parity][y, z products]
 };
 
-// multiplier 0, 1 or 2 of a base coefficient
+// multiplier 0, 1 or 2 of a base coefficient (its bit pattern: integer operations)
 __device__ __forceinline__ double mult(unsigned pack, unsigned state)
 {
     const unsigned m = (pack >> (2 * state)) & 3u;
-    return m == 0u ? 0.0 : (m == 1u ? 1.0 : 2.0);
+    return __hiloint2double(m ? (int)(0x3fe00000u + (m << 20)) : 0, 0);
 }
 
 // Calls f(i, id, x_c, (A x)_c) for the cells of this thread's column on the
@@ -106,23 +108,40 @@ __device__ __forceinline__ void march_rows(const StencilView& A, const double* _
     }
     __shared__ RowTile tile;
     const StencilCoef& c = A.k;
-    const bool same_y = c.y1 == c.x1, same_z = c.z1 == c.y1;
+    // (compared as bit patterns: a comparison of doubles takes the FP64 pipe)
+    const bool same_y = __double_as_longlong(c.y1) == __double_as_longlong(c.x1);
+    const bool same_z = __double_as_longlong(c.z1) == __double_as_longlong(c.y1);
     const int tj = threadIdx.y + 1, tk = threadIdx.x + 1;
-    const bool lo_j = in && threadIdx.y == 0 && j > 0, hi_j = in && threadIdx.y == TBJ - 1 && j < g.ny - 1;
-    const bool lo_k = in && threadIdx.x == 0 && k > 0, hi_k = in && threadIdx.x == TBK - 1 && k < g.nz - 1;
+    // The products around the tile: the row before it by warp 0, the row after it by
+    // warp 1, the columns on either side by a half of warp 2 -- one FP64
+    // instruction of a warp for up to 32 of them (by each row's own edge lanes:
+    // two in every warp).
+    const int j0 = blockIdx.y * TBJ, k0 = blockIdx.x * TBK;
+    int hj = j, hk = k;
+    bool halo = false;
+    if (threadIdx.y == 0) {
+        hj = j0 - 1;
+        halo = hj >= 0 && k < g.nz;
+    } else if (threadIdx.y == 1) {
+        hj = j0 + TBJ;
+        halo = hj < g.ny && k < g.nz;
+    } else if (threadIdx.y == 2 && threadIdx.x < 2 * TBJ) {
+        hj = j0 + (threadIdx.x & (TBJ - 1));
+        hk = threadIdx.x < TBJ ? k0 - 1 : k0 + TBK;
+        halo = hj < g.ny && hk >= 0 && hk < g.nz;
+    }
+    const bool halo_z = threadIdx.y == 2;
+    const double halo_coef = halo_z ? c.z1 : c.y1;
+    const int halo_off = hj * g.sj + hk, hr = hj - j0 + 1, hc = hk - k0 + 1;
     int id = i0 * g.si + j * g.sj + k;
     double xc = in ? x[id] : 0.0;
     double pw = in && i0 > 0 ? c.x1 * x[id - g.si] : 0.0, pc = c.x1 * xc;
     for (int i = i0; i < i1; ++i, id += g.si) {
         auto& ty = tile.v[i & 1][0];
         auto& tz = tile.v[i & 1][same_z ? 0 : 1];
-        const double py = same_y ? pc : c.y1 * xc;
-        ty[tj][tk] = py;
+        ty[tj][tk] = same_y ? pc : c.y1 * xc;
         if (!same_z) tz[tj][tk] = c.z1 * xc;
-        if (lo_j) ty[0][tk] = c.y1 * x[id - g.sj];
-        if (hi_j) ty[TBJ + 1][tk] = c.y1 * x[id + g.sj];
-        if (lo_k) tz[tj][0] = c.z1 * x[id - 1];
-        if (hi_k) tz[tj][TBK + 1] = c.z1 * x[id + 1];
+        if (halo) (halo_z ? tz : ty)[hr][hc] = halo_coef * x[i * g.si + halo_off];
         const double xe = in && i < g.nx - 1 ? x[id + g.si] : 0.0;
         const double pe = c.x1 * xe;
         __syncthreads();   // one barrier per plane: the planes alternate between two tiles
@@ -238,7 +257,7 @@ __global__ void k_expand_stencil(Geo g, StencilView A, double* c, double* n, dou
 // out = A in (+ optional dot in.out reduced into the state).
 enum { DOT_NONE = 0, DOT_ALPHA = 1, DOT_SCAL0 = 2 };
 
-template <int FORM>
+template <int FORM, bool DOT>
 __global__ void k_spmv(Geo g, StencilView A, int ci, const double* __restrict__ p, double* __restrict__ q,
                        double* partials, unsigned* counter, SolverState* st, int dot_mode)
 {
@@ -247,10 +266,9 @@ __global__ void k_spmv(Geo g, StencilView A, int ci, const double* __restrict__ 
     double pq[1] = {0.0};
     march_rows<FORM>(A, p, g, ci, [&](int, int id, double pc, double val) {
         q[id] = val;
-        pq[0] = fma(pc, val, pq[0]);
+        if (DOT) pq[0] = fma(pc, val, pq[0]);
     });
-    if (dot_mode == DOT_NONE) return;
-    if (last_block_sum<1>(pq, partials, counter, sm)) {
+    if (DOT && last_block_sum<1>(pq, partials, counter, sm)) {
         if (threadIdx.x == 0 && threadIdx.y == 0) {
             if (dot_mode == DOT_ALPHA) {
                 st->pq = pq[0];
@@ -412,9 +430,10 @@ __global__ void k_cheb0(Geo g, double alpha0, const double* __restrict__ r, doub
 // pin == nullptr means p_{k-1} = r (first step).  dot_mode != RD_NONE: also
 // r.z' (the last step).
 //
-// Bound by the FP64 pipe: 7 to 8 operations for the row and 5 for the
-// recurrence per cell (18 with every product rounded by itself).
-template <int FORM>
+// Bound by the FP64 pipe: 7 to 10 operations for the row, 5 for the recurrence
+// and one for r.z per cell (18 with every product rounded by itself; formed in
+// every step, r.z cost 5 % of a Chebyshev(4)-PCG iteration).
+template <int FORM, bool DOT>
 __global__ void k_cheb_step(Geo g, StencilView A, int ci, double alpha, double beta,
                             const double* __restrict__ r, const double* __restrict__ zin,
                             const double* pin, double* pout, double* __restrict__ zout,
@@ -430,10 +449,9 @@ __global__ void k_cheb_step(Geo g, StencilView A, int ci, double alpha, double b
         if (pout) pout[id] = pv;
         const double zv = zc + alpha * pv;
         zout[id] = zv;
-        rz[0] = fma(rv, zv, rz[0]);
+        if (DOT) rz[0] = fma(rv, zv, rz[0]);
     });
-    if (dot_mode == RD_NONE) return;
-    if (last_block_sum<1>(rz, partials, counter, sm))
+    if (DOT && last_block_sum<1>(rz, partials, counter, sm))
         if (threadIdx.x == 0 && threadIdx.y == 0) dot_done(st, dot_mode, rz[0]);
 }
 
@@ -664,11 +682,21 @@ static int row_form(const les_ctx* c)
     return pow2(c->coef.x1) && pow2(c->coef.y1) && pow2(c->coef.z1) ? ROW_POW2 : ROW_SHARED;
 }
 
+// Rows without a sum behind them: where they share nothing along i a plane per
+// block (general rows of 200x200x200, a Chebyshev(4) apply: 972 us; marched 1138)
+static MarchGrid plain_grid(const les_ctx* c, int form)
+{
+    return form == ROW_GENERAL && c->g.nx <= 65535 ? MarchGrid{cell_grid(c->g), 1} : march_grid(c);
+}
+
 static void launch_spmv(les_ctx* c, int pid, const double* in, double* out, int dot_mode)
 {
-    const MarchGrid m = march_grid(c);
     const int f = row_form(c);
-    auto k = f == ROW_POW2 ? k_spmv<ROW_POW2> : (f == ROW_SHARED ? k_spmv<ROW_SHARED> : k_spmv<ROW_GENERAL>);
+    const bool dot = dot_mode != DOT_NONE;
+    const MarchGrid m = dot ? march_grid(c) : plain_grid(c, f);
+    auto k = f == ROW_POW2 ? (dot ? k_spmv<ROW_POW2, true> : k_spmv<ROW_POW2, false>)
+                           : (f == ROW_SHARED ? (dot ? k_spmv<ROW_SHARED, true> : k_spmv<ROW_SHARED, false>)
+                                              : (dot ? k_spmv<ROW_GENERAL, true> : k_spmv<ROW_GENERAL, false>));
     if (pid >= 0) launch_p(c, pid, k, m.grid, cell_block(), c->g, stencil_view(c), m.ci, in, out, c->partials,
                            c->counters + 1, c->state, dot_mode);
     else launch(c, k, m.grid, cell_block(), c->g, stencil_view(c), m.ci, in, out, c->partials, c->counters + 1,
@@ -744,17 +772,21 @@ static les_status precond_dot(les_ctx* c, const les_pcg_opts* o, const double* r
         if (!z0_done)
             launch(c, k_cheb0, cell_grid(g), cell_block(), g, alpha, r, zb[cur], c->state, skip_done);
         double* pbuf = c->w[7];
-        const MarchGrid m = march_grid(c);
         const int f = row_form(c);
-        auto kc = f == ROW_POW2 ? k_cheb_step<ROW_POW2>
-                                : (f == ROW_SHARED ? k_cheb_step<ROW_SHARED> : k_cheb_step<ROW_GENERAL>);
+        const MarchGrid md = march_grid(c);
+        const MarchGrid mc = plain_grid(c, f);
+        auto kc = f == ROW_POW2 ? k_cheb_step<ROW_POW2, false>
+                                : (f == ROW_SHARED ? k_cheb_step<ROW_SHARED, false> : k_cheb_step<ROW_GENERAL, false>);
+        auto kd = f == ROW_POW2 ? k_cheb_step<ROW_POW2, true>
+                                : (f == ROW_SHARED ? k_cheb_step<ROW_SHARED, true> : k_cheb_step<ROW_GENERAL, true>);
         for (int kq = 1; kq <= steps; ++kq) {
             double beta = (cc * alpha / 2.0) * (cc * alpha / 2.0);
             alpha = 1.0 / (d - beta);
-            const bool last = kq == steps;
-            launch_p(c, PROF_CHEB64, kc, m.grid, cell_block(), g, A, m.ci, alpha, beta, r, (const double*)zb[cur],
-                     (const double*)(kq == 1 ? nullptr : pbuf), last ? nullptr : pbuf, zb[cur ^ 1], c->state,
-                     skip_done, c->partials, c->counters + 2, last ? dot_mode : (int)RD_NONE);
+            const bool last = kq == steps, dot = last && dot_mode != RD_NONE;
+            const MarchGrid& m = dot ? md : mc;
+            launch_p(c, PROF_CHEB64, dot ? kd : kc, m.grid, cell_block(), g, A, m.ci, alpha, beta, r,
+                     (const double*)zb[cur], (const double*)(kq == 1 ? nullptr : pbuf), last ? nullptr : pbuf,
+                     zb[cur ^ 1], c->state, skip_done, c->partials, c->counters + 2, dot_mode);
             cur ^= 1;
         }
         if (steps > 0) return check_launch(c, "chebyshev pc");   // the last step formed r.z
@@ -824,8 +856,9 @@ les_status pcg_fp64(les_ctx* c, const les_pcg_opts* o, les_pcg_result* res, int 
     les_status st = ensure_work(c);
     if (st) return st;
     if ((st = ic_ready(c, o))) return st;
-    if (pcg64_coop_used(c, o)) {
-        if ((st = pcg64_coop(c, o, row_form(c) == ROW_POW2, keep_tol))) return st;
+    const bool pow2 = row_form(c) == ROW_POW2;
+    if (pcg64_coop_used(c, o, pow2)) {
+        if ((st = pcg64_coop(c, o, pow2, keep_tol))) return st;
         if ((st = wave_check(c))) return st;   // the exchanges' bounded waits
         if ((st = read_state(c))) return st;
         const SolverState& h = *c->h_state;
