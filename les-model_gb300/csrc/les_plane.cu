@@ -61,16 +61,20 @@ bool tile_fit(const Geo& g, int nk, int nj, int h, int threads, PlaneMap& m)
 // warps.  Among equals the one with the fewest warps on an SM, which spreads the
 // work over more of them: 96x64x64, pass B in 144 blocks instead of 96, an
 // iteration 13.5 -> 12.7 us.
-bool plane_tiles(const Geo& g, int h, int levels, int threads, int sms, PlaneMap& best)
+// best == nullptr: only whether there is a tile that fits.
+bool plane_tiles(const Geo& g, int h, int levels, int threads, int sms, PlaneMap* best)
 {
     double best_t = 1e30;
     int best_w = 0;
     for (int nk = 1; nk <= 16; ++nk) {
         int tried = 0;
-        for (int nj = 1; nj <= g.ny && tried < 8; ++nj) {
-            PlaneMap m;
+        PlaneMap m;
+        tile_fit(g, nk, 1, h, threads, m);   // (for lk)
+        const int most = PR * (threads / m.lk);   // rows that fit, the fewest row tiles:
+        for (int nj = most ? (g.ny + most - 1) / most : g.ny + 1; nj <= g.ny && tried < 8; ++nj) {
             if (!tile_fit(g, nk, nj, h, threads, m)) continue;
             if (m.nk != nk || m.nj != nj) continue;   // the same tiles as a smaller count's
+            if (!best) return true;
             ++tried;
             int res = threads / m.threads;
             const size_t by_smem = SMEM_MAX / plane_smem(threads, levels);
@@ -91,7 +95,7 @@ bool plane_tiles(const Geo& g, int h, int levels, int threads, int sms, PlaneMap
                 if (t < best_t || (t == best_t && warps < best_w)) {
                     best_t = t;
                     best_w = warps;
-                    best = m;
+                    *best = m;
                 }
             }
         }
@@ -159,19 +163,20 @@ static bool levels_fit(const les_ctx* c, const les_pcg_opts* o, int S)
     return level_growth(p, S) <= 0x1p60 && std::fabs(p.zs.x) >= 0x1p-126f;
 }
 
-static bool plane_plan(const les_ctx* c, const les_pcg_opts* o, int S, PlaneMap& a, PlaneMap& b)
+// a, b: nullptr to ask only whether there are plans
+static bool plane_plan(const les_ctx* c, int S, PlaneMap* a, PlaneMap* b)
 {
     const Geo& g = c->g;
     const double share = c->share > 0 && c->share <= 1 ? c->share : 1.0;
     const int sms = std::max(1, (int)(c->sms * share));
     if (!plane_tiles(g, 1, 1, plane_threads_a(), sms, a)) return false;
-    if (S == 0) {
-        b = PlaneMap{};
-        b.threads = 512;
-        b.items = std::max(1, std::min(2 * sms, (g.nx * (padded(g).si / PV) + 511) / 512));
-        return true;
+    if (S > 0) return plane_tiles(g, S, S, plane_threads_b(S), sms, b);
+    if (b) {
+        *b = PlaneMap{};
+        b->threads = 512;
+        b->items = std::max(1, std::min(2 * sms, (g.nx * (padded(g).si / PV) + 511) / 512));
     }
-    return plane_tiles(g, S, S, plane_threads_b(S), sms, b);
+    return true;
 }
 
 // The plane marches serve the solves of the register-column passes: they were
@@ -186,14 +191,12 @@ bool plane_used(const les_ctx* c, const les_pcg_opts* o)
     if ((unsigned long long)c->g.nx * c->g.ny * plane_pitch(c->g.nz) >= (1ull << 30)) return false;
     if ((c->tune_tja || c->tune_tjb || c->tune_cia || c->tune_cib) && !c->tune_plane) return false;
     const int S = o->precond == LES_PC_JACOBI ? 0 : o->degree - 1;
-    if (!levels_fit(c, o, S)) return false;
-    PlaneMap a, b;
-    return plane_plan(c, o, S, a, b);
+    return levels_fit(c, o, S) && plane_plan(c, S, nullptr, nullptr);
 }
 
 les_status plane_maps(les_ctx* c, const les_pcg_opts* o, ColPlan& P)
 {
-    if (!plane_plan(c, o, P.S, P.pa, P.pb)) return fail(c, LES_BAD_ARG, "plane march: no tile fits");
+    if (!plane_plan(c, P.S, &P.pa, &P.pb)) return fail(c, LES_BAD_ARG, "plane march: no tile fits");
     P.blocks_a = P.pa.items;
     P.blocks_b = P.pb.items;
     return LES_OK;
