@@ -41,3 +41,23 @@ def test_rows(oracle_lib, h, solids, bad):
             c.precond_apply(G.pcg_opts(precond=G.PC_CHEBYSHEV, lambda_min=3 * np.pi ** 2, lambda_max=lmax,
                                        degree=degree), "p", "b")
             assert np.array_equal(c.download("b"), want, equal_nan=True), degree
+
+
+def test_quotients_of_zeros_keep_their_sign(oracle_lib):
+    """The Jacobi preconditioner's division by a constant: +-0 / A_c is +-0, and
+    subnormals and the largest numbers take the division."""
+    shape, h = (6, 7, 33), (0.07, 0.1, 0.03)
+    om = O.Mesh(*shape, *h)
+    A = oracle_lib.build_stencil(om, np.zeros(om.n, np.uint8))
+    x = np.resize([0.0, -0.0, 1.0, -1.5, 5e-324, -1e-310, 1.7e308, -3e-300, 1e250, np.inf, -np.inf, np.nan], om.n)
+    want = np.zeros(om.n)
+    oracle_lib.jacobi_precond(A, x, want)
+    with G.Context(G.Mesh(*shape, *h)) as c:
+        c.upload_mask(np.zeros(om.n, np.uint8))
+        c.build_stencil()
+        c.upload("p", x)
+        c.precond_apply(G.pcg_opts(precond=G.PC_JACOBI), "p", "b")
+        got = c.download("b")
+    assert np.array_equal(got, want, equal_nan=True)
+    number = ~np.isnan(want)
+    assert np.array_equal(np.signbit(got[number]), np.signbit(want[number]))
