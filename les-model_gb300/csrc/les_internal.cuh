@@ -127,10 +127,8 @@ struct StencilView {
 // multiply-add, and one correction (Brisebarre, Muller and Raina,
 // "Accelerating correctly rounded floating-point division when the divisor is
 // known in advance", IEEE Trans. Computers 53(8), 2004, theorem 3).  The
-// theorem wants no under- or overflow: operands outside a wide exponent range take
-// the division.  A zero's quotient is x y, a zero of the same sign (the division
-// takes twice as long for a zero: Jacobi sweeps of p = 0, 200x100x100, 494 us with
-// zeros divided, 84 so).
+// theorem wants no under- or overflow: operands outside a wide exponent range
+// (zeros among them) take the division.
 struct DivBy {
     double d, y;
     int ok;   // the divisor lies in the range
@@ -143,16 +141,25 @@ inline DivBy div_by_const(double d)
     return DivBy{d, 1.0 / d, std::isfinite(d) && d != 0.0 && e > -200 && e < 200};
 }
 
-// out of line: rare, and large where it is inlined
-__device__ __noinline__ static double div_slow(double x, double d) { return x / d; }
+// Out of line: rare, and large where it is inlined.  A zero over a finite or
+// infinite number is the zero of the operands' signs: the division takes twice as
+// long for zeros as for numbers (Jacobi sweeps from p = 0 at 200x100x100: 494 us,
+// 113 so; tested for in line it cost sweeps of any p up to 13 %).
+__device__ __noinline__ static double div_slow(double x, double d)
+{
+    const int xh = __double2hiint(x), dh = __double2hiint(d);
+    const unsigned long long mag = (unsigned long long)__double_as_longlong(d) << 1;
+    if (((xh << 1) | __double2loint(x)) == 0 && mag != 0ull && mag <= 0xffe0000000000000ull)
+        return __hiloint2double((xh ^ dh) & (int)0x80000000u, 0);
+    return x / d;
+}
 
 __device__ __forceinline__ double div_by(double x, const DivBy& c)
 {
-    const int hi = __double2hiint(x), e = (hi >> 20) & 0x7ff;
-    if (c.ok) {
+    const int e = (__double2hiint(x) >> 20) & 0x7ff;
+    if (c.ok && e > 1023 - 700 && e < 1023 + 700) {
         const double q = x * c.y;
-        if (e > 1023 - 700 && e < 1023 + 700) return fma(fma(-q, c.d, x), c.y, q);
-        if (((hi << 1) | __double2loint(x)) == 0) return q;
+        return fma(fma(-q, c.d, x), c.y, q);
     }
     return div_slow(x, c.d);
 }
