@@ -83,6 +83,7 @@ def test_what_the_copies_leave_allocated():
             c.precond_apply(G.pcg_opts(precond=G.PC_IC), "p", "b")
             return before - torch.cuda.mem_get_info()[0]
 
+    left((9, 7, 35), 1)   # loads the kernels of both forms
     assert left((64, 400, 400), 1) == 0
     assert left((96, 64, 64), 0) == 0
     assert 0 < left((96, 64, 64), 1) < (48 << 20)   # 9 arrays of 16 x 2 tiles, 130 steps, 128 cells: 38 MB
